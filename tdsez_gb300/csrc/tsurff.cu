@@ -37,35 +37,89 @@ struct FaceParams {
     int pa;                      // degree of the normal axis
     const double *wval, *wder;   // p+1 values / derivatives at the wall
     const double *xb, *xc, *wb, *wc;   // node coordinates and weights
-    double Ab, Ac, inv_mass, sigma;
+    double Ab, Ac;
+    int nb, nc;                  // momenta along b and c
+    const double2 *eb, *ec;      // exp(-i k x_q) along b and c: [nk][Q]
+    size_t goff, hoff, toff;     // this face's place in g, H and T
+};
+struct Faces {
+    FaceParams f[6];
+    int nf;
+    double inv_mass;
+};
+
+struct KGrid {
+    int nk[3];
+    const double *k[3];
+};
+
+// per-momentum phases of one sample, one axis after the other:
+// wall[k] = exp(-i (k + A_d) R) and fin[k] = exp(i (t k^2 / 2m + k B_d / m)),
+// so the kernels over the momentum grid multiply table entries instead of
+// calling sincos 2 dim + 1 times per momentum
+struct PhaseParams {
+    KGrid kg;
+    double A[3], B[3], R, t, inv2m, invm;
+    double2 *wall, *fin;
 };
 
 // g[0] = -e (1/m) d_n psi, g[1] = -i sigma e psi / m with e = w exp(-i A_t.x_t)
-__global__ void k_trace(FaceParams f, const double2 *__restrict__ psi, double2 *__restrict__ g) {
-    const int Qb = f.b.Q, Qc = f.c.Q;
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= Qb * Qc) return;
-    const int ib = idx / Qc, ic = idx % Qc;
-    const int ob = f.b.off[ib], oc = f.c.off[ic];
-    double2 v = make_double2(0, 0), dn = make_double2(0, 0);
-    for (int ja = 0; ja <= f.pa; ++ja) {
-        const double va = f.wval[ja], da = f.wder[ja];
-        const size_t ia = (size_t)(f.wall_off + ja) * f.stride[f.a];
-        for (int jb = 0; jb <= f.b.p; ++jb) {
-            const double vb = f.b.val[ib * (f.b.p + 1) + jb];
-            const size_t ibb = ia + (size_t)(ob + jb) * f.stride[(f.a == 0) ? 1 : 0];
-            for (int jc = 0; jc <= f.c.p; ++jc) {
-                const double vc = f.c.val[ic * (f.c.p + 1) + jc];
-                const size_t e = ibb + (size_t)(oc + jc) * f.stride[(f.a == 2) ? 1 : 2];
-                const double2 ps = psi[e];
-                const double wv = va * vb * vc, wd = da * vb * vc;
-                v.x += wv * ps.x; v.y += wv * ps.y;
-                dn.x += wd * ps.x; dn.y += wd * ps.y;
+// at every surface node of every face (blockIdx.y; the row past the last face
+// fills the phase tables). `lanes` threads per node share its (p+1)^(dim-1)
+// tangential products and reduce by shuffles: with a few thousand nodes the
+// kernel is bound by the latency of the gathered loads, which one thread per
+// node issued one after the other (22 us per face at 1024 nodes of degree 4;
+// all four faces of that case take 12 us now).
+__global__ void __launch_bounds__(256) k_trace(const Faces fs, const PhaseParams pp, int lanes,
+                                               const double2 *__restrict__ psi, double2 *__restrict__ gall) {
+    const int gid = blockIdx.x * blockDim.x + threadIdx.x;
+    if ((int)blockIdx.y == fs.nf) {
+        int i = gid;
+        for (int d = 0; d < 3; ++d) {
+            if (i >= 0 && i < pp.kg.nk[d]) {
+                const double k = pp.kg.k[d][i];
+                const int o = (d > 0 ? pp.kg.nk[0] : 0) + (d > 1 ? pp.kg.nk[1] : 0) + i;
+                pp.wall[o] = cexpi(-(k + pp.A[d]) * pp.R);
+                pp.fin[o] = cexpi(pp.t * k * k * pp.inv2m + k * pp.B[d] * pp.invm);
             }
+            i -= pp.kg.nk[d];
         }
+        return;
     }
-    dn.x *= f.sigma * f.inv_mass;
-    dn.y *= f.sigma * f.inv_mass;
+    const FaceParams &f = fs.f[blockIdx.y];
+    const int Qb = f.b.Q, Qc = f.c.Q;
+    const int idx = gid / lanes, lane = gid % lanes;
+    const bool valid = idx < Qb * Qc;
+    const int ib = valid ? idx / Qc : 0, ic = valid ? idx % Qc : 0;
+    const int ob = f.b.off[ib], oc = f.c.off[ic];
+    const size_t sa = (size_t)f.stride[f.a], sb = (size_t)f.stride[f.a == 0 ? 1 : 0], sc = (size_t)f.stride[f.a == 2 ? 1 : 2];
+    double2 v = make_double2(0, 0), dn = make_double2(0, 0);
+    const int nbc = (f.b.p + 1) * (f.c.p + 1);
+    for (int e = lane; valid && e < nbc; e += lanes) {
+        const int jb = e / (f.c.p + 1), jc = e % (f.c.p + 1);
+        const double vt = f.b.val[ib * (f.b.p + 1) + jb] * f.c.val[ic * (f.c.p + 1) + jc];
+        const double2 *q = psi + (size_t)f.wall_off * sa + (size_t)(ob + jb) * sb + (size_t)(oc + jc) * sc;
+        double2 sv = make_double2(0, 0), sd = make_double2(0, 0);
+#pragma unroll 4
+        for (int ja = 0; ja <= f.pa; ++ja) {
+            const double2 ps = q[(size_t)ja * sa];
+            const double va = f.wval[ja], da = f.wder[ja];
+            sv.x += va * ps.x; sv.y += va * ps.y;
+            sd.x += da * ps.x; sd.y += da * ps.y;
+        }
+        v.x += vt * sv.x; v.y += vt * sv.y;
+        dn.x += vt * sd.x; dn.y += vt * sd.y;
+    }
+    for (int o = lanes / 2; o > 0; o >>= 1) {
+        v.x += __shfl_down_sync(0xffffffffu, v.x, o);
+        v.y += __shfl_down_sync(0xffffffffu, v.y, o);
+        dn.x += __shfl_down_sync(0xffffffffu, dn.x, o);
+        dn.y += __shfl_down_sync(0xffffffffu, dn.y, o);
+    }
+    if (!valid || lane != 0) return;
+    const double sm = (f.side ? 1.0 : -1.0) * fs.inv_mass;
+    dn.x *= sm;
+    dn.y *= sm;
     const double xb = f.xb[ib], xc = f.xc[ic];
     double2 e = cexpi(-(f.Ab * xb + f.Ac * xc));
     const double w = f.wb[ib] * f.wc[ic];
@@ -73,96 +127,137 @@ __global__ void k_trace(FaceParams f, const double2 *__restrict__ psi, double2 *
     const double2 g1 = cmul(e, dn);
     // -i sigma e psi / m
     const double2 ev = cmul(e, v);
-    const double s = f.sigma * f.inv_mass;
+    double2 *g = gall + f.goff;
     g[idx] = make_double2(-g1.x, -g1.y);
-    g[(size_t)Qb * Qc + idx] = make_double2(s * ev.y, -s * ev.x);
+    g[(size_t)Qb * Qc + idx] = make_double2(sm * ev.y, -sm * ev.x);
 }
 
-// H[s][ib][kc] = sum_ic g[s][ib][ic] Ec[kc][ic]
-__global__ void k_face_c(const double2 *__restrict__ g, const double2 *__restrict__ Ec, int Qb, int Qc, int nc,
-                         double2 *__restrict__ H) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 2 * Qb * nc) return;
-    const int s = idx / (Qb * nc), r = idx % (Qb * nc), ib = r / nc, kc = r % nc;
-    const double2 *gr = g + (size_t)s * Qb * Qc + (size_t)ib * Qc;
-    const double2 *er = Ec + (size_t)kc * Qc;
-    double2 acc = make_double2(0, 0);
-    for (int q = 0; q < Qc; ++q) {
-        const double2 a = gr[q], b = er[q];
-        acc.x += a.x * b.x - a.y * b.y;
-        acc.y += a.x * b.y + a.y * b.x;
+// The momentum contractions of every face (blockIdx.y), the same form twice:
+//   STAGE 0: H[s][kc][ib] = sum_ic g[s][ib][ic] Ec[kc][ic]
+//   STAGE 1: T[s][kb][kc] = sum_ib H[s][kc][ib] Eb[kb][ib]
+// `lanes` threads split the contracted index (contiguous in both operands)
+// and compute J momenta of one row; FP64 products, the partial sums reduced
+// by shuffles. One thread per output with the whole sum left a 2D face 256
+// serial chains of 1024 dependent FP64 products (515 us per face; 26 us for
+// all four faces split this way). J = 4 reuses the row operand where the
+// outputs fill the chip anyway, which halves the L2 reads of 3D faces.
+template <int STAGE, int J>
+__global__ void __launch_bounds__(256) k_face(const Faces fs, int lanes, const double2 *__restrict__ inall,
+                                              double2 *__restrict__ outall) {
+    const FaceParams &f = fs.f[blockIdx.y];
+    const int Q = STAGE == 0 ? f.c.Q : f.b.Q;
+    const int rows = STAGE == 0 ? f.b.Q : f.nc, nj = STAGE == 0 ? f.nc : f.nb;
+    const double2 *E = STAGE == 0 ? f.ec : f.eb;
+    const double2 *in = inall + (STAGE == 0 ? f.goff : f.hoff);
+    double2 *out = outall + (STAGE == 0 ? f.hoff : f.toff);
+    const int ng = (nj + J - 1) / J;
+    const long long gid = (blockIdx.x * (long long)blockDim.x + threadIdx.x) / lanes;
+    const int lane = threadIdx.x % lanes;
+    const bool valid = gid < 2LL * ng * rows;
+    const int r = (int)(gid % rows);
+    const int j0 = (int)((gid / rows) % ng) * J, s = (int)(gid / ((long long)rows * ng));
+    double2 acc[J];
+#pragma unroll
+    for (int j = 0; j < J; ++j) acc[j] = make_double2(0, 0);
+    if (valid) {
+        const double2 *ir = in + ((size_t)s * rows + r) * Q;
+        for (int q = lane; q < Q; q += lanes) {
+            const double2 a = ir[q];
+#pragma unroll
+            for (int j = 0; j < J; ++j) {
+                const double2 b = E[(size_t)min(j0 + j, nj - 1) * Q + q];
+                acc[j].x += a.x * b.x - a.y * b.y;
+                acc[j].y += a.x * b.y + a.y * b.x;
+            }
+        }
     }
-    H[idx] = acc;
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+        for (int o = lanes / 2; o > 0; o >>= 1) {
+            acc[j].x += __shfl_down_sync(0xffffffffu, acc[j].x, o);
+            acc[j].y += __shfl_down_sync(0xffffffffu, acc[j].y, o);
+        }
+    if (!valid || lane != 0) return;
+#pragma unroll
+    for (int j = 0; j < J; ++j)
+        if (j0 + j < nj) out[((size_t)s * nj + j0 + j) * rows + r] = acc[j];
 }
 
-// T[s][kb][kc] = sum_ib Eb[kb][ib] H[s][ib][kc]
-__global__ void k_face_b(const double2 *__restrict__ H, const double2 *__restrict__ Eb, int Qb, int nb, int nc,
-                         double2 *__restrict__ T) {
-    const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-    if (idx >= 2 * nb * nc) return;
-    const int s = idx / (nb * nc), r = idx % (nb * nc), kb = r / nc, kc = r % nc;
-    double2 acc = make_double2(0, 0);
-    for (int q = 0; q < Qb; ++q) {
-        const double2 a = Eb[(size_t)kb * Qb + q], b = H[(size_t)s * Qb * nc + (size_t)q * nc + kc];
-        acc.x += a.x * b.x - a.y * b.y;
-        acc.y += a.x * b.y + a.y * b.x;
-    }
-    T[idx] = acc;
-}
-
-struct KGrid {
-    int nk[3];
-    const double *k[3];
+struct Finish {
+    double2 pre;       // the common factor
+    double h;          // trapezoid weight
+    int have_prev;
 };
 
-// cur(k) += exp(-i (k_a + A_a) sigma R) (T_1 + (k_a + A_a) T_2)
-__global__ void k_face_acc(KGrid kg, int a, int b, int c, double Aa, double sigmaR, const double2 *__restrict__ T,
-                           double2 *__restrict__ cur, int first) {
-    const size_t tot = (size_t)kg.nk[0] * kg.nk[1] * kg.nk[2];
-    const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
-    if (idx >= tot) return;
-    int kk[3];
+// flux(k) = sum over faces of exp(-i (k_a + A_a) sigma R) (T_1 + (k_a + A_a) T_2),
+// faces 2 a and 2 a + 1 being the sides of axis a
+__device__ __forceinline__ double2 flux_at(const Faces &fs, const PhaseParams &pp, const int *kk, const double2 *Tall) {
+    double2 o = make_double2(0, 0);
+    int woff = 0;
+    for (int a = 0; 2 * a < fs.nf; ++a) {
+        const double2 ph = pp.wall[woff + kk[a]];
+        const double ka = pp.kg.k[a][kk[a]] + pp.A[a];
+        woff += pp.kg.nk[a];
+#pragma unroll
+        for (int side = 0; side < 2; ++side) {
+            const FaceParams &f = fs.f[2 * a + side];
+            const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
+            const double2 *T = Tall + f.toff;
+            const size_t e = (size_t)kk[b] * f.nc + kk[c];
+            const double2 t1 = T[e], t2 = T[(size_t)f.nb * f.nc + e];
+            const double2 v = cmul(make_double2(ph.x, side ? ph.y : -ph.y),
+                                   make_double2(t1.x + ka * t2.x, t1.y + ka * t2.y));
+            o.x += v.x;
+            o.y += v.y;
+        }
+    }
+    return o;
+}
+__device__ __forceinline__ void k_index(const KGrid &kg, size_t idx, int *kk) {
     kk[2] = (int)(idx % kg.nk[2]);
     kk[1] = (int)((idx / kg.nk[2]) % kg.nk[1]);
     kk[0] = (int)(idx / ((size_t)kg.nk[2] * kg.nk[1]));
-    const int nb = kg.nk[b], nc = kg.nk[c];
-    const double ka = kg.k[a][kk[a]] + Aa;
-    const double2 ph = cexpi(-ka * sigmaR);
-    const double2 t1 = T[(size_t)kk[b] * nc + kk[c]];
-    const double2 t2 = T[(size_t)nb * nc + (size_t)kk[b] * nc + kk[c]];
-    const double2 sum = make_double2(t1.x + ka * t2.x, t1.y + ka * t2.y);
-    const double2 v = cmul(ph, sum);
-    double2 o = first ? make_double2(0, 0) : cur[idx];
-    o.x += v.x;
-    o.y += v.y;
-    cur[idx] = o;
+}
+// pre times the Volkov factor prod_d exp(i (t k_d^2 / 2m + k_d B_d / m))
+__device__ __forceinline__ double2 volkov_at(const PhaseParams &pp, const int *kk, double2 pre) {
+    const int *nk = pp.kg.nk;
+    const double2 a = cmul(pre, pp.fin[kk[0]]);
+    return cmul(cmul(a, pp.fin[nk[0] + kk[1]]), pp.fin[nk[0] + nk[1] + kk[2]]);
 }
 
-// cur *= pre * prod_d exp(i (t k_d^2 / 2m + k_d B_d / m)); amp += h (prev + cur); prev = cur
-__global__ void k_finish(KGrid kg, double2 pre, double t, double inv2m, double invm, double B0, double B1,
-                         double B2, double h, int have_prev, double2 *cur, double2 *prev, double2 *amp) {
-    const size_t tot = (size_t)kg.nk[0] * kg.nk[1] * kg.nk[2];
+// one sample: c = pre Volkov(k) flux(k); amp += h (prev + c); prev = c
+__global__ void k_accumulate(const Faces fs, const PhaseParams pp, const double2 *__restrict__ T, Finish fin,
+                             double2 *prev, double2 *amp) {
+    const size_t tot = (size_t)pp.kg.nk[0] * pp.kg.nk[1] * pp.kg.nk[2];
     const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
     if (idx >= tot) return;
     int kk[3];
-    kk[2] = (int)(idx % kg.nk[2]);
-    kk[1] = (int)((idx / kg.nk[2]) % kg.nk[1]);
-    kk[0] = (int)(idx / ((size_t)kg.nk[2] * kg.nk[1]));
-    const double Bs[3] = {B0, B1, B2};
-    double phase = 0.0;
-    for (int d = 0; d < 3; ++d) {
-        const double k = kg.k[d][kk[d]];
-        phase += t * k * k * inv2m + k * Bs[d] * invm;
-    }
-    const double2 c = cmul(cmul(pre, cexpi(phase)), cur[idx]);
-    if (have_prev) {
+    k_index(pp.kg, idx, kk);
+    const double2 c = cmul(volkov_at(pp, kk, fin.pre), flux_at(fs, pp, kk, T));
+    if (fin.have_prev) {
         const double2 p = prev[idx];
         double2 a = amp[idx];
-        a.x += h * (p.x + c.x);
-        a.y += h * (p.y + c.y);
+        a.x += fin.h * (p.x + c.x);
+        a.y += fin.h * (p.y + c.y);
         amp[idx] = a;
     }
     prev[idx] = c;
+}
+
+// end term: amp[q_e] += w_e pre Volkov(k) flux(k); the entries of one node
+// name distinct momenta
+__global__ void k_end_acc(const Faces fs, const PhaseParams pp, const double2 *__restrict__ T, double2 pre,
+                          const int *__restrict__ q, const double *__restrict__ w, int m, double2 *__restrict__ amp) {
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= m) return;
+    const size_t idx = (size_t)q[e];
+    int kk[3];
+    k_index(pp.kg, idx, kk);
+    const double2 c = cmul(volkov_at(pp, kk, pre), flux_at(fs, pp, kk, T));
+    double2 a = amp[idx];
+    a.x += w[e] * c.x;
+    a.y += w[e] * c.y;
+    amp[idx] = a;
 }
 
 inline int blocks_for(size_t n, int t = 256) { return (int)((n + t - 1) / t); }
@@ -251,17 +346,18 @@ void TSurff::setup(const Space &s, const tdz_tsurff_opts &o, tdz_field_fn f, voi
         upload(T.ek, ek);
         nktot *= nk[d];
     }
-    size_t gmax = 0, hmax = 0, tmax = 0;
+    size_t gtot = 0, htot = 0, ttot = 0;   // work arrays of all 2 dim faces
     for (int a = 0; a < dim; ++a) {
         const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
-        gmax = std::max(gmax, (size_t)2 * ax[b].Q * ax[c].Q);
-        hmax = std::max(hmax, (size_t)2 * ax[b].Q * nk[c]);
-        tmax = std::max(tmax, (size_t)2 * nk[b] * nk[c]);
+        gtot += (size_t)4 * ax[b].Q * ax[c].Q;
+        htot += (size_t)4 * ax[b].Q * nk[c];
+        ttot += (size_t)4 * nk[b] * nk[c];
     }
-    g.alloc(gmax * sizeof(double2));
-    H.alloc(hmax * sizeof(double2));
-    T.alloc(tmax * sizeof(double2) * 2 * dim);
-    for (DevBuf *b : {&cur, &prev, &amp}) b->alloc(nktot * sizeof(double2));
+    g.alloc(gtot * sizeof(double2));
+    H.alloc(htot * sizeof(double2));
+    T.alloc(ttot * sizeof(double2));
+    tab.alloc((size_t)2 * (nk[0] + nk[1] + nk[2]) * sizeof(double2));
+    for (DevBuf *b : {&prev, &amp}) b->alloc(nktot * sizeof(double2));
     TDZ_CUDA(cudaMemset(amp.ptr, 0, nktot * sizeof(double2)));
     // wall values and node coordinates / weights per axis
     std::vector<double> wv, wd;
@@ -341,69 +437,134 @@ KGridHost TSurff::kgrid() const {
     return kg;
 }
 
-// cur(k) = the surface integral of the flux of psi against the Volkov states
-// at the current Volkov time, before the common factor (FluxGrid)
-void TSurff::surface_flux(const double2 *psi, cudaStream_t st) {
-    const double *xw = phase.as<double>();
+namespace {
+// smallest power of two >= v, at most 32: threads that share one sum of v terms
+inline int lanes_for(int v) {
+    int l = 1;
+    while (l < v && l < 32) l *= 2;
+    return l;
+}
+
+Faces make_faces(const TSurff &ts) {
+    const double *xw = ts.phase.as<double>();
     size_t xoff[3], woff[3], acc = 0;
-    for (int d = 0; d < 3; ++d) { xoff[d] = acc; acc += nodes[d].size(); }
-    for (int d = 0; d < 3; ++d) { woff[d] = acc; acc += weights[d].size(); }
-    const KGridHost kh = kgrid();
-    KGrid kg;
-    for (int d = 0; d < 3; ++d) { kg.nk[d] = kh.nk[d]; kg.k[d] = kh.k[d]; }
-    int first = 1;
-    for (int a = 0; a < dim; ++a)
+    for (int d = 0; d < 3; ++d) { xoff[d] = acc; acc += ts.nodes[d].size(); }
+    for (int d = 0; d < 3; ++d) { woff[d] = acc; acc += ts.weights[d].size(); }
+    Faces fs{};
+    fs.nf = 2 * ts.dim;
+    fs.inv_mass = 1.0 / ts.mass;
+    size_t go = 0, ho = 0, to = 0;
+    for (int a = 0; a < ts.dim; ++a)
         for (int side = 0; side < 2; ++side) {
             const int b = a == 0 ? 1 : 0, c = a == 2 ? 1 : 2;
-            FaceParams f;
-            f.b = {ax[b].n, ax[b].p, ax[b].Q, ax[b].off.as<int>(), ax[b].val.as<double>(), ax[b].der.as<double>()};
-            f.c = {ax[c].n, ax[c].p, ax[c].Q, ax[c].off.as<int>(), ax[c].val.as<double>(), ax[c].der.as<double>()};
+            FaceParams &f = fs.f[2 * a + side];
+            auto view = [&](int d) {
+                const auto &t = ts.ax[d];
+                return AxisView{t.n, t.p, t.Q, t.off.as<int>(), t.val.as<double>(), t.der.as<double>()};
+            };
+            f.b = view(b);
+            f.c = view(c);
             f.a = a;
             f.side = side;
             f.stride[0] = 1;
-            f.stride[1] = n[0];
-            f.stride[2] = n[0] * n[1];
-            f.wall_off = ax[a].wall_off[side];
-            f.pa = ax[a].p;
-            f.wval = wallv.as<double>() + (a * 2 + side) * 16;
-            f.wder = walld.as<double>() + (a * 2 + side) * 16;
+            f.stride[1] = ts.n[0];
+            f.stride[2] = ts.n[0] * ts.n[1];
+            f.wall_off = ts.ax[a].wall_off[side];
+            f.pa = ts.ax[a].p;
+            f.wval = ts.wallv.as<double>() + (a * 2 + side) * 16;
+            f.wder = ts.walld.as<double>() + (a * 2 + side) * 16;
             f.xb = xw + xoff[b];
             f.xc = xw + xoff[c];
             f.wb = xw + woff[b];
             f.wc = xw + woff[c];
-            f.Ab = A[b];
-            f.Ac = A[c];
-            f.inv_mass = 1.0 / mass;
-            f.sigma = side ? 1.0 : -1.0;
-            const int Qb = ax[b].Q, Qc = ax[c].Q;
-            k_trace<<<blocks_for((size_t)Qb * Qc), 256, 0, st>>>(f, psi, g.as<double2>());
-            k_face_c<<<blocks_for((size_t)2 * Qb * nk[c]), 256, 0, st>>>(g.as<double2>(), ax[c].ek.as<double2>(), Qb,
-                                                                        Qc, nk[c], H.as<double2>());
-            double2 *Tf = T.as<double2>();
-            k_face_b<<<blocks_for((size_t)2 * nk[b] * nk[c]), 256, 0, st>>>(H.as<double2>(), ax[b].ek.as<double2>(),
-                                                                            Qb, nk[b], nk[c], Tf);
-            k_face_acc<<<blocks_for(nktot), 256, 0, st>>>(kg, a, b, c, A[a], f.sigma * R, Tf, cur.as<double2>(), first);
-            first = 0;
-            TDZ_CUDA(cudaGetLastError());
-            count_launch(4);
+            f.Ab = ts.A[b];
+            f.Ac = ts.A[c];
+            f.nb = ts.nk[b];
+            f.nc = ts.nk[c];
+            f.eb = ts.ax[b].ek.as<double2>();
+            f.ec = ts.ax[c].ek.as<double2>();
+            f.goff = go;
+            f.hoff = ho;
+            f.toff = to;
+            go += (size_t)2 * f.b.Q * f.c.Q;
+            ho += (size_t)2 * f.b.Q * f.nc;
+            to += (size_t)2 * f.nb * f.nc;
         }
+    return fs;
 }
+
+PhaseParams make_phases(const TSurff &ts) {
+    PhaseParams pp{};
+    const KGridHost kh = ts.kgrid();
+    int tot = 0;
+    for (int d = 0; d < 3; ++d) {
+        pp.kg.nk[d] = kh.nk[d];
+        pp.kg.k[d] = kh.k[d];
+        pp.A[d] = ts.A[d];
+        pp.B[d] = ts.B[d];
+        tot += kh.nk[d];
+    }
+    pp.R = ts.R;
+    pp.t = ts.vt;
+    pp.inv2m = 0.5 / ts.mass;
+    pp.invm = 1.0 / ts.mass;
+    pp.wall = ts.tab.as<double2>();
+    pp.fin = pp.wall + tot;
+    return pp;
+}
+
+template <int STAGE> void contract_faces(const Faces &fs, const double2 *in, double2 *out, cudaStream_t st) {
+    int qmax = 1;
+    long long gmax1 = 0, gmax4 = 0;
+    for (int i = 0; i < fs.nf; ++i) {
+        const FaceParams &f = fs.f[i];
+        const long long rows = STAGE == 0 ? f.b.Q : f.nc, nj = STAGE == 0 ? f.nc : f.nb;
+        qmax = std::max(qmax, STAGE == 0 ? f.c.Q : f.b.Q);
+        gmax1 = std::max(gmax1, 2 * rows * nj);
+        gmax4 = std::max(gmax4, 2 * rows * ((nj + 3) / 4));
+    }
+    const int lanes = lanes_for(qmax);
+    // four momenta per group once that still leaves 16 warps per SM
+    const bool four = gmax4 * lanes * fs.nf >= (long long)16 * 32 * sm_count();
+    const dim3 grid(blocks_for((size_t)(four ? gmax4 : gmax1) * lanes), fs.nf);
+    if (four) k_face<STAGE, 4><<<grid, 256, 0, st>>>(fs, lanes, in, out);
+    else k_face<STAGE, 1><<<grid, 256, 0, st>>>(fs, lanes, in, out);
+    TDZ_CUDA(cudaGetLastError());
+    count_launch();
+}
+
+// T = the face contractions of psi at the current Volkov time (FluxGrid), and
+// the phase tables of the momentum grid
+void face_contractions(const TSurff &ts, const Faces &fs, const PhaseParams &pp, const double2 *psi, cudaStream_t st) {
+    int nodes = 1, nbc = 1;
+    for (int i = 0; i < fs.nf; ++i) {
+        nodes = std::max(nodes, fs.f[i].b.Q * fs.f[i].c.Q);
+        nbc = std::max(nbc, (fs.f[i].b.p + 1) * (fs.f[i].c.p + 1));
+    }
+    const int lanes = lanes_for(nbc);
+    const int kt = pp.kg.nk[0] + pp.kg.nk[1] + pp.kg.nk[2];
+    double2 *g = ts.g.as<double2>(), *H = ts.H.as<double2>();
+    k_trace<<<dim3(blocks_for(std::max((size_t)nodes * lanes, (size_t)kt)), fs.nf + 1), 256, 0, st>>>(fs, pp, lanes, psi, g);
+    TDZ_CUDA(cudaGetLastError());
+    count_launch();
+    // below 3D axis c is a single node and momentum with factor one: H = g
+    if (ts.dim == 3) contract_faces<0>(fs, g, H, st);
+    contract_faces<1>(fs, ts.dim == 3 ? H : g, ts.T.as<double2>(), st);
+}
+}  // namespace
 
 void TSurff::sample(double t, const double2 *psi, cudaStream_t st) {
     if (have_prev && t == prevT) return;
     TDZ_CHECK(!have_prev || t > prevT, TDZ_ERR_ARG, "t-SURFF sample times must increase");
     advance_volkov(t);
-    surface_flux(psi, st);
-    const KGridHost kh = kgrid();
-    KGrid kg;
-    for (int d = 0; d < 3; ++d) { kg.nk[d] = kh.nk[d]; kg.k[d] = kh.k[d]; }
+    const Faces fs = make_faces(*this);
+    const PhaseParams pp = make_phases(*this);
+    face_contractions(*this, fs, pp, psi, st);
     const double two_pi = 2.0 * std::acos(-1.0);
     const double pref = 0.5 * std::pow(two_pi, -0.5 * dim);
     // pre = (i/2) (2 pi)^{-d/2} exp(i C)
-    const double2 pre = make_double2(-pref * std::sin(C), pref * std::cos(C));
-    k_finish<<<blocks_for(nktot), 256, 0, st>>>(kg, pre, vt, 0.5 / mass, 1.0 / mass, B[0], B[1], B[2],
-                                                 0.5 * (t - prevT), have_prev ? 1 : 0, cur.as<double2>(),
-                                                 prev.as<double2>(), amp.as<double2>());
+    const Finish fin{make_double2(-pref * std::sin(C), pref * std::cos(C)), 0.5 * (t - prevT), have_prev ? 1 : 0};
+    k_accumulate<<<blocks_for(nktot), 256, 0, st>>>(fs, pp, T.as<double2>(), fin, prev.as<double2>(), amp.as<double2>());
     TDZ_CUDA(cudaGetLastError());
     count_launch();
     prevT = t;
@@ -411,43 +572,14 @@ void TSurff::sample(double t, const double2 *psi, cudaStream_t st) {
     ++samples;
 }
 
-namespace {
-// amp[q_e] += w_e pre exp(i (t |k|^2 / 2m + k.B / m)) cur[q_e]; the entries of
-// one node name distinct momenta
-__global__ void k_end_acc(KGrid kg, double2 pre, double t, double inv2m, double invm, double B0, double B1, double B2,
-                          const int *__restrict__ q, const double *__restrict__ w, int m,
-                          const double2 *__restrict__ cur, double2 *__restrict__ amp) {
-    const int e = blockIdx.x * blockDim.x + threadIdx.x;
-    if (e >= m) return;
-    const size_t idx = (size_t)q[e];
-    int kk[3];
-    kk[2] = (int)(idx % kg.nk[2]);
-    kk[1] = (int)((idx / kg.nk[2]) % kg.nk[1]);
-    kk[0] = (int)(idx / ((size_t)kg.nk[2] * kg.nk[1]));
-    const double Bs[3] = {B0, B1, B2};
-    double phase = 0.0;
-    for (int d = 0; d < 3; ++d) {
-        const double k = kg.k[d][kk[d]];
-        phase += t * k * k * inv2m + k * Bs[d] * invm;
-    }
-    const double2 c = cmul(cmul(pre, cexpi(phase)), cur[idx]);
-    double2 a = amp[idx];
-    a.x += w[e] * c.x;
-    a.y += w[e] * c.y;
-    amp[idx] = a;
-}
-}  // namespace
-
 void TSurff::add_weighted_flux(const double2 *phi, const int *q, const double *w, int m, cudaStream_t st) {
     if (m <= 0) return;
-    surface_flux(phi, st);
-    const KGridHost kh = kgrid();
-    KGrid kg;
-    for (int d = 0; d < 3; ++d) { kg.nk[d] = kh.nk[d]; kg.k[d] = kh.k[d]; }
+    const Faces fs = make_faces(*this);
+    const PhaseParams pp = make_phases(*this);
+    face_contractions(*this, fs, pp, phi, st);
     const double pref = 0.5 * std::pow(2.0 * std::acos(-1.0), -0.5 * dim);
     const double2 pre = make_double2(-pref * std::sin(C), pref * std::cos(C));
-    k_end_acc<<<blocks_for((size_t)m), 256, 0, st>>>(kg, pre, vt, 0.5 / mass, 1.0 / mass, B[0], B[1], B[2], q, w, m,
-                                                      cur.as<double2>(), amp_end.as<double2>());
+    k_end_acc<<<blocks_for((size_t)m), 256, 0, st>>>(fs, pp, T.as<double2>(), pre, q, w, m, amp_end.as<double2>());
     TDZ_CUDA(cudaGetLastError());
     count_launch();
 }

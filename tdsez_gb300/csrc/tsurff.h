@@ -55,8 +55,9 @@ struct TSurff {
     };
     std::array<AxisTables, 3> ax;
     DevBuf wallv, walld;                // per axis, side: p+1 values and derivatives at -R/+R
-    DevBuf g, H, T;                     // face work arrays
-    DevBuf cur, prev, amp;              // momentum arrays (complex)
+    DevBuf g, H, T;                     // work arrays of all faces
+    DevBuf tab;                         // per-axis momentum phases of the current sample
+    DevBuf prev, amp;                   // momentum arrays (complex)
     DevBuf phase;                       // node coordinates then weights (3 axes)
     DevBuf kdev;                        // momentum axes
     std::vector<double> kdev_host;
@@ -79,8 +80,6 @@ struct TSurff {
     void interior(const double2 *psi, std::vector<cd> &out, cudaStream_t st);
     void advance_volkov(double t);
     KGridHost kgrid() const;
-    // cur = the flux of psi at the current Volkov time without the common factor
-    void surface_flux(const double2 *psi, cudaStream_t st);
     void sample(double t, const double2 *psi, cudaStream_t st);
     // amp_end[q_e] += w_e flux(phi)(q_e) over m entries (q_e, w_e), the flux at
     // the last sample with its Volkov factor and no time weight
