@@ -302,8 +302,8 @@ struct ZSolveParams {
     float *x;               // in/out: real part of (line (i, j), row k) at x[k ks + j js + i is], imaginary at + cs
     size_t ks;
     int js, is, cs;
-    float2 *ck;             // scratch: elimination state at the start of each row block, [b][e][line]
-    float2 *zb;             // scratch: the band rows of Bc, then of Cc, [2][n2][bw]
+    float2 *ck;             // scratch: elimination state at the start of each row block, [half][b][e][line]
+    float4 *zb;             // scratch: upper band rows of (Bc, Cc) in elimination order, [half][row][P+1]
     const float *bands;     // outer base bands [nb][n2][bw]
     const float *lx, *ly;   // inner eigenvalues
     const float *lxi, *lyi; // their imaginary parts (complex axis pencils), else null
@@ -311,531 +311,329 @@ struct ZSolveParams {
     CombP<float> Bc, Cc;    // A_z(s) = Bc + s Cc
 };
 
-// One banded complex LU (no pivoting) + solve per line (i, j), one thread
-// per line, lines contiguous in memory (coalesced across the warp).
+// ---- line solves along the outer axis: banded complex L D L^T (no pivoting),
+// two threads per line, lines contiguous in memory (coalesced across the warp).
 //
-// The U factor is not stored. The forward pass runs the elimination and the
-// forward substitution down the line and saves only the elimination state
-// (the last P rows of U with their reciprocal pivots, and the last P entries
-// of L^-1 r) at the start of every block of ZBlk::B rows. The backward pass
-// walks the blocks bottom-up: from the block's saved state it redoes the
-// block's elimination (U rows into shared memory, L^-1 r into registers), then
-// back-substitutes the block and writes the solution in place. Per row that
-// is 8 bytes read and the state in the forward pass, 8 bytes read, 8 written
-// and the state in the backward pass (about 40 bytes for P = 3, against
-// 96 with a stored U), and no stores in the forward pass at all. The block's
-// right-hand side and state are prefetched into registers one block ahead;
-// the forward pass streams its rows kZDist ahead through asynchronous copies
-// into shared memory. The band rows of Bc and Cc are evaluated once per solve
-// (k_zbands) and copied into each CTA's shared memory.
-constexpr int kZDist = 32, kZThreads = 128;
+// The line matrices are complex symmetric (combinations of the mass,
+// stiffness, potential and absorbing bands with complex scalars), so one
+// triangle carries everything: row k needs its P+1 upper band entries, and
+// the multiplier of row k-d is u(k-d, k) / u(k-d, k-d).
+//
+// Twisted factorisation: one thread eliminates the first half of the rows from
+// the top, its partner the rest from the bottom (the line read backwards).
+// Each half's elimination keeps the band's columns past its end, so its last P
+// rows carry the coupling to the other half. The two final states meet in
+// shared memory, where both threads solve the same 2P x 2P system for the P
+// unknowns on either side of the cut: with the tail rows scaled by the
+// reciprocal pivots, U1 T1 + W1 T2 = c1 and U2 T2 + W2 T1 = c2 (U unit upper
+// triangular), so S T2 = c2 - W2 U1^-1 c1 with S = U2 - W2 U1^-1 W1, and
+// T1 = U1^-1 (c1 - W1 T2). Each thread then back-substitutes its half from the
+// partner's tail values.
+//
+// No factor is stored: the forward pass saves the elimination state (the live
+// parts of the last P rows) at the start of every block of B rows; the
+// backward pass redoes a block's elimination from it (u rows into shared
+// memory, L^-1 r into registers), back-substitutes and writes the solution in
+// place. Rows and states are fetched into registers one block ahead. Both
+// halves run the same number of full blocks (identity rows in front of the
+// first real row), so the row loop is fully unrolled with static ring slots
+// and a body short enough for the instruction cache.
+//
+// Bound by issue slots and the latency of the recursion (about 12 complex
+// multiply-subtracts per row and pass for P = 3). The former unsymmetric
+// elimination with a 32-row unrolled ring took 257 us per solve on 163 x 163
+// lines of 343 rows (P = 3) and 293 us on 260 lines of 260 rows (P = 4,
+// complex pencils); this one 97 us and 55 us.
+constexpr int kZLines = 64;                      // lines per CTA (two threads each)
 template <int P> struct ZBlk {
-    static constexpr int B = P <= 3 ? 16 : 8;        // rows per block (divides kZDist)
-    static constexpr int NS = P * (P + 1) + P;       // complex entries of the saved state
-    static_assert(B * (P + 1) >= kZDist, "the U block doubles as the forward pass's row ring");
+    static constexpr int B = P == 3 ? 9 : (P == 5 ? 10 : 8);   // rows per block (a multiple of P)
+    static constexpr int NS = P * (P + 1) / 2 + 2 * P;         // complex entries of the saved state
+    static constexpr int NX = P * (P + 1) + P;                 // complex entries exchanged at the cut
+    static_assert(B % P == 0, "ring slots are static within a block");
+    static_assert(NX <= B * (P + 1), "the u block doubles as the exchange buffer");
 };
-
-__device__ __forceinline__ void cp_async4(float *dst, const float *src) {
-    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
-                 : "memory");
-}
-__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
-template <int N> __device__ __forceinline__ void cp_async_wait() {
-    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
-}
+// rows of the upper half, blocks per half
+__host__ __device__ inline int z_half(int n) { return (n + 1) / 2; }
+__host__ __device__ inline int z_blocks(int n, int B) { return (z_half(n) + B - 1) / B; }
 
 template <int P> size_t zsolve_smem(int n2) {
-    return ((size_t)2 * n2 * (2 * P + 1) + (size_t)ZBlk<P>::B * (P + 1) * kZThreads) * sizeof(float2);
+    return (size_t)2 * z_blocks(n2, ZBlk<P>::B) * ZBlk<P>::B * (P + 1) * sizeof(float4) +
+           (size_t)ZBlk<P>::B * (P + 1) * 2 * kZLines * sizeof(float2);
 }
 
-// the band rows of A_z(s) = Bc + s Cc for the current stage: [2][n2][2P+1]
-__global__ void k_zbands(const ZSolveParams prm, int bw) {
-    const int n = prm.n2;
-    for (int e = blockIdx.x * blockDim.x + threadIdx.x; e < n * bw; e += gridDim.x * blockDim.x) {
-        const int k = e / bw, o = e % bw;
-        prm.zb[e] = comb_at<float, float2>(prm.Bc, prm.bands, n, bw, k, o);
-        prm.zb[(size_t)n * bw + e] = comb_at<float, float2>(prm.Cc, prm.bands, n, bw, k, o);
+// the upper band rows of A_z(s) = Bc + s Cc for the current stage, in the
+// elimination order of each half: entry q of local row k couples it to local
+// row k + q; identity rows in front
+template <int P> __global__ void k_zbands(const ZSolveParams prm) {
+    constexpr int B = ZBlk<P>::B, bw = 2 * P + 1;
+    const int n = prm.n2, rows = z_blocks(n, B) * B, h0 = z_half(n);
+    const int e = blockIdx.x * blockDim.x + threadIdx.x;
+    if (e >= 2 * rows * (P + 1)) return;
+    const int q = e % (P + 1), k = (e / (P + 1)) % rows, half = e / ((P + 1) * rows);
+    const int pad = rows - (half ? n - h0 : h0);
+    float2 b = make_float2(k < pad && q == 0 ? 1.f : 0.f, 0.f), c = make_float2(0.f, 0.f);
+    if (k >= pad) {
+        const int row = half ? n - 1 - (k - pad) : k - pad, col = half ? row - q : row + q;
+        if (col >= 0 && col < n) {
+            b = comb_at<float, float2>(prm.Bc, prm.bands, n, bw, row, col - row + P);
+            c = comb_at<float, float2>(prm.Cc, prm.bands, n, bw, row, col - row + P);
+        }
     }
+    prm.zb[e] = make_float4(b.x, b.y, c.x, c.y);
+}
+
+__device__ __forceinline__ float2 csubf(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
+// acc -= a b
+__device__ __forceinline__ void csubmul(float2 &acc, float2 a, float2 b) {
+    acc.x = fmaf(a.y, b.y, fmaf(-a.x, b.x, acc.x));
+    acc.y = fmaf(-a.y, b.x, fmaf(-a.x, b.y, acc.y));
 }
 
 template <int P, bool CI>
-__global__ void __launch_bounds__(kZThreads) k_zsolve(const ZSolveParams prm) {
-    constexpr int BWd = 2 * P + 1, B = ZBlk<P>::B, NS = ZBlk<P>::NS;
-    static_assert(kZDist % B == 0, "row blocks must tile the prefetch ring");
-    extern __shared__ float2 zs_smem[];
-    const int n = prm.n2;
-    float2 *sB = zs_smem, *sC = zs_smem + (size_t)n * BWd;          // band rows of Bc and Cc
-    float2 *sU = zs_smem + (size_t)2 * n * BWd;                      // [row of block][q][thread]
-    for (int e = threadIdx.x; e < 2 * n * BWd; e += blockDim.x) sB[e] = prm.zb[e];
+__global__ void __launch_bounds__(2 * kZLines, P <= 3 ? 3 : 2) k_zsolve(const ZSolveParams prm) {
+    constexpr int B = ZBlk<P>::B, NS = ZBlk<P>::NS, T = 2 * kZLines;
+    extern __shared__ float4 zs_smem[];
+    const int n = prm.n2, nb = z_blocks(n, B), rows = nb * B;
+    float4 *sZ = zs_smem;                                                   // [half][row][P+1]
+    float2 *sU = reinterpret_cast<float2 *>(zs_smem + (size_t)2 * rows * (P + 1));   // [slot][thread]
+    for (int e = threadIdx.x; e < 2 * rows * (P + 1); e += blockDim.x) sZ[e] = prm.zb[e];
     __syncthreads();
+    const int half = threadIdx.x / kZLines;        // 0: from the top, 1: from the bottom
+    const int li = threadIdx.x % kZLines;
     const int nl = prm.n0 * prm.n1;
-    const int l = blockIdx.x * blockDim.x + threadIdx.x;
-    if (l >= nl) return;
+    const int lraw = blockIdx.x * kZLines + li;
+    const bool valid = lraw < nl;
+    const int l = valid ? lraw : nl - 1;           // idle threads shadow a real line, store nothing
+    const int h0 = z_half(n), pad = rows - (half ? n - h0 : h0);
     const int i = l % prm.n0, j = l / prm.n0;
     const float s = prm.lx[i] + (prm.ly ? prm.ly[j] : 0.f);
     const float si = CI ? prm.lxi[i] + (prm.lyi ? prm.lyi[j] : 0.f) : 0.f;
-    float *xl = prm.x + (size_t)j * prm.js + (size_t)i * prm.is;
-    const size_t ks = prm.ks;
     const int cs = prm.cs;
-    auto ldx = [&](int k) { const float *q = xl + (size_t)k * ks; return make_float2(q[0], q[cs]); };
-    auto stx = [&](int k, float2 v) { float *q = xl + (size_t)k * ks; q[0] = v.x; q[cs] = v.y; };
-    float2 *ck = prm.ck + l;
+    // local row k at xl + k ks (rows below pad are identity rows, not in memory)
+    const long long ks = half ? -(long long)prm.ks : (long long)prm.ks;
+    float *xl = prm.x + (size_t)j * prm.js + (size_t)i * prm.is + (half ? (long long)(n - 1) * (long long)prm.ks : 0) -
+                (long long)pad * ks;
     const size_t cst = (size_t)nl;
+    float2 *ck = prm.ck + (size_t)half * nb * NS * cst + l;
+    const float4 *zt = sZ + (size_t)half * rows * (P + 1);
+    float2 *su = sU + threadIdx.x;
 
-    float2 Uw[P][P + 1];     // U rows k-1 .. k-P; [0] holds the reciprocal pivot
-    float2 yw[P];            // L^-1 r at rows k-1 .. k-P
+    // ring of the last P rows: u(k, k+1 .. k+P), the reciprocal pivot, L^-1 r
+    float2 U[P][P], iv[P], y[P];
     auto reset = [&]() {
 #pragma unroll
         for (int d = 0; d < P; ++d) {
-            yw[d] = make_float2(0.f, 0.f);
+            iv[d] = make_float2(1.f, 0.f);
+            y[d] = make_float2(0.f, 0.f);
 #pragma unroll
-            for (int q = 0; q <= P; ++q) Uw[d][q] = make_float2(1.f, 0.f);
+            for (int q = 0; q < P; ++q) U[d][q] = make_float2(0.f, 0.f);
         }
     };
-    // row k: eliminate columns k-P .. k-1 with the U rows in Uw; shifts the
-    // new U row into Uw[0] and L^-1 r into yw[0]
-    auto eliminate = [&](int k, float2 rhs) {
-        float2 a[BWd];
+    // local row b B + r into ring slot r % P
+    auto eliminate = [&](const float4 *zr, int r, float2 rhs) {
+        float2 a[P + 1];
 #pragma unroll
-        for (int o = 0; o < BWd; ++o) {
-            const float2 b = sB[k * BWd + o], c = sC[k * BWd + o];
-            a[o] = CI ? make_float2(fmaf(-si, c.y, fmaf(s, c.x, b.x)), fmaf(si, c.x, fmaf(s, c.y, b.y)))
-                      : make_float2(fmaf(s, c.x, b.x), fmaf(s, c.y, b.y));
+        for (int q = 0; q <= P; ++q) {
+            const float4 z = zr[r * (P + 1) + q];
+            a[q] = CI ? make_float2(fmaf(-si, z.w, fmaf(s, z.z, z.x)), fmaf(si, z.z, fmaf(s, z.w, z.y)))
+                      : make_float2(fmaf(s, z.z, z.x), fmaf(s, z.w, z.y));
         }
 #pragma unroll
         for (int d = P; d >= 1; --d) {
-            if (k - d < 0) continue;
-            const float2 *Ur = Uw[d - 1];   // row k-d: Ur[q] = U(k-d, k-d+q), Ur[0] = 1 / U(k-d, k-d)
-            const float2 f = cmulf(a[P - d], Ur[0]);
+            const int o = (r + P - d) % P;          // slot of row k - d
+            const float2 f = cmulf(U[o][d - 1], iv[o]);
 #pragma unroll
-            for (int q = 1; q <= P; ++q) {
-                const float2 t = cmulf(f, Ur[q]);
-                a[P - d + q].x -= t.x;
-                a[P - d + q].y -= t.y;
-            }
-            const float2 t = cmulf(f, yw[d - 1]);
-            rhs.x -= t.x;
-            rhs.y -= t.y;
+            for (int q = 0; q + d <= P; ++q) csubmul(a[q], f, U[o][d + q - 1]);
+            csubmul(rhs, f, y[o]);
         }
-        a[P] = crecf(a[P]);
+        const int o = r % P;
+        iv[o] = crecf(a[0]);
+        y[o] = rhs;
 #pragma unroll
-        for (int d = P - 1; d > 0; --d) {
-            yw[d] = yw[d - 1];
-#pragma unroll
-            for (int q = 0; q <= P; ++q) Uw[d][q] = Uw[d - 1][q];
-        }
-#pragma unroll
-        for (int q = 0; q <= P; ++q) Uw[0][q] = a[P + q];
-        yw[0] = rhs;
+        for (int q = 0; q < P; ++q) U[o][q] = a[q + 1];
     };
-
-    // forward pass: the state at the start of blocks 1 .. nb-1. The rows
-    // stream through a kZDist-deep ring in shared memory (this thread's
-    // column of the U block, free until the backward pass) filled by
-    // asynchronous copies, one commit group per row, so kZDist rows are
-    // always in flight whatever the compiler's schedule.
-    reset();
-    {
-        float *ring = reinterpret_cast<float *>(sU + threadIdx.x);   // slot u: ring[2 u kZThreads + {0, 1}]
-        auto issue = [&](int k, int u) {
-            if (k < n) {
-                const float *q = xl + (size_t)k * ks;
-                cp_async4(ring + (size_t)2 * u * kZThreads, q);
-                cp_async4(ring + (size_t)2 * u * kZThreads + 1, q + cs);
-            }
-            cp_async_commit();
-        };
-#pragma unroll
-        for (int u = 0; u < kZDist; ++u) issue(u, u);
-        for (int k0 = 0; k0 < n; k0 += kZDist) {
-#pragma unroll
-            for (int u = 0; u < kZDist; ++u) {
-                const int k = k0 + u;
-                if (k < n) {
-                    if (u % B == 0 && k > 0) {
-                        float2 *c = ck + (size_t)(k / B) * NS * cst;
-#pragma unroll
-                        for (int d = 0; d < P; ++d) {
-#pragma unroll
-                            for (int q = 0; q <= P; ++q) c[(size_t)(d * (P + 1) + q) * cst] = Uw[d][q];
-                            c[(size_t)(P * (P + 1) + d) * cst] = yw[d];
-                        }
-                    }
-                    cp_async_wait<kZDist - 1>();   // row k has landed
-                    const float2 rhs = *reinterpret_cast<const float2 *>(ring + (size_t)2 * u * kZThreads);
-                    issue(k + kZDist, u);
-                    eliminate(k, rhs);
-                }
-            }
-        }
-        cp_async_wait<0>();
-    }
-
-    // backward pass, blocks nb-1 .. 0; a block's rows and saved state are
-    // loaded into registers one block ahead
-    const int nb = (n + B - 1) / B;
-    float2 nr[B], nst[NS];
+    // rows of block b (only block 0 has identity rows)
+    float2 nr[B];
     auto fetch = [&](int b) {
 #pragma unroll
         for (int r = 0; r < B; ++r) {
             const int k = b * B + r;
-            nr[r] = k < n ? ldx(k) : make_float2(0.f, 0.f);
-        }
-        if (b > 0) {
-            const float2 *c = ck + (size_t)b * NS * cst;
-#pragma unroll
-            for (int e = 0; e < NS; ++e) nst[e] = c[(size_t)e * cst];
+            nr[r] = make_float2(0.f, 0.f);
+            if (k >= pad) {
+                const float *q = xl + (long long)k * ks;
+                nr[r] = make_float2(q[0], q[cs]);
+            }
         }
     };
-    float2 xw[P];
+    // the live part of the state at the start of a block: row k-d (slot P-d)
+    // still needs u(k-d, k .. k-d+P), its pivot and L^-1 r
+    auto save = [&](int b) {
+        float2 *c = ck + (size_t)b * NS * cst;
+        int e = 0;
 #pragma unroll
-    for (int d = 0; d < P; ++d) xw[d] = make_float2(0.f, 0.f);
-    float2 *su = sU + threadIdx.x;
-    fetch(nb - 1);
-    for (int b = nb - 1; b >= 0; --b) {
+        for (int d = 1; d <= P; ++d) {
+#pragma unroll
+            for (int q = d; q <= P; ++q) c[(size_t)(e++) * cst] = U[P - d][q - 1];
+            c[(size_t)(e++) * cst] = iv[P - d];
+            c[(size_t)(e++) * cst] = y[P - d];
+        }
+    };
+
+    // forward pass of this half
+    reset();
+    fetch(0);
+    for (int b = 0; b < nb; ++b) {
         float2 rr[B];
 #pragma unroll
         for (int r = 0; r < B; ++r) rr[r] = nr[r];
-        if (b > 0) {
+        if (b + 1 < nb) fetch(b + 1);
+        if (b > 0 && valid) save(b);
+        const float4 *zr = zt + (size_t)b * B * (P + 1);
 #pragma unroll
-            for (int d = 0; d < P; ++d) {
-#pragma unroll
-                for (int q = 0; q <= P; ++q) Uw[d][q] = nst[d * (P + 1) + q];
-                yw[d] = nst[P * (P + 1) + d];
-            }
-        } else {
-            reset();
-        }
-        if (b > 0) fetch(b - 1);
-        // redo the block's elimination
-        float2 yb[B];
-#pragma unroll
-        for (int r = 0; r < B; ++r) {
-            const int k = b * B + r;
-            yb[r] = make_float2(0.f, 0.f);
-            if (k < n) {
-                eliminate(k, rr[r]);
-                yb[r] = yw[0];
-#pragma unroll
-                for (int q = 0; q <= P; ++q) su[(size_t)(r * (P + 1) + q) * kZThreads] = Uw[0][q];
-            }
-        }
-        // back substitution of the block
-#pragma unroll
-        for (int r = B - 1; r >= 0; --r) {
-            const int k = b * B + r;
-            if (k < n) {
-                float2 v = yb[r];
-#pragma unroll
-                for (int q = 1; q <= P; ++q) {
-                    if (k + q >= n) continue;
-                    const float2 t = cmulf(su[(size_t)(r * (P + 1) + q) * kZThreads], xw[q - 1]);
-                    v.x -= t.x;
-                    v.y -= t.y;
-                }
-                v = cmulf(v, su[(size_t)(r * (P + 1)) * kZThreads]);
-#pragma unroll
-                for (int d = P - 1; d > 0; --d) xw[d] = xw[d - 1];
-                xw[0] = v;
-                stx(k, v);
-            }
-        }
-    }
-}
-
-// ---- twisted line solve: two threads per line
-// The line is cut at the twist m (a multiple of the block length). One thread
-// factors rows 0 .. m-1 from the top, its partner rows n-1 .. m from the
-// bottom (the same elimination on the reversed line: for a complex-symmetric
-// band matrix, row k read backwards). Each half's elimination runs over the
-// band's columns past its end too, so its last P rows of U carry the
-// coupling to the other half. The two final elimination states meet in shared
-// memory, where both threads solve the same 2P x 2P system for the P unknowns
-// on either side of the twist: with the tail rows scaled by the reciprocal
-// pivots, U1 T1 + W1 T2 = c1 and U2 T2 + W2 T1 = c2 (U unit upper
-// triangular), so S T2 = c2 - W2 U1^-1 c1 with S = U2 - W2 U1^-1 W1, and
-// T1 = U1^-1 (c1 - W1 T2). Each thread then back-substitutes its half from the
-// partner's tail values. This doubles the threads of the latency-bound
-// recursion and halves its length.
-constexpr int kZ2Lines = 64;                     // lines per CTA (two threads each)
-template <int P> struct ZBlk2 {
-    static constexpr int B = P == 2 ? 16 : 8;    // rows per block
-    static constexpr int NS = P * (P + 1) + P;
-    static_assert(B * (P + 1) >= kZDist, "the U block doubles as the row ring");
-    static_assert(NS <= B * (P + 1), "the U block doubles as the exchange buffer");
-};
-
-template <int P> size_t zsolve2_smem(int n2) {
-    return ((size_t)2 * n2 * (2 * P + 1) + (size_t)ZBlk2<P>::B * (P + 1) * 2 * kZ2Lines) * sizeof(float2);
-}
-__host__ __device__ inline int zsolve2_twist(int n2, int B) { return B * ((n2 + B) / (2 * B)); }
-
-__device__ __forceinline__ float2 csubf(float2 a, float2 b) { return make_float2(a.x - b.x, a.y - b.y); }
-
-template <int P, bool CI>
-__global__ void __launch_bounds__(2 * kZ2Lines) k_zsolve2(const ZSolveParams prm) {
-    constexpr int BWd = 2 * P + 1, B = ZBlk2<P>::B, NS = ZBlk2<P>::NS, T = 2 * kZ2Lines;
-    static_assert(kZDist % B == 0, "row blocks must tile the prefetch ring");
-    extern __shared__ float2 zs_smem[];
-    const int n = prm.n2;
-    float2 *sB = zs_smem, *sC = zs_smem + (size_t)n * BWd;
-    float2 *sU = zs_smem + (size_t)2 * n * BWd;   // [slot][thread]: row ring, exchange, U block
-    for (int e = threadIdx.x; e < 2 * n * BWd; e += blockDim.x) sB[e] = prm.zb[e];
-    __syncthreads();
-    const int half = threadIdx.x / kZ2Lines;       // 0: rows 0 .. m-1, 1: rows n-1 .. m
-    const int li = threadIdx.x % kZ2Lines;
-    const int nl = prm.n0 * prm.n1;
-    const int lraw = blockIdx.x * kZ2Lines + li;
-    const bool valid = lraw < nl;
-    const int l = valid ? lraw : nl - 1;           // idle threads shadow a real line, store nothing
-    const int m = zsolve2_twist(n, B);
-    const int L = half ? n - m : m;                // rows of this half
-    const int i = l % prm.n0, j = l / prm.n0;
-    const float s = prm.lx[i] + (prm.ly ? prm.ly[j] : 0.f);
-    const float si = CI ? prm.lxi[i] + (prm.lyi ? prm.lyi[j] : 0.f) : 0.f;
-    float *xl = prm.x + (size_t)j * prm.js + (size_t)i * prm.is;
-    const size_t ks = prm.ks;
-    const int cs = prm.cs;
-    auto phys = [&](int k) { return half ? n - 1 - k : k; };
-    auto ldx = [&](int k) { const float *q = xl + (size_t)phys(k) * ks; return make_float2(q[0], q[cs]); };
-    auto stx = [&](int k, float2 v) {
-        if (valid) {
-            float *q = xl + (size_t)phys(k) * ks;
-            q[0] = v.x;
-            q[cs] = v.y;
-        }
-    };
-    const size_t cst = (size_t)nl;
-    float2 *ck = prm.ck + (size_t)(half ? (m + B - 1) / B : 0) * NS * cst + l;
-
-    float2 Uw[P][P + 1];
-    float2 yw[P];
-    auto reset = [&]() {
-#pragma unroll
-        for (int d = 0; d < P; ++d) {
-            yw[d] = make_float2(0.f, 0.f);
-#pragma unroll
-            for (int q = 0; q <= P; ++q) Uw[d][q] = make_float2(1.f, 0.f);
-        }
-    };
-    // local row k of this half (its band row read backwards in the bottom half)
-    auto eliminate = [&](int k, float2 rhs) {
-        float2 a[BWd];
-        const int pr = phys(k);
-#pragma unroll
-        for (int o = 0; o < BWd; ++o) {
-            const int oo = half ? 2 * P - o : o;
-            const float2 b = sB[pr * BWd + oo], c = sC[pr * BWd + oo];
-            a[o] = CI ? make_float2(fmaf(-si, c.y, fmaf(s, c.x, b.x)), fmaf(si, c.x, fmaf(s, c.y, b.y)))
-                      : make_float2(fmaf(s, c.x, b.x), fmaf(s, c.y, b.y));
-        }
-#pragma unroll
-        for (int d = P; d >= 1; --d) {
-            if (k - d < 0) continue;
-            const float2 *Ur = Uw[d - 1];
-            const float2 f = cmulf(a[P - d], Ur[0]);
-#pragma unroll
-            for (int q = 1; q <= P; ++q) {
-                const float2 t = cmulf(f, Ur[q]);
-                a[P - d + q].x -= t.x;
-                a[P - d + q].y -= t.y;
-            }
-            const float2 t = cmulf(f, yw[d - 1]);
-            rhs.x -= t.x;
-            rhs.y -= t.y;
-        }
-        a[P] = crecf(a[P]);
-#pragma unroll
-        for (int d = P - 1; d > 0; --d) {
-            yw[d] = yw[d - 1];
-#pragma unroll
-            for (int q = 0; q <= P; ++q) Uw[d][q] = Uw[d - 1][q];
-        }
-#pragma unroll
-        for (int q = 0; q <= P; ++q) Uw[0][q] = a[P + q];
-        yw[0] = rhs;
-    };
-
-    // forward pass of this half, rows streamed through the ring
-    reset();
-    {
-        float *ring = reinterpret_cast<float *>(sU + threadIdx.x);
-        auto issue = [&](int k, int u) {
-            if (k < L) {
-                const float *q = xl + (size_t)phys(k) * ks;
-                cp_async4(ring + (size_t)2 * u * T, q);
-                cp_async4(ring + (size_t)2 * u * T + 1, q + cs);
-            }
-            cp_async_commit();
-        };
-#pragma unroll
-        for (int u = 0; u < kZDist; ++u) issue(u, u);
-        for (int k0 = 0; k0 < L; k0 += kZDist) {
-#pragma unroll
-            for (int u = 0; u < kZDist; ++u) {
-                const int k = k0 + u;
-                if (k < L) {
-                    if (u % B == 0 && k > 0 && valid) {
-                        float2 *c = ck + (size_t)(k / B) * NS * cst;
-#pragma unroll
-                        for (int d = 0; d < P; ++d) {
-#pragma unroll
-                            for (int q = 0; q <= P; ++q) c[(size_t)(d * (P + 1) + q) * cst] = Uw[d][q];
-                            c[(size_t)(P * (P + 1) + d) * cst] = yw[d];
-                        }
-                    }
-                    cp_async_wait<kZDist - 1>();
-                    const float2 rhs = *reinterpret_cast<const float2 *>(ring + (size_t)2 * u * T);
-                    issue(k + kZDist, u);
-                    eliminate(k, rhs);
-                }
-            }
-        }
-        cp_async_wait<0>();
+        for (int r = 0; r < B; ++r) eliminate(zr, r, rr[r]);
     }
 
-    // exchange the final states and solve the twist system (same arithmetic in both threads)
+    // exchange the final states ([d-1]: the row d places from the end) and
+    // solve the twist system (same arithmetic in both threads)
     float2 *ex = sU;   // [e][thread]
 #pragma unroll
     for (int d = 0; d < P; ++d) {
+        const int o = P - 1 - d;
+        ex[(size_t)(d * (P + 1)) * T + threadIdx.x] = iv[o];
 #pragma unroll
-        for (int q = 0; q <= P; ++q) ex[(size_t)(d * (P + 1) + q) * T + threadIdx.x] = Uw[d][q];
-        ex[(size_t)(P * (P + 1) + d) * T + threadIdx.x] = yw[d];
+        for (int q = 1; q <= P; ++q) ex[(size_t)(d * (P + 1) + q) * T + threadIdx.x] = U[o][q - 1];
+        ex[(size_t)(P * (P + 1) + d) * T + threadIdx.x] = y[o];
     }
     __syncthreads();
-    float2 U1[P][P], W1[P][P], c1[P], U2[P][P], W2[P][P], c2[P];
-    auto tail = [&](int col, float2 (&U)[P][P], float2 (&W)[P][P], float2 (&c)[P]) {
-        auto st = [&](int e) { return ex[(size_t)e * T + col]; };
+    float2 T1[P], T2[P];
+    {
+        float2 U1[P][P], W1[P][P], c1[P], U2[P][P], W2[P][P], c2[P];
+        auto tail = [&](int col, float2 (&Um)[P][P], float2 (&W)[P][P], float2 (&c)[P]) {
+            auto st = [&](int e) { return ex[(size_t)e * T + col]; };
+#pragma unroll
+            for (int r = 0; r < P; ++r) {
+                const int d = P - 1 - r;
+                const float2 rp = st(d * (P + 1));
+#pragma unroll
+                for (int k = 0; k < P; ++k) {
+                    Um[r][k] = k > r ? cmulf(rp, st(d * (P + 1) + (k - r))) : make_float2(0.f, 0.f);
+                    W[r][k] = k >= P - 1 - r ? cmulf(rp, st(d * (P + 1) + (2 * P - 1 - r - k))) : make_float2(0.f, 0.f);
+                }
+                c[r] = cmulf(rp, st(P * (P + 1) + d));
+            }
+        };
+        tail(li, U1, W1, c1);
+        tail(li + kZLines, U2, W2, c2);
+        __syncthreads();   // the exchange buffer is this thread's u block from here on
+        // z1 = U1^-1 c1, M1 = U1^-1 W1 (unit upper triangular)
+        float2 z1[P], M1[P][P];
+#pragma unroll
+        for (int r = P - 1; r >= 0; --r) {
+            z1[r] = c1[r];
+#pragma unroll
+            for (int k = 0; k < P; ++k) M1[r][k] = W1[r][k];
+#pragma unroll
+            for (int q = r + 1; q < P; ++q) {
+                z1[r] = csubf(z1[r], cmulf(U1[r][q], z1[q]));
+#pragma unroll
+                for (int k = 0; k < P; ++k) M1[r][k] = csubf(M1[r][k], cmulf(U1[r][q], M1[q][k]));
+            }
+        }
+        // S = U2 + I - W2 M1 (U2 holds the strict upper part), g = c2 - W2 z1
+        float2 S[P][P], g[P];
 #pragma unroll
         for (int r = 0; r < P; ++r) {
-            const int d = P - 1 - r;
-            const float2 rp = st(d * (P + 1));
+            g[r] = c2[r];
 #pragma unroll
-            for (int k = 0; k < P; ++k) {
-                U[r][k] = k > r ? cmulf(rp, st(d * (P + 1) + (k - r))) : make_float2(0.f, 0.f);
-                W[r][k] = k >= P - 1 - r ? cmulf(rp, st(d * (P + 1) + (2 * P - 1 - r - k))) : make_float2(0.f, 0.f);
+            for (int k = 0; k < P; ++k) S[r][k] = k == r ? make_float2(1.f, 0.f) : U2[r][k];
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                g[r] = csubf(g[r], cmulf(W2[r][q], z1[q]));
+#pragma unroll
+                for (int k = 0; k < P; ++k) S[r][k] = csubf(S[r][k], cmulf(W2[r][q], M1[q][k]));
             }
-            c[r] = cmulf(rp, st(P * (P + 1) + d));
         }
-    };
-    tail(li, U1, W1, c1);
-    tail(li + kZ2Lines, U2, W2, c2);
-    __syncthreads();   // the exchange buffer is this thread's U block from here on
-    // z1 = U1^-1 c1, M1 = U1^-1 W1 (unit upper triangular)
-    float2 z1[P], M1[P][P];
+        // S T2 = g: Gaussian elimination without pivoting, then T1 = z1 - M1 T2
 #pragma unroll
-    for (int r = P - 1; r >= 0; --r) {
-        z1[r] = c1[r];
+        for (int c = 0; c < P; ++c) {
+            const float2 inv = crecf(S[c][c]);
 #pragma unroll
-        for (int k = 0; k < P; ++k) M1[r][k] = W1[r][k];
+            for (int r = c + 1; r < P; ++r) {
+                const float2 f = cmulf(S[r][c], inv);
 #pragma unroll
-        for (int q = r + 1; q < P; ++q) {
-            z1[r] = csubf(z1[r], cmulf(U1[r][q], z1[q]));
-#pragma unroll
-            for (int k = 0; k < P; ++k) M1[r][k] = csubf(M1[r][k], cmulf(U1[r][q], M1[q][k]));
+                for (int k = c + 1; k < P; ++k) S[r][k] = csubf(S[r][k], cmulf(f, S[c][k]));
+                g[r] = csubf(g[r], cmulf(f, g[c]));
+            }
+            S[c][c] = inv;
         }
-    }
-    // S = U2 + I - W2 M1 (U2 holds the strict upper part), g = c2 - W2 z1
-    float2 S[P][P], g[P];
 #pragma unroll
-    for (int r = 0; r < P; ++r) {
-        g[r] = c2[r];
+        for (int r = P - 1; r >= 0; --r) {
+            float2 v = g[r];
 #pragma unroll
-        for (int k = 0; k < P; ++k) S[r][k] = k == r ? make_float2(1.f, 0.f) : U2[r][k];
-#pragma unroll
-        for (int q = 0; q < P; ++q) {
-            g[r] = csubf(g[r], cmulf(W2[r][q], z1[q]));
-#pragma unroll
-            for (int k = 0; k < P; ++k) S[r][k] = csubf(S[r][k], cmulf(W2[r][q], M1[q][k]));
+            for (int k = r + 1; k < P; ++k) v = csubf(v, cmulf(S[r][k], T2[k]));
+            T2[r] = cmulf(v, S[r][r]);
         }
-    }
-    // S T2 = g: Gaussian elimination without pivoting, then T1 = z1 - M1 T2
 #pragma unroll
-    for (int c = 0; c < P; ++c) {
-        const float2 inv = crecf(S[c][c]);
+        for (int r = 0; r < P; ++r) {
+            T1[r] = z1[r];
 #pragma unroll
-        for (int r = c + 1; r < P; ++r) {
-            const float2 f = cmulf(S[r][c], inv);
-#pragma unroll
-            for (int k = c + 1; k < P; ++k) S[r][k] = csubf(S[r][k], cmulf(f, S[c][k]));
-            g[r] = csubf(g[r], cmulf(f, g[c]));
+            for (int k = 0; k < P; ++k) T1[r] = csubf(T1[r], cmulf(M1[r][k], T2[k]));
         }
-        S[c][c] = inv;
-    }
-    float2 T2[P], T1[P];
-#pragma unroll
-    for (int r = P - 1; r >= 0; --r) {
-        float2 v = g[r];
-#pragma unroll
-        for (int k = r + 1; k < P; ++k) v = csubf(v, cmulf(S[r][k], T2[k]));
-        T2[r] = cmulf(v, S[r][r]);
-    }
-#pragma unroll
-    for (int r = 0; r < P; ++r) {
-        T1[r] = z1[r];
-#pragma unroll
-        for (int k = 0; k < P; ++k) T1[r] = csubf(T1[r], cmulf(M1[r][k], T2[k]));
     }
 
-    // backward pass of this half; row L + c of this half is the partner's tail row P-1-c
-    const int nb = (L + B - 1) / B;
-    float2 nr[B], nst[NS];
-    auto fetch = [&](int b) {
+    // backward pass of this half; local row rows + c is the partner's tail row P-1-c
+    float2 nst[NS];
+    auto fetch_state = [&](int b) {
+        const float2 *c = ck + (size_t)b * NS * cst;
 #pragma unroll
-        for (int r = 0; r < B; ++r) {
-            const int k = b * B + r;
-            nr[r] = k < L ? ldx(k) : make_float2(0.f, 0.f);
-        }
-        if (b > 0) {
-            const float2 *c = ck + (size_t)b * NS * cst;
-#pragma unroll
-            for (int e = 0; e < NS; ++e) nst[e] = c[(size_t)e * cst];
-        }
+        for (int e = 0; e < NS; ++e) nst[e] = c[(size_t)e * cst];
     };
     float2 xw[P];
 #pragma unroll
     for (int c = 0; c < P; ++c) xw[c] = half ? T1[P - 1 - c] : T2[P - 1 - c];
-    float2 *su = sU + threadIdx.x;
     fetch(nb - 1);
+    if (nb > 1) fetch_state(nb - 1);
     for (int b = nb - 1; b >= 0; --b) {
-        float2 rr[B];
-#pragma unroll
-        for (int r = 0; r < B; ++r) rr[r] = nr[r];
-        if (b > 0) {
-#pragma unroll
-            for (int d = 0; d < P; ++d) {
-#pragma unroll
-                for (int q = 0; q <= P; ++q) Uw[d][q] = nst[d * (P + 1) + q];
-                yw[d] = nst[P * (P + 1) + d];
-            }
-        } else {
-            reset();
-        }
-        if (b > 0) fetch(b - 1);
         float2 yb[B];
 #pragma unroll
-        for (int r = 0; r < B; ++r) {
-            const int k = b * B + r;
-            yb[r] = make_float2(0.f, 0.f);
-            if (k < L) {
-                eliminate(k, rr[r]);
-                yb[r] = yw[0];
+        for (int r = 0; r < B; ++r) yb[r] = nr[r];
+        reset();
+        if (b > 0) {
+            int e = 0;
 #pragma unroll
-                for (int q = 0; q <= P; ++q) su[(size_t)(r * (P + 1) + q) * T] = Uw[0][q];
+            for (int d = 1; d <= P; ++d) {
+#pragma unroll
+                for (int q = d; q <= P; ++q) U[P - d][q - 1] = nst[e++];
+                iv[P - d] = nst[e++];
+                y[P - d] = nst[e++];
             }
+            fetch(b - 1);
+            if (b > 1) fetch_state(b - 1);
+        }
+        // redo the block's elimination
+        const float4 *zr = zt + (size_t)b * B * (P + 1);
+#pragma unroll
+        for (int r = 0; r < B; ++r) {
+            eliminate(zr, r, yb[r]);
+            yb[r] = y[r % P];
+            su[(size_t)(r * (P + 1)) * T] = iv[r % P];
+#pragma unroll
+            for (int q = 1; q <= P; ++q) su[(size_t)(r * (P + 1) + q) * T] = U[r % P][q - 1];
         }
 #pragma unroll
         for (int r = B - 1; r >= 0; --r) {
+            float2 v = yb[r];
+#pragma unroll
+            for (int q = P; q >= 1; --q) csubmul(v, su[(size_t)(r * (P + 1) + q) * T], xw[q - 1]);
+            v = cmulf(v, su[(size_t)(r * (P + 1)) * T]);
+#pragma unroll
+            for (int d = P - 1; d > 0; --d) xw[d] = xw[d - 1];
+            xw[0] = v;
             const int k = b * B + r;
-            if (k < L) {
-                float2 v = yb[r];
-#pragma unroll
-                for (int q = 1; q <= P; ++q) v = csubf(v, cmulf(su[(size_t)(r * (P + 1) + q) * T], xw[q - 1]));
-                v = cmulf(v, su[(size_t)(r * (P + 1)) * T]);
-#pragma unroll
-                for (int d = P - 1; d > 0; --d) xw[d] = xw[d - 1];
-                xw[0] = v;
-                stx(k, v);
+            if (valid && k >= pad) {
+                float *q = xl + (long long)k * ks;
+                q[0] = v.x;
+                q[cs] = v.y;
             }
         }
     }
@@ -848,22 +646,16 @@ template <int P, bool CI> void launch_zsolve_t(const ZSolveParams &zp, cudaStrea
     // that solves of different lengths from several host threads cannot
     // lower it under each other's launches
     static const bool attr = [] {
-        TDZ_CUDA(cudaFuncSetAttribute(k_zsolve2<P, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
         TDZ_CUDA(cudaFuncSetAttribute(k_zsolve<P, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
         return true;
     }();
     (void)attr;
     const int nl = zp.n0 * zp.n1;
-    k_zbands<<<(zp.n2 * (2 * P + 1) + 255) / 256, 256, 0, st>>>(zp, 2 * P + 1);
-    if (zp.n2 >= 4 * ZBlk2<P>::B) {
-        const size_t smem = zsolve2_smem<P>(zp.n2);
-        TDZ_CHECK(smem <= kMax, TDZ_ERR_UNSUPPORTED, "outer axis too long for the FDM line solve");
-        k_zsolve2<P, CI><<<(nl + kZ2Lines - 1) / kZ2Lines, 2 * kZ2Lines, smem, st>>>(zp);
-        return;
-    }
     const size_t smem = zsolve_smem<P>(zp.n2);
     TDZ_CHECK(smem <= kMax, TDZ_ERR_UNSUPPORTED, "outer axis too long for the FDM line solve");
-    k_zsolve<P, CI><<<(nl + kZThreads - 1) / kZThreads, kZThreads, smem, st>>>(zp);
+    const int entries = 2 * z_blocks(zp.n2, ZBlk<P>::B) * ZBlk<P>::B * (P + 1);
+    k_zbands<P><<<(entries + 127) / 128, 128, 0, st>>>(zp);
+    k_zsolve<P, CI><<<(nl + kZLines - 1) / kZLines, 2 * kZLines, smem, st>>>(zp);
 }
 
 // complex eigenvalues (complex axis pencils) take the variant with the
@@ -873,21 +665,21 @@ template <int P> void launch_zsolve(const ZSolveParams &zp, cudaStream_t st) {
     else launch_zsolve_t<P, false>(zp, st);
 }
 
-// saved-state scratch of the line solves (float2 entries): the larger of the
-// one-thread and the two-thread layouts
+// scratch of the line solves: saved states (float2 entries) and band rows (float4 entries)
+template <int P> size_t state_entries(int n2, size_t lines) {
+    return (size_t)2 * z_blocks(n2, ZBlk<P>::B) * ZBlk<P>::NS * lines;
+}
 size_t zsolve_state_size(int P, int n2, size_t lines) {
-    auto sz = [&](int B, int NS, int B2) {
-        const int m = zsolve2_twist(n2, B2);
-        const size_t one = (size_t)((n2 + B - 1) / B) * NS * lines;
-        const size_t two = (size_t)((m + B2 - 1) / B2 + (n2 - m + B2 - 1) / B2) * NS * lines;
-        return std::max(one, two);
-    };
     switch (P) {
-    case 2: return sz(ZBlk<2>::B, ZBlk<2>::NS, ZBlk2<2>::B);
-    case 3: return sz(ZBlk<3>::B, ZBlk<3>::NS, ZBlk2<3>::B);
-    case 4: return sz(ZBlk<4>::B, ZBlk<4>::NS, ZBlk2<4>::B);
-    default: return sz(ZBlk<5>::B, ZBlk<5>::NS, ZBlk2<5>::B);
+    case 2: return state_entries<2>(n2, lines);
+    case 3: return state_entries<3>(n2, lines);
+    case 4: return state_entries<4>(n2, lines);
+    default: return state_entries<5>(n2, lines);
     }
+}
+size_t zsolve_band_size(int P, int n2) {
+    const int B = P == 2 ? ZBlk<2>::B : P == 3 ? ZBlk<3>::B : P == 4 ? ZBlk<4>::B : ZBlk<5>::B;
+    return (size_t)2 * z_blocks(n2, B) * B * (P + 1);
 }
 
 }  // namespace
@@ -1033,7 +825,7 @@ void PcFDM::setup(Operator *op_, int prec) {
         return;
     }
     ufac.alloc(zsolve_state_size(P, n[dim - 1], N / n[dim - 1]) * sizeof(float2));
-    zb.alloc((size_t)2 * n[dim - 1] * (2 * P + 1) * sizeof(float2));
+    zb.alloc(zsolve_band_size(P, n[dim - 1]) * sizeof(float4));
     if (tensor) {
         npart.alloc((size_t)16 * sm_count() * sizeof(double));
         ldx = (n[0] + 3) / 4 * 4;
@@ -1104,7 +896,7 @@ ZSolveParams line_params(const PcFDM &f) {
     const int outer = dim - 1;
     ZSolveParams zp{};
     zp.ck = f.ufac.as<float2>();
-    zp.zb = f.zb.as<float2>();
+    zp.zb = f.zb.as<float4>();
     zp.bands = op->dev32[outer].as<float>();
     zp.lx = f.lam[0].as<float>();
     zp.ly = dim == 3 ? f.lam[1].as<float>() : nullptr;

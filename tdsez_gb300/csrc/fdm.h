@@ -40,7 +40,7 @@ struct PcFDM : Precond {
     // the inverse is exact (to FP32) for the operator's current stage: nothing
     // dropped, or the dropped terms' stage scalars are zero now
     bool exact_now() const;
-    DevBuf zb;                 // FP32 band rows of the line matrices, Bc then Cc, [2][n_outer][2P+1]
+    DevBuf zb;                 // FP32 upper band rows (Bc, Cc) of the line matrices in elimination order
     DevBuf b1, b2, ufac;       // FP32 work vectors and the saved elimination states of the line solves
     bool exact = true;         // false: inner one-axis terms were dropped (stiffness-only pencil, or a
                                // field along an inner axis)
