@@ -166,6 +166,7 @@ ApplyParams<T> make_params(const Operator &op, const Plan &pl, const void *x, vo
     prm.zC = eval_comb<T>(pl.zC, sg);
     prm.za_kind = comb_kind(pl.zA, sg);
     prm.zc_kind = comb_kind(pl.zC, sg);
+    prm.xt_kind = comb_kind(pl.xT, sg);
     prm.p = s.ax[0].p;
     prm.walls = 0;
     if (pl.walls) {

@@ -662,7 +662,7 @@ inline void run3d_rb(const ApplyParams<T> &prm0, cudaStream_t st) {
 // 3D: the register-blocked kernel for FP32 and double-float arithmetic (with
 // compile-time outer-combination kinds for the CN stage, KC = 2, and the
 // mass, KA = 1), the plane-ring kernel of apply_kernels.cuh for native FP64;
-// 2D: the row-tile kernel.
+// 2D: the tile kernel.
 template <class T, class MC, int P>
 inline void dispatch_rb(bool hb, bool hc, const ApplyParams<T> &prm, cudaStream_t st) {
     if (!hb && hc && prm.zc_kind == 2) { run3d_rb<T, MC, P, false, true, 0, 2>(prm, st); return; }   // CN stage

@@ -47,6 +47,7 @@ template <class T> struct ApplyParams {
     T wall_re[2], wall_im[2];   // 1D walls: diagonal values, wall = 0 / n-1
     int walls;
     int za_kind, zc_kind;       // outer combinations: 0 complex, 1 real, 2 imaginary (fewer products)
+    int xt_kind;                // the same of the stream-B combination along x (2D)
     const void *sub;            // non-null: y = sub - op x (a residual), same layout as y
     // 3D only: per-CTA partial sums of the stored y, red[blockIdx.x] (FP64):
     // red_mode 1: sum |y|^2, 2: sum conj(dotv) y (dotv laid out as y)
@@ -381,81 +382,104 @@ __global__ void __launch_bounds__(TX *TY) k_apply3d(const __grid_constant__ Appl
 }
 
 // ---------------------------------------------------------------- 2D kernel
-// x stage on a TX-wide row tile, outer stage along y with the register ring.
-template <class T, int P, bool HB, bool HC, int TX>
-__global__ void __launch_bounds__(TX) k_apply2d(const ApplyParams<T> prm) {
+// A CTA owns a kTX2 x kTY2 output tile: the halo tile of the input in shared
+// memory, the x stage of its kTY2 + 2P rows, then the y stage, one output per
+// thread; two barriers in all. A 2D operator is small (a few hundred thousand
+// coefficients at most in practice), so what counts is the latency of one
+// tile and having enough tiles: streaming row by row through a register ring
+// recomputed no halo rows but left a 260 x 260 grid 48 CTAs of 24 dependent
+// row steps (double-float, degree 4: 224 us; this kernel 19 us on its 297
+// tiles, the x stage computed twice over).
+constexpr int kTX2 = 32, kTY2 = 8;
+template <class T, int P, bool HB, bool HC> struct Shape2D {
     using C = typename CT<T>::type;
-    constexpr int BW = 2 * P + 1, RX = TX + 2 * P;
-    __shared__ C sIn[RX];
-    __shared__ C sZA[BW], sZC[BW];
-    __shared__ T sZM[BW];
-    const int tx = threadIdx.x;
-    const int n0 = prm.n0, n1 = prm.n1;
-    const int x0 = blockIdx.x * TX, gx = x0 + tx;
-    const int z0 = blockIdx.y * prm.zchunk;
-    const int z1 = min(n1, z0 + prm.zchunk);
-    if (z0 >= z1) return;
+    static constexpr int BW = 2 * P + 1, RY = kTY2 + 2 * P, RX = kTX2 + 2 * P;
+    static constexpr int NU = 1 + (HB ? 1 : 0) + (HC ? 1 : 0);
+    static constexpr size_t smem = sizeof(C) * (size_t)(RY * RX + NU * RY * kTX2 + BW * kTY2 * (HC ? 2 : 1)) +
+                                   (HB ? sizeof(T) * BW * kTY2 : 0);
+};
+
+// sum_j a_j v_j, the a_j complex or all imaginary (the uniform branch outside the loop)
+template <int BW, class C> __device__ __forceinline__ C dot_kind(const C (&a)[BW], const C *v, int stride, int kind) {
+    C s = czero<C>();
+    if (kind == 2) {
+#pragma unroll
+        for (int j = 0; j < BW; ++j) ifma(s, a[j].y, v[j * stride]);
+    } else {
+#pragma unroll
+        for (int j = 0; j < BW; ++j) cfma(s, a[j], v[j * stride]);
+    }
+    return s;
+}
+
+template <class T, int P, bool HB, bool HC>
+__global__ void __launch_bounds__(kTX2 *kTY2) k_apply2d(const __grid_constant__ ApplyParams<T> prm) {
+    using S = Shape2D<T, P, HB, HC>;
+    using C = typename S::C;
     using MC = typename MemC<T>::type;
+    constexpr int BW = S::BW, RY = S::RY, RX = S::RX, UT = 1, US = HB ? 2 : 1, NT = kTX2 * kTY2;
+    extern __shared__ __align__(16) unsigned char raw2d[];
+    C *sIn = reinterpret_cast<C *>(raw2d);          // [RY][RX]
+    C *sU = sIn + RY * RX;                          // [stream][RY][kTX2]
+    C *sZA = sU + S::NU * RY * kTX2;                // [row][BW]
+    C *sZC = sZA + kTY2 * BW;
+    T *sZM = reinterpret_cast<T *>(sZC + (HC ? kTY2 * BW : 0));
+    const int tx = threadIdx.x, ty = threadIdx.y, tid = ty * kTX2 + tx;
+    const int n0 = prm.n0, n1 = prm.n1;
+    const int tilesX = (n0 + kTX2 - 1) / kTX2;
+    const int x0 = (blockIdx.x % tilesX) * kTX2, y0 = (blockIdx.x / tilesX) * kTY2, gx = x0 + tx, gy = y0 + ty;
     const MC *__restrict__ X = static_cast<const MC *>(prm.x);
     MC *__restrict__ Y = static_cast<MC *>(prm.y);
-    T xm[BW], xs[HC ? BW : 1];
-    C xt[HB ? BW : 1];
-#pragma unroll
-    for (int j = 0; j < BW; ++j) {
-        const bool in = gx < n0;
-        xm[j] = in ? prm.b0[((size_t)kM * n0 + gx) * BW + j] : T(0);
-        if constexpr (HC) xs[j] = in ? prm.b0[((size_t)kS * n0 + gx) * BW + j] : T(0);
-        if constexpr (HB) xt[j] = in ? comb_at<T, C>(prm.xT, prm.b0, n0, BW, gx, j) : czero<C>();
+    for (int e = tid; e < RY * RX; e += NT) {
+        const int yy = y0 - P + e / RX, xx = x0 - P + e % RX;
+        sIn[e] = (yy >= 0 && yy < n1 && xx >= 0 && xx < n0) ? load_c<C>(X[(size_t)yy * n0 + xx]) : czero<C>();
     }
-    C acc[BW];
+    for (int e = tid; e < kTY2 * BW; e += NT) {
+        const int yy = y0 + e / BW, o = e % BW;
+        const bool in = yy < n1;
+        sZA[e] = in ? comb_at<T, C>(prm.zA, prm.b1, n1, BW, yy, o) : czero<C>();
+        if constexpr (HC) sZC[e] = in ? comb_at<T, C>(prm.zC, prm.b1, n1, BW, yy, o) : czero<C>();
+        if constexpr (HB) sZM[e] = in ? prm.b1[((size_t)kM * n1 + yy) * BW + o] : T(0);
+    }
+    {
+        // band rows of this thread's column
+        T xm[BW], xs[HC ? BW : 1];
+        C xt[HB ? BW : 1];
 #pragma unroll
-    for (int s = 0; s < BW; ++s) acc[s] = czero<C>();
-    const int zs = z0 - P;
-    const int nplanes = (z1 - z0) + 2 * P;
-    for (int base = 0; base < nplanes; base += BW) {
+        for (int j = 0; j < BW; ++j) {
+            const bool in = gx < n0;
+            xm[j] = in ? prm.b0[((size_t)kM * n0 + gx) * BW + j] : T(0);
+            if constexpr (HC) xs[j] = in ? prm.b0[((size_t)kS * n0 + gx) * BW + j] : T(0);
+            if constexpr (HB) xt[j] = in ? comb_at<T, C>(prm.xT, prm.b0, n0, BW, gx, j) : czero<C>();
+        }
+        __syncthreads();
+        for (int r = ty; r < RY; r += kTY2) {
+            const C *v = sIn + r * RX + tx;
+            C uM = czero<C>();
 #pragma unroll
-        for (int ph = 0; ph < BW; ++ph) {
-            const int it = base + ph;
-            if (it >= nplanes) break;
-            const int zin = zs + it;
-            if (zin >= 0 && zin < n1) {
-                __syncthreads();
-                for (int c = tx; c < RX; c += TX) {
-                    const int xx = x0 - P + c;
-                    sIn[c] = (xx >= 0 && xx < n0) ? load_c<C>(X[(size_t)zin * n0 + xx]) : czero<C>();
-                }
-                if (tx < BW) {
-                    sZA[tx] = comb_at<T, C>(prm.zA, prm.b1, n1, BW, zin, tx);
-                    if constexpr (HB) sZM[tx] = prm.b1[((size_t)kM * n1 + zin) * BW + tx];
-                    if constexpr (HC) sZC[tx] = comb_at<T, C>(prm.zC, prm.b1, n1, BW, zin, tx);
-                }
-                __syncthreads();
-                C uM = czero<C>(), uT = czero<C>(), uS = czero<C>();
+            for (int j = 0; j < BW; ++j) rfma(uM, xm[j], v[j]);
+            sU[r * kTX2 + tx] = cnorm(uM);
+            if constexpr (HC) {
+                C uS = czero<C>();
 #pragma unroll
-                for (int j = 0; j < BW; ++j) {
-                    const C v = sIn[tx + j];
-                    rfma(uM, xm[j], v);
-                    if constexpr (HB) cfma(uT, xt[j], v);
-                    if constexpr (HC) rfma(uS, xs[j], v);
-                }
-                uM = cnorm(uM);
-                if constexpr (HB) uT = cnorm(uT);
-                if constexpr (HC) uS = cnorm(uS);
-#pragma unroll
-                for (int o = 0; o < BW; ++o) {
-                    C &a = acc[(ph - P + o + 2 * BW) % BW];
-                    kfma(a, sZA[o], uM, prm.za_kind);
-                    if constexpr (HB) rfma(a, sZM[o], uT);
-                    if constexpr (HC) kfma(a, sZC[o], uS, prm.zc_kind);
-                }
+                for (int j = 0; j < BW; ++j) rfma(uS, xs[j], v[j]);
+                sU[(US * RY + r) * kTX2 + tx] = cnorm(uS);
             }
-            if (it >= 2 * P) {
-                const int m = zin - P;
-                if (gx < n0) Y[(size_t)m * n0 + gx] = out_value<T, MC>(prm, (size_t)m * n0 + gx, acc[(ph - P + 2 * BW) % BW]);
-            }
-            acc[(ph - P + 2 * BW) % BW] = czero<C>();
+            if constexpr (HB) sU[(UT * RY + r) * kTX2 + tx] = cnorm(dot_kind<BW, C>(xt, v, 1, prm.xt_kind));
         }
     }
+    __syncthreads();
+    if (gx >= n0 || gy >= n1) return;
+    C out = czero<C>();
+    const C *u = sU + ty * kTX2 + tx;
+#pragma unroll
+    for (int j = 0; j < BW; ++j) {
+        kfma(out, sZA[ty * BW + j], u[j * kTX2], prm.za_kind);
+        if constexpr (HB) rfma(out, sZM[ty * BW + j], u[(UT * RY + j) * kTX2]);
+        if constexpr (HC) kfma(out, sZC[ty * BW + j], u[(US * RY + j) * kTX2], prm.zc_kind);
+    }
+    const size_t e = (size_t)gy * n0 + gx;
+    Y[e] = out_value<T, MC>(prm, e, out);
 }
 
 // ---------------------------------------------------------------- 1D kernel
@@ -492,22 +516,13 @@ __global__ void k_apply1d(const ApplyParams<T> prm) {
 }
 
 // ---------------------------------------------------------------- launch helpers
-constexpr int kTX3 = 32, kTY3 = 8, kTX2 = 128;
+constexpr int kTX3 = 32, kTY3 = 8;
 // tile height: 8 rows for FP32; 16 for FP64 and double-float, which recompute
 // the 2p halo rows of the x stage (ratio (16 + 2p) / 16 instead of (8 + 2p) / 8),
 // except with all three streams, whose registers need the smaller CTA
 template <class T, bool HB, bool HC> struct TileY {
     static constexpr int v = std::is_same<T, float>::value || (HB && HC) ? 8 : 16;
 };
-
-// z chunk per CTA: about `target` CTAs in total (0: 8 per SM), chunks no
-// shorter than 4p planes (the 2p halo planes of a chunk are re-read)
-inline int pick_chunk(int tiles, int n_outer, int P, int target = 0) {
-    if (target <= 0) target = 8 * sm_count();
-    int chunks = (target + tiles - 1) / tiles;
-    chunks = std::max(1, std::min(chunks, n_outer / std::max(1, 4 * P)));
-    return (n_outer + chunks - 1) / chunks;
-}
 
 // tile width 16..32 (multiple of 4) with the least padding of n0; ties go to the wider
 inline int pick_tile_x(int n0) {
@@ -639,12 +654,17 @@ inline void run3d(const ApplyParams<T> &prm0, cudaStream_t st) {
 }
 
 template <class T, int P, bool HB, bool HC>
-inline void run2d(const ApplyParams<T> &prm0, cudaStream_t st) {
-    ApplyParams<T> prm = prm0;
-    const int tiles = (prm.n0 + kTX2 - 1) / kTX2;
-    prm.zchunk = pick_chunk(tiles, prm.n1, P);
-    dim3 grid(tiles, (prm.n1 + prm.zchunk - 1) / prm.zchunk);
-    k_apply2d<T, P, HB, HC, kTX2><<<grid, kTX2, 0, st>>>(prm);
+inline void run2d(const ApplyParams<T> &prm, cudaStream_t st) {
+    auto kern = k_apply2d<T, P, HB, HC>;
+    constexpr size_t smem = Shape2D<T, P, HB, HC>::smem;
+    static const bool attr = [&] {
+        TDZ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
+        return true;
+    }();
+    (void)attr;
+    const long long tiles = (long long)((prm.n0 + kTX2 - 1) / kTX2) * ((prm.n1 + kTY2 - 1) / kTY2);
+    TDZ_CHECK(tiles < (1LL << 31), TDZ_ERR_UNSUPPORTED, "too many tiles for the 2D apply");
+    kern<<<(unsigned)tiles, dim3(kTX2, kTY2), smem, st>>>(prm);
 }
 
 // per-degree entry points (apply_p<P>.cu)
