@@ -1,10 +1,10 @@
 // Non-separable soft-core potential term by per-element quadrature (quad.h).
-// One CTA per element: gather the (p+1)^d coefficients, interpolate to the
-// Q^d Gauss points axis by axis (sum factorisation, shared memory ping-pong),
-// multiply by w V with V from the closed form, project back axis by axis and
-// add coef * result to y with atomics (neighbouring elements share
-// coefficients). Work per element 2 d Q (p+1)^d (d-dimensional sum
-// factorisation): the per-element tensor-contraction flops of this term.
+// 3D: one CTA per element (k_quad): gather the (p+1)^3 coefficients,
+// interpolate to the Q^3 Gauss points axis by axis (sum factorisation, shared
+// memory ping-pong), multiply by w V with V from the closed form, project back
+// axis by axis and add coef * result to y with atomics (neighbouring elements
+// share coefficients); or, for ordinary knots, the streaming kernel below.
+// 2D: the assembled stencil (k_stencil2).
 #include "quad.h"
 
 #include <algorithm>
@@ -45,23 +45,23 @@ template <class T> __device__ __forceinline__ T rsqrt_t(T v);
 template <> __device__ __forceinline__ float rsqrt_t<float>(float v) { return rsqrtf(v); }
 template <> __device__ __forceinline__ double rsqrt_t<double>(double v) { return 1.0 / sqrt(v); }
 
-template <class T, int P, int DIM>
+template <class T, int P>
 __global__ void __launch_bounds__(kQThreads) k_quad(const QuadParams<T> prm) {
     using C = typename CT<T>::type;
     constexpr int NP = P + 1;
     constexpr int M = NP > kMaxQ ? NP : kMaxQ;
-    constexpr int CAP = DIM == 3 ? M * M * M : M * M;
+    constexpr int CAP = M * M * M;
     __shared__ C bufA[CAP], bufB[CAP];
     __shared__ T sN[3][kMaxQ * NP], sW[3][kMaxQ], sX[3][kMaxQ];
     const int Q = prm.nq, tid = threadIdx.x;
     int e = blockIdx.x;
     int el[3] = {0, 0, 0};
-    for (int d = 0; d < DIM; ++d) { el[d] = e % prm.nel[d]; e /= prm.nel[d]; }
+    for (int d = 0; d < 3; ++d) { el[d] = e % prm.nel[d]; e /= prm.nel[d]; }
     int o[3] = {0, 0, 0};
-    for (int d = 0; d < DIM; ++d) o[d] = prm.off[d][el[d]];
-    for (int d = 0; d < DIM; ++d)
+    for (int d = 0; d < 3; ++d) o[d] = prm.off[d][el[d]];
+    for (int d = 0; d < 3; ++d)
         for (int i = tid; i < Q * NP; i += kQThreads) sN[d][i] = prm.N[d][(size_t)el[d] * Q * NP + i];
-    for (int d = 0; d < DIM; ++d)
+    for (int d = 0; d < 3; ++d)
         for (int i = tid; i < Q; i += kQThreads) {
             sW[d][i] = prm.w[d][(size_t)el[d] * Q + i];
             sX[d][i] = prm.xq[d][(size_t)el[d] * Q + i];
@@ -69,119 +69,192 @@ __global__ void __launch_bounds__(kQThreads) k_quad(const QuadParams<T> prm) {
     const C *X = static_cast<const C *>(prm.x);
     C *Y = static_cast<C *>(prm.y);
     // extents of the local tensor [z][y][x] during the passes
-    if constexpr (DIM == 3) {
-        for (int i = tid; i < NP * NP * NP; i += kQThreads) {
-            const int kx = i % NP, ky = (i / NP) % NP, kz = i / (NP * NP);
-            bufA[i] = X[((size_t)(o[2] + kz) * prm.n[1] + (o[1] + ky)) * prm.n[0] + o[0] + kx];
+    for (int i = tid; i < NP * NP * NP; i += kQThreads) {
+        const int kx = i % NP, ky = (i / NP) % NP, kz = i / (NP * NP);
+        bufA[i] = X[((size_t)(o[2] + kz) * prm.n[1] + (o[1] + ky)) * prm.n[0] + o[0] + kx];
+    }
+    __syncthreads();
+    // x: A[kz][ky][kx] -> B[kz][ky][qx]
+    for (int i = tid; i < NP * NP * Q; i += kQThreads) {
+        const int qx = i % Q, r = i / Q;
+        C acc = czero<C>();
+        for (int k = 0; k < NP; ++k) rfma(acc, sN[0][qx * NP + k], bufA[r * NP + k]);
+        bufB[i] = acc;
+    }
+    __syncthreads();
+    // y: B[kz][ky][qx] -> A[kz][qy][qx]
+    for (int i = tid; i < NP * Q * Q; i += kQThreads) {
+        const int qx = i % Q, qy = (i / Q) % Q, kz = i / (Q * Q);
+        C acc = czero<C>();
+        for (int k = 0; k < NP; ++k) rfma(acc, sN[1][qy * NP + k], bufB[(kz * NP + k) * Q + qx]);
+        bufA[i] = acc;
+    }
+    __syncthreads();
+    // z: A[kz][qy][qx] -> B[qz][qy][qx], times w V
+    for (int i = tid; i < Q * Q * Q; i += kQThreads) {
+        const int qx = i % Q, qy = (i / Q) % Q, qz = i / (Q * Q);
+        C acc = czero<C>();
+        for (int k = 0; k < NP; ++k) rfma(acc, sN[2][qz * NP + k], bufA[(k * Q + qy) * Q + qx]);
+        T v = T(0);
+        for (int c = 0; c < prm.nsoft; ++c) {
+            const T dx = sX[0][qx] - prm.soft[c][1], dy = sX[1][qy] - prm.soft[c][2], dz = sX[2][qz] - prm.soft[c][3];
+            v -= prm.soft[c][0] * rsqrt_t<T>(dx * dx + dy * dy + dz * dz + prm.soft[c][4]);
         }
-        __syncthreads();
-        // x: A[kz][ky][kx] -> B[kz][ky][qx]
-        for (int i = tid; i < NP * NP * Q; i += kQThreads) {
-            const int qx = i % Q, r = i / Q;
-            C acc = czero<C>();
-            for (int k = 0; k < NP; ++k) rfma(acc, sN[0][qx * NP + k], bufA[r * NP + k]);
-            bufB[i] = acc;
+        const T f = sW[0][qx] * sW[1][qy] * sW[2][qz] * v;
+        acc.x *= f;
+        acc.y *= f;
+        bufB[i] = acc;
+    }
+    __syncthreads();
+    // back z: B[qz][qy][qx] -> A[kz][qy][qx]
+    for (int i = tid; i < NP * Q * Q; i += kQThreads) {
+        const int qx = i % Q, qy = (i / Q) % Q, kz = i / (Q * Q);
+        C acc = czero<C>();
+        for (int q = 0; q < Q; ++q) rfma(acc, sN[2][q * NP + kz], bufB[(q * Q + qy) * Q + qx]);
+        bufA[i] = acc;
+    }
+    __syncthreads();
+    // back y: A[kz][qy][qx] -> B[kz][ky][qx]
+    for (int i = tid; i < NP * NP * Q; i += kQThreads) {
+        const int qx = i % Q, ky = (i / Q) % NP, kz = i / (Q * NP);
+        C acc = czero<C>();
+        for (int q = 0; q < Q; ++q) rfma(acc, sN[1][q * NP + ky], bufA[(kz * Q + q) * Q + qx]);
+        bufB[i] = acc;
+    }
+    __syncthreads();
+    // back x and scatter: B[kz][ky][qx] -> y
+    for (int i = tid; i < NP * NP * NP; i += kQThreads) {
+        const int kx = i % NP, r = i / NP, ky = r % NP, kz = r / NP;
+        C acc = czero<C>();
+        for (int q = 0; q < Q; ++q) rfma(acc, sN[0][q * NP + kx], bufB[r * Q + q]);
+        C out;
+        out.x = prm.cre * acc.x - prm.cim * acc.y;
+        out.y = prm.cre * acc.y + prm.cim * acc.x;
+        atomic_add_c(&Y[((size_t)(o[2] + kz) * prm.n[1] + (o[1] + ky)) * prm.n[0] + o[0] + kx], out);
+    }
+}
+
+// ---------------------------------------------------------------- 2D stencil
+// The term couples a coefficient to the (2p+1)^2 around it. Its entries are
+// stored one triangle only, entry-major (entry e of every coefficient is
+// contiguous): e = 0 the diagonal, then the offsets (dx, dy) with dy > 0 or
+// dy = 0 and dx > 0; the mirrored ones are read at the partner coefficient.
+//
+// Bound by GB300's FP64 pipe (FP64 vectors): 2 (2p+1)^2 products per
+// coefficient, against 2 (p+1)^2 (4 (p+1)) products and (p+1)^2 potential
+// values (FP64 square root and division) per element when the quadrature is
+// redone in every apply, which took 251 us on 256^2 elements of degree 4 with
+// atomics; the stencil takes 26 us there, and is deterministic.
+inline int quad2_entries(int p) { return ((2 * p + 1) * (2 * p + 1) + 1) / 2; }
+// entry e >= 0 of the triangle <-> offset (dx, dy): e = dy (2p+1) + dx, dx in -p..p
+// (dy = 0: dx >= 0), so that e runs over 0 .. quad2_entries - 1
+__host__ __device__ constexpr int quad2_entry(int p, int dx, int dy) { return dy * (2 * p + 1) + dx; }
+
+struct Asm2Params {
+    int n0, n1, Q, p;
+    const int *off[2], *elo[2], *ehi[2];   // element windows; elements of each coefficient's support
+    const double *N[2], *w[2], *xq[2];
+    int nel0, nel1, nsoft;
+    double soft[kMaxSoft][5];
+    double *wv;                            // w V at the Gauss points, [nel1 Q][nel0 Q]
+    double *st64;
+    float *st32;
+};
+
+__global__ void k_wv2(const Asm2Params prm) {
+    const size_t n = (size_t)prm.nel0 * prm.Q * prm.nel1 * prm.Q;
+    for (size_t e = blockIdx.x * (size_t)blockDim.x + threadIdx.x; e < n; e += (size_t)gridDim.x * blockDim.x) {
+        const int qx = (int)(e % ((size_t)prm.nel0 * prm.Q)), qy = (int)(e / ((size_t)prm.nel0 * prm.Q));
+        double v = 0.0;
+        for (int c = 0; c < prm.nsoft; ++c) {
+            const double dx = prm.xq[0][qx] - prm.soft[c][1], dy = prm.xq[1][qy] - prm.soft[c][2];
+            v -= prm.soft[c][0] / sqrt(dx * dx + dy * dy + prm.soft[c][4]);
         }
-        __syncthreads();
-        // y: B[kz][ky][qx] -> A[kz][qy][qx]
-        for (int i = tid; i < NP * Q * Q; i += kQThreads) {
-            const int qx = i % Q, qy = (i / Q) % Q, kz = i / (Q * Q);
-            C acc = czero<C>();
-            for (int k = 0; k < NP; ++k) rfma(acc, sN[1][qy * NP + k], bufB[(kz * NP + k) * Q + qx]);
-            bufA[i] = acc;
-        }
-        __syncthreads();
-        // z: A[kz][qy][qx] -> B[qz][qy][qx], times w V
-        for (int i = tid; i < Q * Q * Q; i += kQThreads) {
-            const int qx = i % Q, qy = (i / Q) % Q, qz = i / (Q * Q);
-            C acc = czero<C>();
-            for (int k = 0; k < NP; ++k) rfma(acc, sN[2][qz * NP + k], bufA[(k * Q + qy) * Q + qx]);
-            T v = T(0);
-            for (int c = 0; c < prm.nsoft; ++c) {
-                const T dx = sX[0][qx] - prm.soft[c][1], dy = sX[1][qy] - prm.soft[c][2], dz = sX[2][qz] - prm.soft[c][3];
-                v -= prm.soft[c][0] * rsqrt_t<T>(dx * dx + dy * dy + dz * dz + prm.soft[c][4]);
+        prm.wv[e] = prm.w[0][qx] * prm.w[1][qy] * v;
+    }
+}
+
+// one thread per coefficient and entry (blockIdx.y)
+__global__ void __launch_bounds__(128) k_assemble2(const Asm2Params prm) {
+    const size_t N = (size_t)prm.n0 * prm.n1;
+    const size_t idx = blockIdx.x * (size_t)blockDim.x + threadIdx.x;
+    if (idx >= N) return;
+    const int bw = 2 * prm.p + 1, np = prm.p + 1, Q = prm.Q;
+    const int e = blockIdx.y;
+    // dy (2p+1) + dx with dx in -p..p
+    const int dy = (e + prm.p) / bw, dx = e - dy * bw;
+    const int i = (int)(idx % prm.n0), j = (int)(idx / prm.n0);
+    const int i2 = i + dx, j2 = j + dy;
+    double sum = 0.0;
+    if (i2 >= 0 && i2 < prm.n0 && j2 < prm.n1) {
+        const int x0 = max(prm.elo[0][i], prm.elo[0][i2]), x1 = min(prm.ehi[0][i], prm.ehi[0][i2]);
+        const int y0 = max(prm.elo[1][j], prm.elo[1][j2]), y1 = min(prm.ehi[1][j], prm.ehi[1][j2]);
+        for (int ey = y0; ey <= y1; ++ey) {
+            const double *Ny = prm.N[1] + (size_t)ey * Q * np - prm.off[1][ey];
+            for (int qy = 0; qy < Q; ++qy) {
+                const double fy = Ny[qy * np + j] * Ny[qy * np + j2];
+                const double *wv = prm.wv + ((size_t)ey * Q + qy) * prm.nel0 * Q;
+                double row = 0.0;
+                for (int ex = x0; ex <= x1; ++ex) {
+                    const double *Nx = prm.N[0] + (size_t)ex * Q * np - prm.off[0][ex];
+                    for (int qx = 0; qx < Q; ++qx) row = fma(wv[ex * Q + qx], Nx[qx * np + i] * Nx[qx * np + i2], row);
+                }
+                sum = fma(fy, row, sum);
             }
-            const T f = sW[0][qx] * sW[1][qy] * sW[2][qz] * v;
-            acc.x *= f;
-            acc.y *= f;
-            bufB[i] = acc;
-        }
-        __syncthreads();
-        // back z: B[qz][qy][qx] -> A[kz][qy][qx]
-        for (int i = tid; i < NP * Q * Q; i += kQThreads) {
-            const int qx = i % Q, qy = (i / Q) % Q, kz = i / (Q * Q);
-            C acc = czero<C>();
-            for (int q = 0; q < Q; ++q) rfma(acc, sN[2][q * NP + kz], bufB[(q * Q + qy) * Q + qx]);
-            bufA[i] = acc;
-        }
-        __syncthreads();
-        // back y: A[kz][qy][qx] -> B[kz][ky][qx]
-        for (int i = tid; i < NP * NP * Q; i += kQThreads) {
-            const int qx = i % Q, ky = (i / Q) % NP, kz = i / (Q * NP);
-            C acc = czero<C>();
-            for (int q = 0; q < Q; ++q) rfma(acc, sN[1][q * NP + ky], bufA[(kz * Q + q) * Q + qx]);
-            bufB[i] = acc;
-        }
-        __syncthreads();
-        // back x and scatter: B[kz][ky][qx] -> y
-        for (int i = tid; i < NP * NP * NP; i += kQThreads) {
-            const int kx = i % NP, r = i / NP, ky = r % NP, kz = r / NP;
-            C acc = czero<C>();
-            for (int q = 0; q < Q; ++q) rfma(acc, sN[0][q * NP + kx], bufB[r * Q + q]);
-            C out;
-            out.x = prm.cre * acc.x - prm.cim * acc.y;
-            out.y = prm.cre * acc.y + prm.cim * acc.x;
-            atomic_add_c(&Y[((size_t)(o[2] + kz) * prm.n[1] + (o[1] + ky)) * prm.n[0] + o[0] + kx], out);
-        }
-    } else {
-        for (int i = tid; i < NP * NP; i += kQThreads) {
-            const int kx = i % NP, ky = i / NP;
-            bufA[i] = X[(size_t)(o[1] + ky) * prm.n[0] + o[0] + kx];
-        }
-        __syncthreads();
-        // x: A[ky][kx] -> B[ky][qx]
-        for (int i = tid; i < NP * Q; i += kQThreads) {
-            const int qx = i % Q, ky = i / Q;
-            C acc = czero<C>();
-            for (int k = 0; k < NP; ++k) rfma(acc, sN[0][qx * NP + k], bufA[ky * NP + k]);
-            bufB[i] = acc;
-        }
-        __syncthreads();
-        // y: B[ky][qx] -> A[qy][qx], times w V
-        for (int i = tid; i < Q * Q; i += kQThreads) {
-            const int qx = i % Q, qy = i / Q;
-            C acc = czero<C>();
-            for (int k = 0; k < NP; ++k) rfma(acc, sN[1][qy * NP + k], bufB[k * Q + qx]);
-            T v = T(0);
-            for (int c = 0; c < prm.nsoft; ++c) {
-                const T dx = sX[0][qx] - prm.soft[c][1], dy = sX[1][qy] - prm.soft[c][2];
-                v -= prm.soft[c][0] * rsqrt_t<T>(dx * dx + dy * dy + prm.soft[c][4]);
-            }
-            const T f = sW[0][qx] * sW[1][qy] * v;
-            acc.x *= f;
-            acc.y *= f;
-            bufA[i] = acc;
-        }
-        __syncthreads();
-        // back y: A[qy][qx] -> B[ky][qx]
-        for (int i = tid; i < NP * Q; i += kQThreads) {
-            const int qx = i % Q, ky = i / Q;
-            C acc = czero<C>();
-            for (int q = 0; q < Q; ++q) rfma(acc, sN[1][q * NP + ky], bufA[q * Q + qx]);
-            bufB[i] = acc;
-        }
-        __syncthreads();
-        // back x and scatter
-        for (int i = tid; i < NP * NP; i += kQThreads) {
-            const int kx = i % NP, ky = i / NP;
-            C acc = czero<C>();
-            for (int q = 0; q < Q; ++q) rfma(acc, sN[0][q * NP + kx], bufB[ky * Q + q]);
-            C out;
-            out.x = prm.cre * acc.x - prm.cim * acc.y;
-            out.y = prm.cre * acc.y + prm.cim * acc.x;
-            atomic_add_c(&Y[(size_t)(o[1] + ky) * prm.n[0] + o[0] + kx], out);
         }
     }
+    prm.st64[(size_t)e * N + idx] = sum;
+    prm.st32[(size_t)e * N + idx] = (float)sum;
+}
+
+// y += coef * V_q x from the stencil; a 32 x 8 tile of coefficients per CTA
+constexpr int kStX = 32, kStY = 8;
+template <class T, int P>
+__global__ void __launch_bounds__(kStX *kStY) k_stencil2(const T *__restrict__ st, int n0, int n1, T cre, T cim,
+                                                         const typename CT<T>::type *__restrict__ x,
+                                                         typename CT<T>::type *__restrict__ y) {
+    using C = typename CT<T>::type;
+    constexpr int RX = kStX + 2 * P, RY = kStY + 2 * P;
+    __shared__ C sx[RY][RX];
+    const int tilesX = (n0 + kStX - 1) / kStX;
+    const int x0 = (blockIdx.x % tilesX) * kStX, y0 = (blockIdx.x / tilesX) * kStY;
+    const int tx = threadIdx.x, ty = threadIdx.y;
+    for (int e = ty * kStX + tx; e < RY * RX; e += kStX * kStY) {
+        const int gy = y0 - P + e / RX, gx = x0 - P + e % RX;
+        sx[e / RX][e % RX] = gy >= 0 && gy < n1 && gx >= 0 && gx < n0 ? x[(size_t)gy * n0 + gx] : czero<C>();
+    }
+    __syncthreads();
+    const int gx = x0 + tx, gy = y0 + ty;
+    if (gx >= n0 || gy >= n1) return;
+    const size_t N = (size_t)n0 * n1, idx = (size_t)gy * n0 + gx;
+    C up = czero<C>(), lo = czero<C>();   // the triangle and its mirror
+#pragma unroll
+    for (int dy = 0; dy <= P; ++dy)
+#pragma unroll
+        for (int dx = -P; dx <= P; ++dx) {
+            if (dy == 0 && dx < 0) continue;
+            const T *row = st + (size_t)quad2_entry(P, dx, dy) * N;
+            rfma(up, row[idx], sx[ty + P + dy][tx + P + dx]);
+            if (dy == 0 && dx == 0) continue;
+            // the partner (gx - dx, gy - dy); outside the grid x is zero there
+            const bool in = gx - dx >= 0 && gx - dx < n0 && gy - dy >= 0;
+            rfma(lo, in ? row[idx - (size_t)dy * n0 - dx] : T(0), sx[ty + P - dy][tx + P - dx]);
+        }
+    up.x += lo.x;
+    up.y += lo.y;
+    C o = y[idx];
+    o.x += cre * up.x - cim * up.y;
+    o.y += cre * up.y + cim * up.x;
+    y[idx] = o;
+}
+
+template <class T, int P> void launch_stencil2(const QuadTerm &q, cd coef, const void *x, void *y, cudaStream_t st) {
+    using C = typename CT<T>::type;
+    const long long tiles = (long long)((q.n[0] + kStX - 1) / kStX) * ((q.n[1] + kStY - 1) / kStY);
+    TDZ_CHECK(tiles < (1LL << 31), TDZ_ERR_UNSUPPORTED, "too many coefficients for the quadrature term");
+    const T *tab = static_cast<const T *>((sizeof(T) == 8 ? q.st64 : q.st32).ptr);
+    k_stencil2<T, P><<<(unsigned)tiles, dim3(kStX, kStY), 0, st>>>(tab, q.n[0], q.n[1], (T)coef.real(), (T)coef.imag(),
+                                                                   static_cast<const C *>(x), static_cast<C *>(y));
 }
 
 // ---------------------------------------------------------------- streaming 3D kernel
@@ -469,14 +542,22 @@ QuadParams<T> make_qparams(const QuadTerm &q, cd coef, const void *x, void *y) {
 
 template <class T, int P>
 void launch_q(const QuadTerm &q, const QuadParams<T> &prm, cudaStream_t st) {
-    const long long nel = (long long)q.nel[0] * q.nel[1] * (q.dim == 3 ? q.nel[2] : 1);
+    const long long nel = (long long)q.nel[0] * q.nel[1] * q.nel[2];
     TDZ_CHECK(nel < (1LL << 31), TDZ_ERR_UNSUPPORTED, "too many elements for the quadrature term");
-    if (q.dim == 3) k_quad<T, P, 3><<<(unsigned)nel, kQThreads, 0, st>>>(prm);
-    else k_quad<T, P, 2><<<(unsigned)nel, kQThreads, 0, st>>>(prm);
+    k_quad<T, P><<<(unsigned)nel, kQThreads, 0, st>>>(prm);
 }
 
 template <class T>
 void dispatch_q(const QuadTerm &q, cd coef, const void *x, void *y, cudaStream_t st) {
+    if (q.dim == 2) {
+        switch (q.p) {
+        case 2: launch_stencil2<T, 2>(q, coef, x, y, st); return;
+        case 3: launch_stencil2<T, 3>(q, coef, x, y, st); return;
+        case 4: launch_stencil2<T, 4>(q, coef, x, y, st); return;
+        case 5: launch_stencil2<T, 5>(q, coef, x, y, st); return;
+        default: throw Error(TDZ_ERR_UNSUPPORTED, "quadrature term supports degrees 2..5");
+        }
+    }
     const QuadParams<T> prm = make_qparams<T>(q, coef, x, y);
     if (stream_ok(q)) {   // FP32: FP32 arithmetic; FP64 vectors: double-float arithmetic
         using A = typename std::conditional<std::is_same<T, float>::value, float, dff>::type;
@@ -495,6 +576,52 @@ void dispatch_q(const QuadTerm &q, cd coef, const void *x, void *y, cudaStream_t
     case 5: launch_q<T, 5>(q, prm, st); break;
     default: throw Error(TDZ_ERR_UNSUPPORTED, "quadrature term supports degrees 2..5");
     }
+}
+
+void assemble2(QuadTerm &q, const Space &s) {
+    Asm2Params prm{};
+    prm.n0 = q.n[0];
+    prm.n1 = q.n[1];
+    prm.Q = q.nq;
+    prm.p = q.p;
+    prm.nel0 = q.nel[0];
+    prm.nel1 = q.nel[1];
+    DevBuf lo[2], hi[2], wv;
+    for (int d = 0; d < 2; ++d) {
+        const Axis1D &a = s.ax[d];
+        std::vector<int> l(a.n, a.nel), h(a.n, -1);
+        for (int e = 0; e < a.nel; ++e)
+            for (int k = a.offset[e]; k <= a.offset[e] + a.p; ++k) {
+                l[k] = std::min(l[k], e);
+                h[k] = std::max(h[k], e);
+            }
+        upload(lo[d], l);
+        upload(hi[d], h);
+        prm.off[d] = q.off[d].as<int>();
+        prm.elo[d] = lo[d].as<int>();
+        prm.ehi[d] = hi[d].as<int>();
+        prm.N[d] = q.N64[d].as<double>();
+        prm.w[d] = q.w64[d].as<double>();
+        prm.xq[d] = q.x64[d].as<double>();
+    }
+    prm.nsoft = q.nsoft;
+    for (int c = 0; c < q.nsoft; ++c)
+        for (int k = 0; k < 5; ++k) prm.soft[c][k] = q.soft[c][k];
+    const size_t N = (size_t)q.n[0] * q.n[1], pts = (size_t)q.nel[0] * q.nel[1] * q.nq * q.nq;
+    const int ne = quad2_entries(q.p);
+    wv.alloc(pts * sizeof(double));
+    q.st64.alloc(N * ne * sizeof(double));
+    q.st32.alloc(N * ne * sizeof(float));
+    prm.wv = wv.as<double>();
+    prm.st64 = q.st64.as<double>();
+    prm.st32 = q.st32.as<float>();
+    const size_t blocks = (N + 127) / 128;
+    TDZ_CHECK(blocks < (1ull << 31), TDZ_ERR_UNSUPPORTED, "too many coefficients for the quadrature term");
+    k_wv2<<<(int)std::min<size_t>((pts + 255) / 256, (size_t)16 * sm_count()), 256>>>(prm);
+    k_assemble2<<<dim3((unsigned)blocks, ne), 128>>>(prm);
+    TDZ_CUDA(cudaGetLastError());
+    count_launch(2);
+    TDZ_CUDA(cudaStreamSynchronize(nullptr));   // the stencil is used on any stream
 }
 
 }  // namespace
@@ -531,6 +658,7 @@ void QuadTerm::build(const Space &s, int nsoft_, const double *soft_) {
         upload(w32[d], std::vector<float>(a.wq.begin(), a.wq.end()));
         upload(x32[d], std::vector<float>(a.xq.begin(), a.xq.end()));
     }
+    if (dim == 2) assemble2(*this, s);
 }
 
 void QuadTerm::apply(cd coef, int prec, const void *x, void *y, cudaStream_t st) const {

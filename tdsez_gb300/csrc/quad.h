@@ -5,10 +5,15 @@
 // the s V block of TDSEZFormHam (src/assembly/assembly.cpp:703-864) and of the
 // sum-factorised element kernel SumFactElement (src/assembly/sumfact.cpp:471-523)
 // for a potential that is not a sum of one-axis functions (the 2D and 3D
-// soft-core Coulomb cases). Applied matrix-free: per element the (p+1)^d
-// local coefficients are interpolated to the Q^d Gauss points one axis at a
-// time, multiplied by w V (V evaluated in the kernel from the closed form, no
-// table), projected back one axis at a time and added to y.
+// soft-core Coulomb cases).
+//
+// 3D: applied matrix-free. Per element the (p+1)^3 local coefficients are
+// interpolated to the Q^3 Gauss points one axis at a time, multiplied by w V
+// (V evaluated in the kernel from the closed form, no table), projected back
+// one axis at a time and added to y.
+// 2D: the term's (2p+1)^2-point stencil, assembled once on the device when the
+// operator is built (FP64 quadrature, one triangle: (2p+1)^2 / 2 real entries
+// per coefficient, 22 MB for 256^2 elements of degree 4).
 #pragma once
 
 #include "space.h"
@@ -26,6 +31,7 @@ struct QuadTerm {
     bool consecutive = false;         // every element's window starts one coefficient after the last one's
     // per axis: first basis index per element, basis values [e][q][a], weights [e][q], points [e][q]
     DevBuf off[3], N32[3], N64[3], w64[3], x64[3], w32[3], x32[3];
+    DevBuf st64, st32;                // 2D stencil (quad2_entries() per coefficient, entry-major)
     void build(const Space &s, int nsoft_, const double *soft_);
     // y += coef * V_q x (complex coef; prec TDZ_FP32 or FP64 vectors)
     void apply(cd coef, int prec, const void *x, void *y, cudaStream_t st) const;
