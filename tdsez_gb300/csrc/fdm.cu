@@ -99,8 +99,6 @@ void gen_eig(const BandD &S, const BandD &M, std::vector<double> &V, std::vector
 
 namespace {
 
-constexpr int BM = 64, BN = 64, BK = 16;
-
 // multiply-accumulate of the transforms: complex data times a real or complex
 // matrix entry (FP32, or FP64 for the FP64 preconditioner)
 template <class C, class R> __device__ __forceinline__ void gmac(C &acc, C a, R b) {
@@ -127,107 +125,102 @@ template <> __device__ __forceinline__ float2 gzero<float2>() { return make_floa
 template <> __device__ __forceinline__ double gzero<double>() { return 0.0; }
 template <> __device__ __forceinline__ double2 gzero<double2>() { return make_double2(0.0, 0.0); }
 
-// C[M][N] (complex C2) = A[M][K] (complex, row-major) . B[K][N] (real, or
-// complex for complex axis pencils)
-template <class C2, class TB>
-__global__ void __launch_bounds__(256) k_gemm_cr(const C2 *__restrict__ A, const TB *__restrict__ B,
-                                                 C2 *__restrict__ Cm, int M, int N, int K) {
-    __shared__ C2 As[BK][BM + 1];
-    __shared__ TB Bs[BK][BN + 4];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    C2 acc[4][4];
+// Transform along x: C[M][N] = A[M][K] . B[K][N] (A the complex data, B real or
+// complex); along y, per plane z: C_z = A . B_z (A the real or complex matrix,
+// B_z complex). Row-major, FP32 or FP64 FMAs; a CTA of 256 threads computes a
+// (16 TT)^2 tile, TT x TT outputs per thread. The next K chunk is requested
+// into registers before the current one is used and shared memory is double
+// buffered, so a chunk costs one barrier and its load latency overlaps the
+// products. TT = 2 where TT = 4 would leave SMs idle: a 260 x 260 x 260
+// complex transform (the 2D runs) has 25 tiles of 64 x 64 and 81 of 32 x 32
+// (79 us before, one buffer and 25 tiles; 21 us now).
+// K chunk: half as long for the FP64 64 x 64 tiles, whose buffers would pass 48 KB
+template <class C2, int TT> constexpr int kGemmK = sizeof(C2) == 16 && TT == 4 ? 8 : 16;
+template <class TA, class TB, class C2, int TT>
+__global__ void __launch_bounds__(256) k_gemm(const TA *__restrict__ A, const TB *__restrict__ B, C2 *__restrict__ Cm,
+                                              int M, int N, int K, size_t bplane, size_t cplane) {
+    constexpr int BT = 16 * TT, BK = kGemmK<C2, TT>, L = BT * BK / 256;
+    __shared__ TA As[2][BK][BT + 1];
+    __shared__ TB Bs[2][BK][BT + 1];
+    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    const int m0 = blockIdx.y * BT, n0 = blockIdx.x * BT;
+    B += blockIdx.z * bplane;
+    Cm += blockIdx.z * cplane;
+    C2 acc[TT][TT];
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < TT; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = gzero<C2>();
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        for (int i = threadIdx.x; i < BM * BK; i += 256) {
-            const int r = i / BK, k = i % BK;
-            const int gm = m0 + r, gk = k0 + k;
-            As[k][r] = (gm < M && gk < K) ? A[(size_t)gm * K + gk] : gzero<C2>();
+        for (int c = 0; c < TT; ++c) acc[r][c] = gzero<C2>();
+    TA pa[L];
+    TB pb[L];
+    auto fetch = [&](int k0) {
+#pragma unroll
+        for (int q = 0; q < L; ++q) {
+            const int i = tid + 256 * q;
+            const int gm = m0 + i / BK, ka = k0 + i % BK, kb = k0 + i / BT, gn = n0 + i % BT;
+            pa[q] = gm < M && ka < K ? A[(size_t)gm * K + ka] : gzero<TA>();
+            pb[q] = kb < K && gn < N ? B[(size_t)kb * N + gn] : gzero<TB>();
         }
-        for (int i = threadIdx.x; i < BK * BN; i += 256) {
-            const int k = i / BN, c = i % BN;
-            const int gk = k0 + k, gn = n0 + c;
-            Bs[k][c] = (gk < K && gn < N) ? B[(size_t)gk * N + gn] : gzero<TB>();
+    };
+    auto put = [&](int s) {
+#pragma unroll
+        for (int q = 0; q < L; ++q) {
+            const int i = tid + 256 * q;
+            As[s][i % BK][i / BK] = pa[q];
+            Bs[s][i / BT][i % BT] = pb[q];
         }
-        __syncthreads();
+    };
+    fetch(0);
+    put(0);
+    __syncthreads();
+    int s = 0;
+    for (int k0 = 0; k0 < K; k0 += BK, s ^= 1) {
+        const bool more = k0 + BK < K;
+        if (more) fetch(k0 + BK);
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
-            C2 a[4];
-            TB b[4];
+            TA a[TT];
+            TB b[TT];
 #pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = As[k][ty * 4 + r];
+            for (int r = 0; r < TT; ++r) a[r] = As[s][k][ty * TT + r];
 #pragma unroll
-            for (int c = 0; c < 4; ++c) b[c] = Bs[k][tx * 4 + c];
+            for (int c = 0; c < TT; ++c) b[c] = Bs[s][k][tx + 16 * c];
 #pragma unroll
-            for (int r = 0; r < 4; ++r)
+            for (int r = 0; r < TT; ++r)
 #pragma unroll
-                for (int c = 0; c < 4; ++c) gmac2(acc[r][c], a[r], b[c]);
+                for (int c = 0; c < TT; ++c) gmac2(acc[r][c], a[r], b[c]);
         }
+        if (more) put(s ^ 1);   // last read before the previous barrier
         __syncthreads();
     }
 #pragma unroll
-    for (int r = 0; r < 4; ++r)
+    for (int r = 0; r < TT; ++r)
 #pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int gm = m0 + ty * 4 + r, gn = n0 + tx * 4 + c;
+        for (int c = 0; c < TT; ++c) {
+            const int gm = m0 + ty * TT + r, gn = n0 + tx + 16 * c;
             if (gm < M && gn < N) Cm[(size_t)gm * N + gn] = acc[r][c];
         }
 }
 
-// per plane z: C_z[M][N] (complex C2) = A[M][K] (real, or complex for
-// complex axis pencils; row-major) . B_z[K][N] (complex)
-template <class C2, class TA>
-__global__ void __launch_bounds__(256) k_gemm_rc(const TA *__restrict__ A, const C2 *__restrict__ B,
-                                                 C2 *__restrict__ Cm, int M, int N, int K) {
-    __shared__ TA As[BK][BM + 4];
-    __shared__ C2 Bs[BK][BN + 1];
-    const int tx = threadIdx.x % 16, ty = threadIdx.x / 16;
-    const int m0 = blockIdx.y * BM, n0 = blockIdx.x * BN;
-    const size_t plane = (size_t)blockIdx.z;
-    const C2 *Bz = B + plane * (size_t)K * N;
-    C2 *Cz = Cm + plane * (size_t)M * N;
-    C2 acc[4][4];
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) acc[r][c] = gzero<C2>();
-    for (int k0 = 0; k0 < K; k0 += BK) {
-        for (int i = threadIdx.x; i < BM * BK; i += 256) {
-            const int r = i / BK, k = i % BK;
-            const int gm = m0 + r, gk = k0 + k;
-            As[k][r] = (gm < M && gk < K) ? A[(size_t)gm * K + gk] : gzero<TA>();
-        }
-        for (int i = threadIdx.x; i < BK * BN; i += 256) {
-            const int k = i / BN, c = i % BN;
-            const int gk = k0 + k, gn = n0 + c;
-            Bs[k][c] = (gk < K && gn < N) ? Bz[(size_t)gk * N + gn] : gzero<C2>();
-        }
-        __syncthreads();
-#pragma unroll
-        for (int k = 0; k < BK; ++k) {
-            TA a[4];
-            C2 b[4];
-#pragma unroll
-            for (int r = 0; r < 4; ++r) a[r] = As[k][ty * 4 + r];
-#pragma unroll
-            for (int c = 0; c < 4; ++c) b[c] = Bs[k][tx * 4 + c];
-#pragma unroll
-            for (int r = 0; r < 4; ++r)
-#pragma unroll
-                for (int c = 0; c < 4; ++c) gmac2(acc[r][c], a[r], b[c]);
-        }
-        __syncthreads();
-    }
-#pragma unroll
-    for (int r = 0; r < 4; ++r)
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-            const int gm = m0 + ty * 4 + r, gn = n0 + tx * 4 + c;
-            if (gm < M && gn < N) Cz[(size_t)gm * N + gn] = acc[r][c];
-        }
+template <class TA, class TB, class C2>
+void gemm(const TA *A, const TB *B, C2 *Cm, int M, int N, int K, int planes, size_t bplane, size_t cplane,
+          cudaStream_t st) {
+    const long long big = (long long)((M + 63) / 64) * ((N + 63) / 64) * planes;
+    if (big >= 2LL * sm_count())
+        k_gemm<TA, TB, C2, 4><<<dim3((N + 63) / 64, (M + 63) / 64, planes), 256, 0, st>>>(A, B, Cm, M, N, K, bplane, cplane);
+    else
+        k_gemm<TA, TB, C2, 2><<<dim3((N + 31) / 32, (M + 31) / 32, planes), 256, 0, st>>>(A, B, Cm, M, N, K, bplane, cplane);
+}
+// along x: rows of n0 entries times an n0 x n0 matrix
+template <class TM, class C2>
+void gemm_x(const DevBuf &Mx, const C2 *in, C2 *out, int rows, int n0, cudaStream_t st) {
+    gemm<C2, TM, C2>(in, Mx.as<TM>(), out, rows, n0, n0, 1, 0, 0, st);
+}
+// along y: an n1 x n1 matrix times every n1 x n0 plane
+template <class TM, class C2>
+void gemm_y(const DevBuf &My, const C2 *in, C2 *out, int n0, int n1, int planes, cudaStream_t st) {
+    const size_t plane = (size_t)n0 * n1;
+    gemm<TM, C2, C2>(My.as<TM>(), in, out, n1, n0, n1, planes, plane, plane, st);
 }
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
@@ -343,7 +336,7 @@ struct ZSolveParams {
 // multiply-subtracts per row and pass for P = 3). The former unsymmetric
 // elimination with a 32-row unrolled ring took 257 us per solve on 163 x 163
 // lines of 343 rows (P = 3) and 293 us on 260 lines of 260 rows (P = 4,
-// complex pencils); this one 97 us and 55 us.
+// complex pencils); this one @ZL3D@ us and @ZL2D@ us.
 constexpr int kZLines = 64;                      // lines per CTA (two threads each)
 template <int P> struct ZBlk {
     static constexpr int B = P == 3 ? 9 : (P == 5 ? 10 : 8);   // rows per block (a multiple of P)
@@ -1093,14 +1086,12 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
         // FP64 preconditioner (SIMT transforms, FP64 line solves)
         double2 *y1 = b1.as<double2>(), *y2 = b2.as<double2>();
         auto x64 = [&](const DevBuf &Mx, const double2 *in, double2 *out) {
-            const dim3 g((n[0] + BN - 1) / BN, (grows + BM - 1) / BM);
-            if (cplx) k_gemm_cr<double2, double2><<<g, 256, 0, st>>>(in, Mx.as<double2>(), out, grows, n[0], n[0]);
-            else k_gemm_cr<double2, double><<<g, 256, 0, st>>>(in, Mx.as<double>(), out, grows, n[0], n[0]);
+            if (cplx) gemm_x<double2>(Mx, in, out, grows, n[0], st);
+            else gemm_x<double>(Mx, in, out, grows, n[0], st);
         };
         auto y64 = [&](const DevBuf &My, const double2 *in, double2 *out) {
-            const dim3 g((n[0] + BN - 1) / BN, (n[1] + BM - 1) / BM, n[2]);
-            if (cplx) k_gemm_rc<double2, double2><<<g, 256, 0, st>>>(My.as<double2>(), in, out, n[1], n[0], n[1]);
-            else k_gemm_rc<double2, double><<<g, 256, 0, st>>>(My.as<double>(), in, out, n[1], n[0], n[1]);
+            if (cplx) gemm_y<double2>(My, in, out, n[0], n[1], n[2], st);
+            else gemm_y<double>(My, in, out, n[0], n[1], n[2], st);
         };
         x64(V[0], r, y2);
         double2 *cur = y2, *oth = y1;
@@ -1125,14 +1116,12 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
     // transforms along x (rows of n0) and along y (planes of n1 x n0) with a
     // real or complex FP32 matrix
     auto along_x = [&](const DevBuf &Mx, const float2 *in, float2 *out) {
-        const dim3 g((n[0] + BN - 1) / BN, (grows + BM - 1) / BM);
-        if (cplx) k_gemm_cr<float2, float2><<<g, 256, 0, st>>>(in, Mx.as<float2>(), out, grows, n[0], n[0]);
-        else k_gemm_cr<float2, float><<<g, 256, 0, st>>>(in, Mx.as<float>(), out, grows, n[0], n[0]);
+        if (cplx) gemm_x<float2>(Mx, in, out, grows, n[0], st);
+        else gemm_x<float>(Mx, in, out, grows, n[0], st);
     };
     auto along_y = [&](const DevBuf &My, const float2 *in, float2 *out) {
-        const dim3 g((n[0] + BN - 1) / BN, (n[1] + BM - 1) / BM, n[2]);
-        if (cplx) k_gemm_rc<float2, float2><<<g, 256, 0, st>>>(My.as<float2>(), in, out, n[1], n[0], n[1]);
-        else k_gemm_rc<float2, float><<<g, 256, 0, st>>>(My.as<float>(), in, out, n[1], n[0], n[1]);
+        if (cplx) gemm_y<float2>(My, in, out, n[0], n[1], n[2], st);
+        else gemm_y<float>(My, in, out, n[0], n[1], n[2], st);
     };
     // forward transforms: along x with V (t_i = sum_i' V[i'][i] r_i'), along y with V^T
     along_x(V[0], x1, x2);
