@@ -190,28 +190,22 @@ void launch_1d(const ApplyParams<T> &prm, cudaStream_t st) {
 
 }  // namespace
 
-// sum of the fused-reduction partials, one block, fixed order
-__global__ void k_apply_red_finish(const double2 *part, int n, double2 *out) {
-    __shared__ double2 s[256];
+// sum of the fused-reduction partials, one CTA, fixed order
+constexpr int kRedThreads = 512;
+__global__ void __launch_bounds__(kRedThreads) k_apply_red_finish(const double2 *part, double2 *out) {
     double2 t = make_double2(0.0, 0.0);
-    for (int i = threadIdx.x; i < n; i += blockDim.x) {
-        t.x += part[i].x;
-        t.y += part[i].y;
+#pragma unroll
+    for (int i = threadIdx.x; i < kApplyRedCap; i += kRedThreads) {
+        const double2 v = part[i];
+        t.x += v.x;
+        t.y += v.y;
     }
-    s[threadIdx.x] = t;
-    __syncthreads();
-    for (int h = blockDim.x / 2; h > 0; h >>= 1) {
-        if ((int)threadIdx.x < h) {
-            s[threadIdx.x].x += s[threadIdx.x + h].x;
-            s[threadIdx.x].y += s[threadIdx.x + h].y;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = s[0];
+    t = block_sum<kRedThreads>(t.x, t.y);
+    if (threadIdx.x == 0) *out = t;
 }
 
 void apply_red_finish(const double2 *part, double2 *out, cudaStream_t st) {
-    k_apply_red_finish<<<1, 256, 0, st>>>(part, kApplyRedCap, out);
+    k_apply_red_finish<<<1, kRedThreads, 0, st>>>(part, out);
     TDZ_CUDA(cudaGetLastError());
     count_launch();
 }

@@ -49,15 +49,15 @@ template <class MC> struct IsF64Mem { static constexpr bool v = std::is_same<MC,
 // FP64 -> FP32 keeping the leading 24 significand bits (truncation, relative
 // error below 2^-23) with integer operations; |v| < 2^-100 gives 0, values
 // beyond the FP32 range a non-finite result
-__device__ __forceinline__ float d2f_trunc(double v) {
-    const unsigned long long u = (unsigned long long)__double_as_longlong(v);
-    const unsigned int h32 = (unsigned int)(u >> 32);
+__device__ __forceinline__ float d2f_trunc(double v) {   // the high part of dff_split
+    const unsigned int h32 = (unsigned int)__double2hiint(v), l32 = (unsigned int)__double2loint(v);
     const unsigned int sign = h32 & 0x80000000u;
-    const int e = (int)((h32 >> 20) & 0x7FFu) - 1023;
-    if (e < -100) return __uint_as_float(sign);
-    if (e > 127) return __uint_as_float(sign | 0x7F800000u | (e == 1024 && (u << 12) ? 0x400000u : 0u));
-    const unsigned int m23 = ((h32 & 0xFFFFFu) << 3) | ((unsigned int)u >> 29);
-    return __uint_as_float(sign | ((unsigned int)(e + 127) << 23) | m23);
+    const unsigned int hb = ((__funnelshift_l(l32, h32, 3) ^ 0x40000000u) & 0x7FFFFFFFu) | sign;
+    const unsigned int above = (h32 & 0x7FFFFFFFu) - ((1023u - 100u) << 20);
+    if (above < (228u << 20)) return __uint_as_float(hb);
+    if ((int)above < 0) return __uint_as_float(sign);
+    const bool nan = (h32 & 0x7FF00000u) == 0x7FF00000u && ((h32 & 0xFFFFFu) | l32);
+    return __uint_as_float(sign | (nan ? 0x7FC00000u : 0x7F800000u));
 }
 
 // memory complex -> arithmetic complex
@@ -81,8 +81,7 @@ template <> __device__ __forceinline__ double2 rb_store<double2, cdff>(const cdf
 // sub - v in the arithmetic type (the residual of a fused b - A x)
 template <class C, class MC> __device__ __forceinline__ C rb_sub(const MC &b, C v) {
     C r = rb_load<C, MC>(b);
-    r.x = tfma(decltype(v.x)(-1.f), v.x, r.x);
-    r.y = tfma(decltype(v.y)(-1.f), v.y, r.y);
+    rfma(r, decltype(cre(v))(-1.f), v);
     return cnorm(r);
 }
 
@@ -376,13 +375,13 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
 #pragma unroll
             for (int r = 0; r < R; ++r) {
                 C &a = acc[r][(ring + o) % BW];
-                if constexpr (KA == 1) rfma(a, za.x, wA[r]);
-                else if constexpr (KA == 2) ifma(a, za.y, wA[r]);
+                if constexpr (KA == 1) rfma(a, cre(za), wA[r]);
+                else if constexpr (KA == 2) ifma(a, cim(za), wA[r]);
                 else cfma(a, za, wA[r]);
                 if constexpr (HB) rfma(a, zm, wB[r]);
                 if constexpr (HC) {
-                    if constexpr (KC == 1) rfma(a, zc.x, wC[r]);
-                    else if constexpr (KC == 2) ifma(a, zc.y, wC[r]);
+                    if constexpr (KC == 1) rfma(a, cre(zc), wC[r]);
+                    else if constexpr (KC == 2) ifma(a, cim(zc), wC[r]);
                     else cfma(a, zc, wC[r]);
                 }
             }

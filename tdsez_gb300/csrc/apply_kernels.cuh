@@ -82,13 +82,13 @@ __device__ __forceinline__ MC out_value_sub(const ApplyParams<T> &prm, MC b, C v
 // entry o of row i of a combination of base bands
 template <class T, class C>
 __device__ __forceinline__ C comb_at(const CombP<T> &cb, const T *bands, int n, int bw, int i, int o) {
-    C z = czero<C>();
+    T re = T(0), im = T(0);
     for (int t = 0; t < cb.n; ++t) {
         const T b = bands[((size_t)cb.base[t] * n + i) * bw + o];
-        z.x = tfma(cb.re[t], b, z.x);
-        z.y = tfma(cb.im[t], b, z.y);
+        re = tfma(cb.re[t], b, re);
+        im = tfma(cb.im[t], b, im);
     }
-    return cnorm(z);
+    return cnorm(cmake<C, T>(re, im));
 }
 
 // ---------------------------------------------------------------- 3D kernel
@@ -242,14 +242,14 @@ __device__ __noinline__ double2 apply3d_run(const ApplyParams<T> &prm, int x0, i
 #pragma unroll
         for (int o = 0; o < BW; ++o) {
             C &a = acc[(ring + o) % BW];
-            if constexpr (KA == 1) rfma(a, zA[o].x, wA);
-            else if constexpr (KA == 2) ifma(a, zA[o].y, wA);
+            if constexpr (KA == 1) rfma(a, cre(zA[o]), wA);
+            else if constexpr (KA == 2) ifma(a, cim(zA[o]), wA);
             else cfma(a, zA[o], wA);
             if constexpr (HB) rfma(a, sZM[(size_t)it * BW + o], wB);
             if constexpr (HC) {
                 const C zc = sZC[(size_t)it * BW + o];
-                if constexpr (KC == 1) rfma(a, zc.x, wC);
-                else if constexpr (KC == 2) ifma(a, zc.y, wC);
+                if constexpr (KC == 1) rfma(a, cre(zc), wC);
+                else if constexpr (KC == 2) ifma(a, cim(zc), wC);
                 else cfma(a, zc, wC);
             }
         }
@@ -404,7 +404,7 @@ template <int BW, class C> __device__ __forceinline__ C dot_kind(const C (&a)[BW
     C s = czero<C>();
     if (kind == 2) {
 #pragma unroll
-        for (int j = 0; j < BW; ++j) ifma(s, a[j].y, v[j * stride]);
+        for (int j = 0; j < BW; ++j) ifma(s, cim(a[j]), v[j * stride]);
     } else {
 #pragma unroll
         for (int j = 0; j < BW; ++j) cfma(s, a[j], v[j * stride]);

@@ -19,6 +19,11 @@ namespace {
 constexpr int kThreads = 256;
 // about 8 CTAs per SM: latency hiding for the double-float dots
 inline int red_blocks() { return 8 * sm_count(); }
+// CTAs of a reduction over n: two elements per thread before more CTAs, since
+// a CTA's cross-thread sums and its partial cost more than an element
+inline int red_grid(size_t n, int cap) {
+    return (int)std::min<size_t>((size_t)cap, std::max<size_t>(1, (n + 2 * kThreads - 1) / (2 * kThreads)));
+}
 
 inline int grid_for(size_t n) {
     const size_t b = (n + kThreads - 1) / kThreads;
@@ -87,11 +92,46 @@ inline CoefDF coef_df(const CoefPack &cp, int k) {
 
 __device__ __forceinline__ cdff ld_df(const double2 &v) { return load_c<cdff>(v); }
 __device__ __forceinline__ double2 st_df(const cdff &c) { return store_c<double2>(c); }
-__host__ __device__ inline cdff mk_df(dff re, dff im) {
-    cdff c;
-    c.x = re;
-    c.y = im;
-    return c;
+__host__ __device__ inline cdff mk_df(dff re, dff im) { return make_cdff(re, im); }
+
+// a + b, renormalised (both components)
+__device__ __forceinline__ cdff add_df(const cdff &a, const cdff &b) {
+    const float2 s = __fadd2_rn(a.hi, b.hi), bv = sub2(s, a.hi);
+    const float2 err = __fadd2_rn(sub2(a.hi, sub2(s, bv)), sub2(b.hi, bv));
+    cdff r;
+    r.hi = s;
+    r.lo = __fadd2_rn(__fadd2_rn(a.lo, b.lo), err);
+    return cnorm(r);
+}
+// CTA sums of R double-float accumulators into partial[i][block]: within a
+// warp in double-float on the FP32 pipes, across warps in FP64. (FP64 shuffles
+// for every warp cost more than the sums themselves: GB300 issues an FP64
+// instruction of a warp in 16 clocks of the whole SM, and 1216 CTAs with five
+// results spent 27 us in this tail alone.)
+template <int R> __device__ __forceinline__ void cta_partials(cdff (&acc)[R], double2 *partial) {
+    __shared__ double2 red[kThreads / 32][R];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        cdff v = cnorm(acc[i]);
+#pragma unroll
+        for (int off = 16; off > 0; off >>= 1) {
+            cdff o;
+            o.hi.x = __shfl_down_sync(0xffffffffu, v.hi.x, off);
+            o.hi.y = __shfl_down_sync(0xffffffffu, v.hi.y, off);
+            o.lo.x = __shfl_down_sync(0xffffffffu, v.lo.x, off);
+            o.lo.y = __shfl_down_sync(0xffffffffu, v.lo.y, off);
+            v = add_df(v, o);
+        }
+        if (lane == 0) red[warp][i] = make_double2(dff_to_double(v.re()), dff_to_double(v.im()));
+    }
+    __syncthreads();
+    if (threadIdx.x < R) {
+        double re = 0.0, im = 0.0;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) { re += red[w][threadIdx.x].x; im += red[w][threadIdx.x].y; }
+        partial[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = make_double2(re, im);
+    }
 }
 
 template <int K>
@@ -104,23 +144,7 @@ __global__ void __launch_bounds__(kThreads) k_mdot_df(PtrPack V, const double2 *
 #pragma unroll
         for (int i = 0; i < K; ++i) cfma_conj(acc[i], ld_df(static_cast<const double2 *>(V.p[i])[e]), wv);
     }
-    __shared__ double2 red[kThreads / 32][K];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int i = 0; i < K; ++i) {
-        double re = dff_to_double(acc[i].x), im = dff_to_double(acc[i].y);
-        for (int off = 16; off > 0; off >>= 1) {
-            re += __shfl_down_sync(0xffffffffu, re, off);
-            im += __shfl_down_sync(0xffffffffu, im, off);
-        }
-        if (lane == 0) red[warp][i] = make_double2(re, im);
-    }
-    __syncthreads();
-    if (threadIdx.x < K) {
-        double re = 0.0, im = 0.0;
-        for (int w2 = 0; w2 < kThreads / 32; ++w2) { re += red[w2][threadIdx.x].x; im += red[w2][threadIdx.x].y; }
-        partial[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = make_double2(re, im);
-    }
+    cta_partials<K>(acc, partial);
 }
 
 // w += sum_i a_i V_i: the increment in double-float, the final add in FP64,
@@ -132,8 +156,8 @@ __global__ void k_maxpy_df(double2 *w, PtrPack V, CoefDF a, size_t n) {
 #pragma unroll
         for (int i = 0; i < K; ++i) cfma(acc, mk_df(a.re[i], a.im[i]), ld_df(static_cast<const double2 *>(V.p[i])[e]));
         double2 v = w[e];
-        v.x += dff_to_double(acc.x);
-        v.y += dff_to_double(acc.y);
+        v.x += dff_to_double(acc.re());
+        v.y += dff_to_double(acc.im());
         w[e] = v;
     }
 }
@@ -156,7 +180,7 @@ __global__ void k_cn_combine(double2 *psi, const double2 *x, const double2 *z, c
         cdff t = czero<cdff>();
         cfma(t, c, ld_df(z[i]));
         const double2 xv = x[i], pv = psi[i];
-        psi[i] = make_double2(fma(2.0, xv.x, -pv.x) + dff_to_double(t.x), fma(2.0, xv.y, -pv.y) + dff_to_double(t.y));
+        psi[i] = make_double2(fma(2.0, xv.x, -pv.x) + dff_to_double(t.re()), fma(2.0, xv.y, -pv.y) + dff_to_double(t.im()));
     }
 }
 
@@ -192,7 +216,7 @@ __global__ void k_scale_df(double2 *x, cdff a, size_t n) {
 __global__ void k_cast64to32_df(const double2 *x, float2 *y, size_t n) {
     for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < n; i += (size_t)gridDim.x * blockDim.x) {
         const cdff v = ld_df(x[i]);
-        y[i] = make_float2(__fadd_rn(v.x.hi, v.x.lo), __fadd_rn(v.y.hi, v.y.lo));
+        y[i] = __fadd2_rn(v.hi, v.lo);
     }
 }
 
@@ -238,25 +262,14 @@ __global__ void __launch_bounds__(kThreads) k_gs_df(double2 *w, PtrPack V, CoefD
 #pragma unroll
             for (int i = 0; i < K; ++i) cfma_conj(acc[i], v[i], x);
         }
-        if constexpr (MODE != 0) cfma_conj(acc[R - 1], x, x);
+        if constexpr (MODE != 0) fma2(acc[R - 1], x.hi, x.lo, x.hi, x.lo);
     }
-    __shared__ double2 red[kThreads / 32][R];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-#pragma unroll
-    for (int i = 0; i < R; ++i) {
-        double re = dff_to_double(acc[i].x), im = dff_to_double(acc[i].y);
-        for (int off = 16; off > 0; off >>= 1) {
-            re += __shfl_down_sync(0xffffffffu, re, off);
-            im += __shfl_down_sync(0xffffffffu, im, off);
-        }
-        if (lane == 0) red[warp][i] = make_double2(re, im);
+    // |w|^2: the sums of the squares of the real and of the imaginary parts
+    if constexpr (MODE != 0) {
+        const cdff t = cnorm(acc[R - 1]);
+        acc[R - 1] = add_df(make_cdff(t.re(), dff(0.f)), make_cdff(t.im(), dff(0.f)));
     }
-    __syncthreads();
-    if (threadIdx.x < R) {
-        double re = 0.0, im = 0.0;
-        for (int w2 = 0; w2 < kThreads / 32; ++w2) { re += red[w2][threadIdx.x].x; im += red[w2][threadIdx.x].y; }
-        partial[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = make_double2(re, im);
-    }
+    cta_partials<R>(acc, partial);
 }
 
 // per-block partial sums of conj(V_i) w, i < k; partial layout [i][block]
@@ -297,25 +310,18 @@ __global__ void __launch_bounds__(kThreads) k_mdot(PtrPack V, const typename CT<
     }
 }
 
-// result[i] = sum over blocks of partial[i][block] (one block per i, fixed order)
-__global__ void k_finish(const double2 *partial, int blocks, double2 *result) {
-    __shared__ double2 red[kThreads];
+// result[i] = sum over blocks of partial[i][block] (one CTA per i, fixed order)
+__global__ void __launch_bounds__(kThreads) k_finish(const double2 *partial, int blocks, double2 *result) {
     const int i = blockIdx.x;
     double re = 0.0, im = 0.0;
-    for (int b = threadIdx.x; b < blocks; b += blockDim.x) {
-        re += partial[(size_t)i * blocks + b].x;
-        im += partial[(size_t)i * blocks + b].y;
+#pragma unroll 4
+    for (int b = threadIdx.x; b < blocks; b += kThreads) {
+        const double2 v = partial[(size_t)i * blocks + b];
+        re += v.x;
+        im += v.y;
     }
-    red[threadIdx.x] = make_double2(re, im);
-    __syncthreads();
-    for (int s = blockDim.x / 2; s > 0; s >>= 1) {
-        if (threadIdx.x < s) {
-            red[threadIdx.x].x += red[threadIdx.x + s].x;
-            red[threadIdx.x].y += red[threadIdx.x + s].y;
-        }
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) result[i] = red[0];
+    const double2 t = block_sum<kThreads>(re, im);
+    if (threadIdx.x == 0) result[i] = t;
 }
 
 template <class T, int K>
@@ -462,9 +468,10 @@ void mdot(Reducer &r, const void *const *V, int k, const void *w, size_t n, int 
         const int kk = std::min(kMaxDot, k - c0);
         PtrPack pp{};
         for (int i = 0; i < kk; ++i) pp.p[i] = V[c0 + i];
-        if (prec == TDZ_FP64) mdot_dispatch<double>(kk, pp, w, n, r.partial.as<double2>(), r.blocks, st);
-        else mdot_dispatch<float>(kk, pp, w, n, r.partial.as<double2>(), r.blocks, st);
-        k_finish<<<kk, kThreads, 0, st>>>(r.partial.as<double2>(), r.blocks, r.result.as<double2>());
+        const int nb = red_grid(n, r.blocks);
+        if (prec == TDZ_FP64) mdot_dispatch<double>(kk, pp, w, n, r.partial.as<double2>(), nb, st);
+        else mdot_dispatch<float>(kk, pp, w, n, r.partial.as<double2>(), nb, st);
+        k_finish<<<kk, kThreads, 0, st>>>(r.partial.as<double2>(), nb, r.result.as<double2>());
         TDZ_CUDA(cudaGetLastError());
     count_launch();
         TDZ_CUDA(cudaMemcpyAsync(r.host, r.result.ptr, sizeof(double2) * kk, cudaMemcpyDeviceToHost, st));
@@ -477,9 +484,10 @@ void dot_device(Reducer &r, const void *x, const void *y, size_t n, int prec, do
     r.init();
     PtrPack pp{};
     pp.p[0] = x;
-    if (prec == TDZ_FP64) mdot_dispatch<double>(1, pp, y, n, r.partial.as<double2>(), r.blocks, st);
-    else mdot_dispatch<float>(1, pp, y, n, r.partial.as<double2>(), r.blocks, st);
-    k_finish<<<1, kThreads, 0, st>>>(r.partial.as<double2>(), r.blocks, out);
+    const int nb = red_grid(n, r.blocks);
+    if (prec == TDZ_FP64) mdot_dispatch<double>(1, pp, y, n, r.partial.as<double2>(), nb, st);
+    else mdot_dispatch<float>(1, pp, y, n, r.partial.as<double2>(), nb, st);
+    k_finish<<<1, kThreads, 0, st>>>(r.partial.as<double2>(), nb, out);
     TDZ_CUDA(cudaGetLastError());
     count_launch(2);
 }
@@ -489,6 +497,7 @@ void mdot_partials(const void *const *V, int k, const void *w, size_t n, int pre
     TDZ_CHECK(k >= 1 && k <= kMaxDot, TDZ_ERR_INTERNAL, "bad multi-dot width");
     PtrPack pp{};
     for (int i = 0; i < k; ++i) pp.p[i] = V[i];
+    blocks = red_grid(n, blocks);
     if (prec == TDZ_FP64) mdot_dispatch<double>(k, pp, w, n, partial, blocks, st);
     else mdot_dispatch<float>(k, pp, w, n, partial, blocks, st);
     k_finish<<<k, kThreads, 0, st>>>(partial, blocks, out);
@@ -528,12 +537,13 @@ void gs_update(Reducer &r, void *w, int k, const void *const *V, const cd *a, si
     const CoefDF cd_ = coef_df(cp, k);
     double2 *wp = static_cast<double2 *>(w);
     double2 *part = r.partial.as<double2>();
+    const int nb = red_grid(n, r.blocks);
     switch (k) {
 #define TDZ_CASE(K)                                                                                       \
     case K:                                                                                               \
-        if (dots && norm) k_gs_df<K, 2><<<r.blocks, kThreads, 0, st>>>(wp, pp, cd_, n, part);             \
-        else if (norm) k_gs_df<K, 1><<<r.blocks, kThreads, 0, st>>>(wp, pp, cd_, n, part);               \
-        else k_gs_df<K, 0><<<r.blocks, kThreads, 0, st>>>(wp, pp, cd_, n, part);                         \
+        if (dots && norm) k_gs_df<K, 2><<<nb, kThreads, 0, st>>>(wp, pp, cd_, n, part);             \
+        else if (norm) k_gs_df<K, 1><<<nb, kThreads, 0, st>>>(wp, pp, cd_, n, part);               \
+        else k_gs_df<K, 0><<<nb, kThreads, 0, st>>>(wp, pp, cd_, n, part);                         \
         break;
         TDZ_CASE(1) TDZ_CASE(2) TDZ_CASE(3) TDZ_CASE(4) TDZ_CASE(5) TDZ_CASE(6) TDZ_CASE(7) TDZ_CASE(8)
         TDZ_CASE(9) TDZ_CASE(10) TDZ_CASE(11) TDZ_CASE(12) TDZ_CASE(13) TDZ_CASE(14) TDZ_CASE(15) TDZ_CASE(16)
@@ -541,7 +551,7 @@ void gs_update(Reducer &r, void *w, int k, const void *const *V, const cd *a, si
     default: break;
     }
     const int nres = (dots ? k : 0) + (norm ? 1 : 0);
-    k_finish<<<nres, kThreads, 0, st>>>(part, r.blocks, r.result.as<double2>());
+    k_finish<<<nres, kThreads, 0, st>>>(part, nb, r.result.as<double2>());
     TDZ_CUDA(cudaGetLastError());
     count_launch(2);
     TDZ_CUDA(cudaMemcpyAsync(r.host, r.result.ptr, sizeof(double2) * nres, cudaMemcpyDeviceToHost, st));

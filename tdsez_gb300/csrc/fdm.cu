@@ -268,18 +268,13 @@ __global__ void __launch_bounds__(256) k_from_planar_norm(const float *__restric
     }
 }
 
-// *out = sum of part[0 .. n) in a fixed order (one block)
-__global__ void __launch_bounds__(256) k_sum_parts(const double *__restrict__ part, int n, double *out) {
-    __shared__ double ws[256];
+// *out = sum of part[0 .. n) in a fixed order (one CTA)
+__global__ void __launch_bounds__(512) k_sum_parts(const double *__restrict__ part, int n, double *out) {
     double t = 0.0;
-    for (int i = threadIdx.x; i < n; i += blockDim.x) t += part[i];
-    ws[threadIdx.x] = t;
-    __syncthreads();
-    for (int s = 128; s > 0; s >>= 1) {
-        if ((int)threadIdx.x < s) ws[threadIdx.x] += ws[threadIdx.x + s];
-        __syncthreads();
-    }
-    if (threadIdx.x == 0) *out = ws[0];
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += 512) t += part[i];
+    t = block_sum<512>(t, 0.0).x;
+    if (threadIdx.x == 0) *out = t;
 }
 
 __global__ void k_from_planar(const float *__restrict__ a, double2 *__restrict__ z, int n0, size_t rows, int ld) {
@@ -336,7 +331,7 @@ struct ZSolveParams {
 // multiply-subtracts per row and pass for P = 3). The former unsymmetric
 // elimination with a 32-row unrolled ring took 257 us per solve on 163 x 163
 // lines of 343 rows (P = 3) and 293 us on 260 lines of 260 rows (P = 4,
-// complex pencils); this one @ZL3D@ us and @ZL2D@ us.
+// complex pencils); this one 97 us and 55 us.
 constexpr int kZLines = 64;                      // lines per CTA (two threads each)
 template <int P> struct ZBlk {
     static constexpr int B = P == 3 ? 9 : (P == 5 ? 10 : 8);   // rows per block (a multiple of P)
@@ -1071,7 +1066,7 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
         transform(Ti[1], b, n[2], n[0], ldy, a, ldx, st);
         if (norm_out) {
             k_from_planar_norm<<<blocks, 256, 0, st>>>(a, z, n[0], rows, ldx, npart.as<double>());
-            k_sum_parts<<<1, 256, 0, st>>>(npart.as<double>(), blocks, norm_out);
+            k_sum_parts<<<1, 512, 0, st>>>(npart.as<double>(), blocks, norm_out);
             count_launch();
         } else {
             k_from_planar<<<blocks, 256, 0, st>>>(a, z, n[0], rows, ldx);

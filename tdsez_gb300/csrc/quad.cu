@@ -320,11 +320,12 @@ template <> struct QArith<dff> {
         return v;
     }
     __device__ static void scale(cdff &f, dff w) {
-        f.x = renorm(tfma(f.x, w, dff(0.f)));
-        f.y = renorm(tfma(f.y, w, dff(0.f)));
+        cdff r = czero<cdff>();
+        rfma(r, w, f);
+        f = cnorm(r);
     }
     __device__ static void atomic_out(double2 *dst, cdff a, double cre, double cim) {
-        const double ax = dff_to_double(a.x), ay = dff_to_double(a.y);
+        const double ax = dff_to_double(a.re()), ay = dff_to_double(a.im());
         atomicAdd(&dst->x, cre * ax - cim * ay);
         atomicAdd(&dst->y, cre * ay + cim * ax);
     }

@@ -594,9 +594,7 @@ __global__ void k_axis_dense(const double2 *__restrict__ F, const double2 *__res
         const long long b = t % B, r = t / B;
         const int k = (int)(r % nk);
         const long long a = r / nk;
-        cdff acc;
-        acc.x = dff(0.f);
-        acc.y = dff(0.f);
+        cdff acc = czero<cdff>();
         const double2 *fk = F + (size_t)k * ni;
         const double2 *ia = in + (size_t)a * ni * B + b;
         for (int i = 0; i < ni; ++i) {
