@@ -197,9 +197,12 @@ __device__ __noinline__ double2 apply3d_run(const ApplyParams<T> &prm, int x0, i
         if (it < hi) load_plane(zs + it);
     };
     // x stage of plane it: sIn[it & 1] -> sU[it & 1]
+    // rows of the halo tile that an output row inside the grid reads
+    const int rows_in = min(RY, n1 - y0 + 2 * P);
     auto xstage = [&](int it) {
         const int buf = it & 1;
         for (int r = ty; r < RY; r += TY) {
+            if (r >= rows_in) break;   // nobody reads the rows past the grid's last one
             C uM = czero<C>(), uT = czero<C>(), uS = czero<C>();
 #pragma unroll
             for (int j = 0; j < BW; ++j) {
@@ -261,7 +264,7 @@ __device__ __noinline__ double2 apply3d_run(const ApplyParams<T> &prm, int x0, i
     // buffer a step writes was last read before the previous barrier.
     auto step = [&](int it, int ring) {
         xstage(it + 1);                // a plane past hi leaves results that nobody reads
-        yzstage(it, ring);
+        if (gy < n1) yzstage(it, ring);
         store_in(it + 2);
         fetch(it + 3);
         __syncthreads();
