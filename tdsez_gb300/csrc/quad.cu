@@ -270,32 +270,10 @@ template <class T, int P> void launch_stencil2(const QuadTerm &q, cd coef, const
 // overlap by p coefficients per axis, chunk ends by p planes). Versus one CTA
 // per element: each interpolated plane serves p + 1 elements and the
 // coefficients receive (1 + p/TE)^2 atomic adds instead of (p+1)^3.
-// FP32 arithmetic on FP32 vectors, or double-float arithmetic on FP64
-// vectors (the FGMRES applies: 1/sqrt of the potential by rsqrtf and one
-// Newton step in double-float, about 48 bits).
+// Double-float arithmetic on FP64 vectors (the FGMRES applies: 1/sqrt of the
+// potential by rsqrtf and one Newton step in double-float, about 48 bits);
+// FP32 vectors take the column kernel below.
 template <class A> struct QArith;
-template <> struct QArith<float> {
-    using C = float2;
-    using MC = float2;
-    using TT = float;
-    __device__ static float from(TT v) { return v; }
-    __device__ static float one() { return 1.f; }
-    // -Z / sqrt(r2 + a) summed over the centres at (x, y, z)
-    __device__ static float pot(const QuadParams<TT> &prm, float x, float y, float z) {
-        float v = 0.f;
-        for (int k = 0; k < prm.nsoft; ++k) {
-            const float dx = x - prm.soft[k][1], dy = y - prm.soft[k][2], dz = z - prm.soft[k][3];
-            v -= prm.soft[k][0] * rsqrtf(dx * dx + dy * dy + dz * dz + prm.soft[k][4]);
-        }
-        return v;
-    }
-    __device__ static float mul(float a, float b) { return a * b; }
-    __device__ static void scale(float2 &f, float w) { f.x *= w; f.y *= w; }
-    __device__ static void atomic_out(float2 *dst, float2 a, double cre, double cim) {
-        atomicAdd(&dst->x, (float)cre * a.x - (float)cim * a.y);
-        atomicAdd(&dst->y, (float)cre * a.y + (float)cim * a.x);
-    }
-};
 template <> struct QArith<dff> {
     using C = cdff;
     using MC = double2;
@@ -339,7 +317,7 @@ template <class A, int P, int TE> struct QStream {
 constexpr int kQsThreads = 512;
 // tile side in elements: the two rings of (TE (p+1))^2 points fit the 227 KB of shared memory
 template <class A, int P> constexpr int qs_te() {
-    return std::is_same<A, float>::value ? (P <= 4 ? 8 : 6) : (P <= 3 ? 7 : (P == 4 ? 6 : 4));
+    return P <= 3 ? 7 : (P == 4 ? 6 : 4);
 }
 
 template <class A, int P, int TE>
@@ -492,8 +470,228 @@ __global__ void __launch_bounds__(kQsThreads) k_quad3_stream(const QuadParams<ty
     for (int c = 1; c <= P; ++c) flush_plane(czl + c);
 }
 
+// ---------------------------------------------------------------- column 3D kernel
+// The FP32 form of the streaming kernel, with the rings in registers. A CTA owns
+// 8 x 8 elements in (x, y) and streams a chunk of their z column; thread (ex,
+// qy) owns the Q quadrature columns of element ex at quadrature row qy, so a
+// column's interpolated planes (v, the last p + 1) and its z-projected
+// accumulators (g, the next p + 1) never leave its registers, and the
+// contractions along x at either end are register loops too. Per coefficient
+// plane: y interpolation through shared memory (sX -> sY), then per thread the
+// x interpolation, the z element (interpolate, times w V from the closed form,
+// project back), the x projection, and a rotation over the 8 lanes of a row
+// that adds up the coefficients shared by neighbouring elements; the finished
+// row sums (sS) are projected along y and added to y with one atomic per
+// coefficient and tile. Two barriers per plane: the y projection of the last
+// plane runs beside the y interpolation of the next. Complex products are
+// packed FP32 (one issue slot for both components).
+//
+// Bound by issue slots (about 760 instructions per thread and plane at p = 4,
+// 10 warps per SM). The kernel above, with both rings in shared memory and
+// five barriers per plane, took 657 us for 96^3 elements of degree 4; this one
+// 305 us. Double-float keeps the rings in shared memory: they would need 200
+// registers.
+template <int P> struct QCols {
+    static constexpr int NP = P + 1, Q = P + 1, TE = 8, TQ = TE * Q, TC = TE + P, NT = TE * TQ;
+    static constexpr int PY = 24;            // row pitch of sY: two rows of 8 lanes hit different banks
+    static constexpr int NZ = Q * NP + 2 * Q;   // z tables of one element: N, w, x
+};
+__device__ __forceinline__ float2 pfma(float a, float2 v, float2 acc) { return __ffma2_rn(make_float2(a, a), v, acc); }
+
+template <int P>
+__global__ void __launch_bounds__(QCols<P>::NT, P <= 3 ? 2 : 1) k_quad3_cols(const QuadParams<float> prm, int zchunk) {
+    using S = QCols<P>;
+    constexpr int NP = S::NP, Q = S::Q, TE = S::TE, TQ = S::TQ, TC = S::TC, NT = S::NT, PY = S::PY, NZ = S::NZ;
+    __shared__ float2 sX[TC * TC], sY[TQ * PY], sS[TQ * TC];
+    __shared__ float sNy[TQ * NP], sZ[NZ];
+    constexpr bool kNxReg = P <= 4;          // x tables in registers, or (degree 5) in shared memory
+    __shared__ float sNx[kNxReg ? 1 : Q * NP * TE];
+    const int tid = threadIdx.x, ex = tid & 7, qy = tid >> 3;
+    const int nelx = prm.nel[0], nely = prm.nel[1], nelz = prm.nel[2];
+    const int tilesX = (nelx + TE - 1) / TE;
+    const int ex0 = (blockIdx.x % tilesX) * TE, ey0 = (blockIdx.x / tilesX) * TE;
+    const int ez0 = blockIdx.y * zchunk, nelc = min(nelz, ez0 + zchunk) - ez0;
+    if (nelc <= 0) return;
+    const int n0 = prm.n[0], n1 = prm.n[1], n2 = prm.n[2];
+    const int cx0 = prm.off[0][ex0], cy0 = prm.off[1][ey0], cz0 = prm.off[2][ez0];
+    const float2 *__restrict__ X = static_cast<const float2 *>(prm.x);
+    float2 *__restrict__ Y = static_cast<float2 *>(prm.y);
+    // this thread's element and row (elements past the grid: zero tables, no contribution)
+    const bool inx = ex0 + ex < nelx, iny = ey0 + qy / Q < nely;
+    float nxr[kNxReg ? Q * NP : 1], wxy[Q], xx[Q];
+    if constexpr (kNxReg) {
+#pragma unroll
+        for (int i = 0; i < Q * NP; ++i) nxr[i] = inx ? prm.N[0][(size_t)(ex0 + ex) * Q * NP + i] : 0.f;
+    } else {
+        for (int i = tid; i < Q * NP * TE; i += NT)
+            sNx[i] = ex0 + i % TE < nelx ? prm.N[0][(size_t)(ex0 + i % TE) * Q * NP + i / TE] : 0.f;
+    }
+    auto nx = [&](int q, int c) {
+        if constexpr (kNxReg) return nxr[q * NP + c];
+        else return sNx[(q * NP + c) * TE + ex];
+    };
+    const float wy = iny ? prm.w[1][(size_t)ey0 * Q + qy] : 0.f, yy = iny ? prm.xq[1][(size_t)ey0 * Q + qy] : 0.f;
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+        wxy[q] = inx ? prm.w[0][(size_t)(ex0 + ex) * Q + q] * wy : 0.f;
+        xx[q] = inx ? prm.xq[0][(size_t)(ex0 + ex) * Q + q] : 0.f;
+    }
+    for (int i = tid; i < TQ * NP; i += NT)
+        sNy[i] = ey0 + i / (Q * NP) < nely ? prm.N[1][(size_t)ey0 * Q * NP + i] : 0.f;
+    // coefficient plane k of the chunk: one element per thread, a plane ahead
+    const int lx = cx0 + tid % TC, ly = cy0 + tid / TC;
+    const bool ldr = tid < TC * TC && lx < n0 && ly < n1;
+    const int nplanes = nelc + P;
+    auto load_x = [&](int k) {
+        return ldr && k < nplanes && cz0 + k < n2 ? X[((size_t)(cz0 + k) * n1 + ly) * n0 + lx] : make_float2(0.f, 0.f);
+    };
+    auto load_z = [&](int e) {   // z tables of element ez0 + e
+        if (tid >= NZ || e < 0 || e >= nelc) return 0.f;
+        const size_t el = ez0 + e;
+        return tid < Q * NP ? prm.N[2][el * Q * NP + tid]
+                            : tid < Q * NP + Q ? prm.w[2][el * Q + tid - Q * NP] : prm.xq[2][el * Q + tid - Q * NP - Q];
+    };
+    if (tid < TC * TC) sX[tid] = load_x(0);
+    float2 px = load_x(1);
+    float pz = load_z(-P);
+    __syncthreads();
+
+    float2 v[Q][NP], g[Q][NP];
+#pragma unroll
+    for (int q = 0; q < Q; ++q)
+#pragma unroll
+        for (int c = 0; c < NP; ++c) v[q][c] = g[q][c] = make_float2(0.f, 0.f);
+
+    // step k: plane k enters the rings, element k - P is integrated, plane
+    // k - P leaves (the last P steps only drain)
+#pragma unroll 1
+    for (int k = 0; k < nelc + 2 * P + 1; ++k) {
+        // y interpolation of plane k; y projection of the plane that left in the last step
+        if (k < nplanes)
+            for (int i = tid; i < TQ * TC; i += NT) {
+                const int r = i / TC, ix = i % TC, e = r / Q;
+                float2 a = make_float2(0.f, 0.f);
+#pragma unroll
+                for (int c = 0; c < NP; ++c) a = pfma(sNy[r * NP + c], sX[(e + c) * TC + ix], a);
+                sY[r * PY + ix] = a;
+            }
+        if (tid < NZ) sZ[tid] = pz;
+        const int i = NT - 1 - tid, kz = cz0 + k - 1 - P;
+        if (k > P && i < TC * TC) {
+            const int iy = i / TC, ix = i % TC, gy = cy0 + iy, gx = cx0 + ix;
+            float2 a = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int c = 0; c < NP; ++c) {
+                const int e = iy - c;
+                if (e < 0 || e >= TE) continue;
+#pragma unroll
+                for (int q = 0; q < Q; ++q) a = pfma(sNy[(e * Q + q) * NP + c], sS[(e * Q + q) * TC + ix], a);
+            }
+            if (gy < n1 && gx < n0 && kz < n2)
+                atomicAdd(&Y[((size_t)kz * n1 + gy) * n0 + gx],
+                          make_float2(prm.cre * a.x - prm.cim * a.y, prm.cre * a.y + prm.cim * a.x));
+        }
+        __syncthreads();
+        if (k == nelc + 2 * P) break;
+        // the next plane and the next element's z tables
+        if (tid < TC * TC) sX[tid] = px;
+        px = load_x(k + 2);
+        pz = load_z(k + 1 - P);
+        // x interpolation of this thread's element
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+#pragma unroll
+            for (int c = 0; c < P; ++c) v[q][c] = v[q][c + 1];
+            v[q][P] = make_float2(0.f, 0.f);
+        }
+        if (k < nplanes) {
+#pragma unroll
+            for (int c = 0; c < NP; ++c) {
+                const float2 u = sY[qy * PY + ex + c];
+#pragma unroll
+                for (int q = 0; q < Q; ++q) v[q][P] = pfma(nx(q, c), u, v[q][P]);
+            }
+        }
+        if (k < P) {
+            __syncthreads();
+            continue;
+        }
+        if (k < nplanes) {
+#pragma unroll
+            for (int qz = 0; qz < Q; ++qz) {
+                const float wz = sZ[Q * NP + qz], zz = sZ[Q * NP + Q + qz];
+                float pot[Q];
+#pragma unroll
+                for (int q = 0; q < Q; ++q) pot[q] = 0.f;
+                for (int m = 0; m < prm.nsoft; ++m) {
+                    const float dy = yy - prm.soft[m][2], dz = zz - prm.soft[m][3];
+                    const float r = fmaf(dz, dz, fmaf(dy, dy, prm.soft[m][4]));
+#pragma unroll
+                    for (int q = 0; q < Q; ++q) {
+                        const float dx = xx[q] - prm.soft[m][1];
+                        pot[q] = fmaf(-prm.soft[m][0], rsqrtf(fmaf(dx, dx, r)), pot[q]);
+                    }
+                }
+                float nz[NP];
+#pragma unroll
+                for (int c = 0; c < NP; ++c) nz[c] = sZ[qz * NP + c];
+#pragma unroll
+                for (int q = 0; q < Q; ++q) {
+                    float2 f = make_float2(0.f, 0.f);
+#pragma unroll
+                    for (int c = 0; c < NP; ++c) f = pfma(nz[c], v[q][c], f);
+                    const float wv = wxy[q] * wz * pot[q];
+                    f = __fmul2_rn(f, make_float2(wv, wv));
+#pragma unroll
+                    for (int c = 0; c < NP; ++c) g[q][c] = pfma(nz[c], f, g[q][c]);
+                }
+            }
+        }
+        // plane k - P is complete: project along x. part(c) belongs to
+        // coefficient ex + c; rotated by c lanes it lands on lane (ex + c) & 7,
+        // as coefficient ex + c (main) or, past the eighth, 8 + lane (over)
+        float2 main = make_float2(0.f, 0.f), over = make_float2(0.f, 0.f);
+#pragma unroll
+        for (int c = 0; c < NP; ++c) {
+            float2 part = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < Q; ++q) part = pfma(nx(q, c), g[q][0], part);
+            float2 r;
+            r.x = __shfl_sync(0xffffffffu, part.x, (ex - c) & 7, 8);
+            r.y = __shfl_sync(0xffffffffu, part.y, (ex - c) & 7, 8);
+            if (ex >= c) main = __fadd2_rn(main, r);
+            else over = __fadd2_rn(over, r);
+        }
+        sS[qy * TC + ex] = main;
+        if (ex < P) sS[qy * TC + TE + ex] = over;
+#pragma unroll
+        for (int q = 0; q < Q; ++q) {
+#pragma unroll
+            for (int c = 0; c < P; ++c) g[q][c] = g[q][c + 1];
+            g[q][P] = make_float2(0.f, 0.f);
+        }
+        __syncthreads();
+    }
+}
+
 // the streaming kernel applies: 3D, Q = p + 1, consecutive element offsets on every axis
 bool stream_ok(const QuadTerm &q) { return q.dim == 3 && q.nq == q.p + 1 && q.consecutive; }
+
+template <int P> void launch_q3c(const QuadTerm &q, const QuadParams<float> &prm, cudaStream_t st) {
+    using S = QCols<P>;
+    const int tiles = ((q.nel[0] + S::TE - 1) / S::TE) * ((q.nel[1] + S::TE - 1) / S::TE);
+    // z chunks: the fewest plane steps of a full wave, halo planes included
+    const int slots = sm_count() * (P <= 3 ? 2 : 1);
+    int best = 1;
+    long long cost = -1;
+    for (int c = 1; c <= 32 && c <= q.nel[2]; ++c) {
+        const int z = (q.nel[2] + c - 1) / c;
+        const long long t = ((long long)tiles * ((q.nel[2] + z - 1) / z) + slots - 1) / slots * (z + 2 * P + 1);
+        if (cost < 0 || t < cost) { cost = t; best = c; }
+    }
+    const int zchunk = (q.nel[2] + best - 1) / best;
+    k_quad3_cols<P><<<dim3(tiles, (q.nel[2] + zchunk - 1) / zchunk), S::NT, 0, st>>>(prm, zchunk);
+}
 
 template <class A, int P>
 void launch_q3s(const QuadTerm &q, const QuadParams<typename QArith<A>::TT> &prm, cudaStream_t st) {
@@ -561,12 +759,16 @@ void dispatch_q(const QuadTerm &q, cd coef, const void *x, void *y, cudaStream_t
     }
     const QuadParams<T> prm = make_qparams<T>(q, coef, x, y);
     if (stream_ok(q)) {   // FP32: FP32 arithmetic; FP64 vectors: double-float arithmetic
-        using A = typename std::conditional<std::is_same<T, float>::value, float, dff>::type;
+        auto stream = [&](auto deg) {
+            constexpr int P = decltype(deg)::value;
+            if constexpr (std::is_same<T, float>::value) launch_q3c<P>(q, prm, st);
+            else launch_q3s<dff, P>(q, prm, st);
+        };
         switch (q.p) {
-        case 2: launch_q3s<A, 2>(q, prm, st); return;
-        case 3: launch_q3s<A, 3>(q, prm, st); return;
-        case 4: launch_q3s<A, 4>(q, prm, st); return;
-        case 5: launch_q3s<A, 5>(q, prm, st); return;
+        case 2: stream(std::integral_constant<int, 2>{}); return;
+        case 3: stream(std::integral_constant<int, 3>{}); return;
+        case 4: stream(std::integral_constant<int, 4>{}); return;
+        case 5: stream(std::integral_constant<int, 5>{}); return;
         default: break;
         }
     }
