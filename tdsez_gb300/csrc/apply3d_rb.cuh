@@ -474,34 +474,23 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
         }
     };
 
-    if constexpr (kShiftRing<T>) {
-        // double-float: one copy of the step, the ring shifts down by one slot per plane
+    // One copy of the step; the ring shifts down by one slot per plane. A plane
+    // loop unrolled by the ring length with fixed slots saves the moves but is
+    // seven times the code: a CTA of a small grid runs it once or twice and
+    // waits for instructions (FP32, 16 x 20 x 40 elements of degree 3: 31 us
+    // unrolled, 15 us shifted with runs down to two planes; 160 x 160 x 320:
+    // 164 and 150 us)
 #pragma unroll 1
-        for (int it = 0; it < nplanes; ++it) {
-            MC sv[R];
-            side_load(it, sv);
-            if (it >= lo && it < hi) step(it, 0);
-            finish(it, 0, sv);
+    for (int it = 0; it < nplanes; ++it) {
+        MC sv[R];
+        side_load(it, sv);
+        if (it >= lo && it < hi) step(it, 0);
+        finish(it, 0, sv);
 #pragma unroll
-            for (int r = 0; r < R; ++r) {
+        for (int r = 0; r < R; ++r) {
 #pragma unroll
-                for (int s = 0; s + 1 < BW; ++s) acc[r][s] = acc[r][s + 1];
-                acc[r][BW - 1] = czero<C>();
-            }
-        }
-    } else {
-        // FP32: the plane loop unrolled by the ring length, fixed slots
-        for (int base = 0; base < nplanes; base += BW) {
-#pragma unroll
-            for (int ph = 0; ph < BW; ++ph) {
-                const int it = base + ph;
-                if (it >= nplanes) break;
-                const int ring = (ph - P + 2 * BW) % BW;
-                MC sv[R];
-                side_load(it, sv);
-                if (it >= lo && it < hi) step(it, ring);
-                finish(it, ring, sv);
-            }
+            for (int s = 0; s + 1 < BW; ++s) acc[r][s] = acc[r][s + 1];
+            acc[r][BW - 1] = czero<C>();
         }
     }
     if constexpr (!Sh::kTma) asm volatile("cp.async.wait_group 0;\n" ::: "memory");
@@ -600,9 +589,11 @@ inline void run3d_rb(const ApplyParams<T> &prm0, cudaStream_t st) {
         rb_make_map(&map, prm0.x, prm0.n0, prm0.n1, n2, 2 * Sh::RX, Sh::RY);
     }
     auto tiles_for = [&](int txw) { return ((prm0.n0 + txw - 1) / txw) * ((prm0.n1 + Sh::TY - 1) / Sh::TY); };
+    // runs of two planes at least: the 2p halo planes are then most of a run, but
+    // a grid that small leaves the chip idle and what counts is a run's length
     auto seg_for = [&](int txw, long long g) {
         const long long total = (long long)tiles_for(txw) * n2;
-        return (int)std::min<long long>(total, std::max<long long>(4 * P, (total + g - 1) / g));
+        return (int)std::min<long long>(total, std::max<long long>(2, (total + g - 1) / g));
     };
     auto launch = [&](int txw, int seg, bool candidate = false) {
         ApplyParams<T> prm = prm0;

@@ -99,9 +99,6 @@ __device__ __forceinline__ C comb_at(const CombP<T> &cb, const T *bands, int n, 
 // results are double-buffered.
 constexpr int kLoadsPerThread3 = 4;   // covers (TY+2p)(TX+2p) / (TX TY) for p <= 5
 
-// ring of output planes: unrolled with fixed slots (FP32) or shifted per plane
-template <class T> constexpr bool kShiftRing = !std::is_same<T, float>::value;
-
 // TX is the largest tile width; the launch may use a narrower one
 // (blockDim.x = 16..TX) to fit n0 with less padding. KA / KC: the kind of the
 // outer combinations fixed at compile time (0 complex, 1 real, 2 imaginary);
@@ -310,33 +307,16 @@ __device__ __noinline__ double2 apply3d_run(const ApplyParams<T> &prm, int x0, i
         }
     };
 
-    if constexpr (kShiftRing<T>) {
-        // FP64 / double-float: one copy of the step; the ring shifts down by one
-        // slot per plane (a few register moves), which keeps the long
-        // emulated-FP64 body inside the instruction cache
+    // One copy of the step; the ring shifts down by one slot per plane (a few
+    // register moves), which keeps the body inside the instruction cache
 #pragma unroll 1
-        for (int it = 0; it < nplanes; ++it) {
-            const MC sv = side_load(it);
-            if (it >= lo && it < hi) step(it, 0);
-            finish(it, acc[0], sv);
+    for (int it = 0; it < nplanes; ++it) {
+        const MC sv = side_load(it);
+        if (it >= lo && it < hi) step(it, 0);
+        finish(it, acc[0], sv);
 #pragma unroll
-            for (int s = 0; s + 1 < BW; ++s) acc[s] = acc[s + 1];
-            acc[BW - 1] = czero<C>();
-        }
-    } else {
-        // FP32: the plane loop unrolled by the ring length, fixed slots
-        for (int base = 0; base < nplanes; base += BW) {
-#pragma unroll
-            for (int ph = 0; ph < BW; ++ph) {
-                const int it = base + ph;
-                if (it >= nplanes) break;
-                const int ring = (ph - P + 2 * BW) % BW;
-                const MC sv = side_load(it);
-                if (it >= lo && it < hi) step(it, ring);
-                finish(it, acc[ring], sv);
-                acc[ring] = czero<C>();
-            }
-        }
+        for (int s = 0; s + 1 < BW; ++s) acc[s] = acc[s + 1];
+        acc[BW - 1] = czero<C>();
     }
     return racc;
 }

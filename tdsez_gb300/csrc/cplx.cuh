@@ -169,11 +169,23 @@ template <> __device__ __forceinline__ void ifma<dff, cdff>(cdff &acc, dff b, cd
     // i v first: loops over b share it
     fma2(acc, make_float2(b.hi, b.hi), make_float2(b.lo, b.lo), make_float2(-v.hi.y, v.hi.x), make_float2(-v.lo.y, v.lo.x));
 }
+// FP32 pairs packed as well (3D apply of 8.8 M FP32 coefficients, degree 3: 184 us
+// scalar, 150 us packed)
+template <> __device__ __forceinline__ void rfma<float, float2>(float2 &acc, float a, float2 v) {
+    acc = __ffma2_rn(make_float2(a, a), v, acc);
+}
+template <> __device__ __forceinline__ void ifma<float, float2>(float2 &acc, float b, float2 v) {
+    acc = __ffma2_rn(make_float2(b, b), make_float2(-v.y, v.x), acc);
+}
 template <class C> __device__ __forceinline__ void cfma(C &acc, C a, C v) {
     acc.x = tfma(a.x, v.x, acc.x);
     acc.x = tfma(-a.y, v.y, acc.x);
     acc.y = tfma(a.x, v.y, acc.y);
     acc.y = tfma(a.y, v.x, acc.y);
+}
+template <> __device__ __forceinline__ void cfma<float2>(float2 &acc, float2 a, float2 v) {
+    rfma(acc, a.x, v);
+    ifma(acc, a.y, v);
 }
 template <> __device__ __forceinline__ void cfma<cdff>(cdff &acc, cdff a, cdff v) {
     rfma(acc, a.re(), v);
