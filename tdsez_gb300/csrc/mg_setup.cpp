@@ -338,36 +338,26 @@ void chebyshev(MGLevel &m, int prec, double mu_a, double mu_b, double w, int ste
     }
     const cd theta = alpha + g * center;
     const cd delta = g * focal;
-    const size_t n = m.ndof;
-    // r = b - A x
-    if (x_zero) blas::copy(m.b.ptr, m.r.ptr, n, prec, st);
-    else {
-        op.apply(TDZ_STAGE, prec, m.x.ptr, m.t1.ptr, st);
-        blas::axpbypcz(m.r.ptr, 1.0, m.b.ptr, 0.0, m.t1.ptr, -1.0, n, prec, st);
+    // r = b - A x (x = 0: r is b itself, first written by the second step)
+    const void *r = m.b.ptr;
+    if (!x_zero) {
+        op.residual(TDZ_STAGE, prec, m.x.ptr, m.b.ptr, m.r.ptr, st);
+        r = m.r.ptr;
     }
-    if (std::abs(delta) <= 1e-12 * std::abs(theta)) {
-        // degenerate segment: damped Richardson x += M^-1 r / theta
-        blas::copy(m.r.ptr, m.z.ptr, n, prec, st);
-        m.minv.apply(m.z.ptr, prec, st);
-        if (x_zero) blas::axpby(m.x.ptr, 1.0 / theta, m.z.ptr, 0.0, n, prec, st);
-        else blas::axpby(m.x.ptr, 1.0 / theta, m.z.ptr, 1.0, n, prec, st);
-        return;
-    }
-    const cd sigma1 = theta / delta;
+    // A step is one apply (r -= A d in its store) and the line solves of M^-1 r,
+    // whose last axis forms d and x from z while it stores (ChebStep).
+    const bool degenerate = std::abs(delta) <= 1e-12 * std::abs(theta);   // damped Richardson, one step
+    const cd sigma1 = degenerate ? cd(1.0) : theta / delta;
     cd rho = 1.0 / sigma1;
-    blas::copy(m.r.ptr, m.z.ptr, n, prec, st);
-    m.minv.apply(m.z.ptr, prec, st);
-    blas::axpby(m.d.ptr, 1.0 / theta, m.z.ptr, 0.0, n, prec, st);
-    if (x_zero) blas::copy(m.d.ptr, m.x.ptr, n, prec, st);
-    else blas::axpby(m.x.ptr, 1.0, m.d.ptr, 1.0, n, prec, st);
+    const ChebStep first{1.0 / theta, 0.0, m.d.ptr, m.x.ptr, x_zero};
+    m.minv.apply(r, m.z.ptr, prec, st, &first);
+    if (degenerate) return;
     for (int k = 1; k < steps; ++k) {
-        op.apply(TDZ_STAGE, prec, m.d.ptr, m.t1.ptr, st);
-        blas::axpby(m.r.ptr, -1.0, m.t1.ptr, 1.0, n, prec, st);
-        blas::copy(m.r.ptr, m.z.ptr, n, prec, st);
-        m.minv.apply(m.z.ptr, prec, st);
+        op.residual(TDZ_STAGE, prec, m.d.ptr, r, m.r.ptr, st);
+        r = m.r.ptr;
         const cd rn = 1.0 / (2.0 * sigma1 - rho);
-        blas::axpby(m.d.ptr, 2.0 * rn / delta, m.z.ptr, rn * rho, n, prec, st);
-        blas::axpby(m.x.ptr, 1.0, m.d.ptr, 1.0, n, prec, st);
+        const ChebStep next{2.0 * rn / delta, rn * rho, m.d.ptr, m.x.ptr, false};
+        m.minv.apply(r, m.z.ptr, prec, st, &next);
         rho = rn;
     }
 }
@@ -395,9 +385,7 @@ void Multigrid::vcycle(int l, cudaStream_t st) {
     }
     const double lo = m.mu_hi / opt.ratio;
     chebyshev(m, prec, lo, m.mu_hi, m.w_max, opt.smooth, true, st);
-    // r = b - A x
-    m.opp->apply(TDZ_STAGE, prec, m.x.ptr, m.t1.ptr, st);
-    blas::axpbypcz(m.r.ptr, 1.0, m.b.ptr, 0.0, m.t1.ptr, -1.0, m.ndof, prec, st);
+    m.opp->residual(TDZ_STAGE, prec, m.x.ptr, m.b.ptr, m.r.ptr, st);
     // restrict: axis 2, then 1, then 0 (shrinking early)
     MGLevel &c = lv[l + 1];
     const int dim = m.space.dim;

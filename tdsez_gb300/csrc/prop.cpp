@@ -32,8 +32,7 @@ void PcMass::apply(const double2 *r, double2 *z, cudaStream_t st) {
     // M^-1 approximates A^-1 up to the (non-zero) stage scalar alpha
     const cd a = 1.0 / op->sigma[0];
     if (prec == TDZ_FP64) {
-        blas::copy(r, z, n, TDZ_FP64, st);
-        ks.apply(z, TDZ_FP64, st);
+        ks.apply(r, z, TDZ_FP64, st);
         blas::scale(z, a, n, TDZ_FP64, st);
     } else {
         blas::cast(r, TDZ_FP64, buf.ptr, TDZ_FP32, n, st);
