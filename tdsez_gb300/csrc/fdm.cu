@@ -1052,8 +1052,15 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
         // [z][y][c][x] -> [z][x'][c][y] -> [z][y'][c][x'] -> line solves -> [z][x][c][y'] -> [z][y][c][x]
         float *a = pa.as<float>(), *b = pb.as<float>();
         const int blocks = (int)std::min<size_t>((N + 255) / 256, (size_t)16 * sm_count());
-        k_to_planar<<<blocks, 256, 0, st>>>(r, a, n[0], rows, ldx);
-        transform(Tf[0], a, n[2], n[1], ldx, b, ldy, st);
+        // the first and last transforms read and write the natural-order FP64
+        // vectors themselves where their kernel can
+        if (transform_natural(Tf[0])) {
+            transform_from64(Tf[0], r, n[2], n[1], b, ldy, st);
+        } else {
+            k_to_planar<<<blocks, 256, 0, st>>>(r, a, n[0], rows, ldx);
+            count_launch();
+            transform(Tf[0], a, n[2], n[1], ldx, b, ldy, st);
+        }
         transform(Tf[1], b, n[2], n[0], ldy, a, ldx, st);
         ZSolveParams zp = line_params(*this);
         zp.x = a;
@@ -1063,16 +1070,21 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
         zp.cs = ldx;
         line_solve(P, zp, st);
         transform(Ti[0], a, n[2], n[1], ldx, b, ldy, st);
-        transform(Ti[1], b, n[2], n[0], ldy, a, ldx, st);
-        if (norm_out) {
-            k_from_planar_norm<<<blocks, 256, 0, st>>>(a, z, n[0], rows, ldx, npart.as<double>());
-            k_sum_parts<<<1, 512, 0, st>>>(npart.as<double>(), blocks, norm_out);
-            count_launch();
+        int parts = blocks;
+        if (transform_natural(Ti[1])) {
+            transform_to64(Ti[1], b, n[2], n[0], ldy, z, norm_out ? npart.as<double>() : nullptr, st);
+            parts = transform_norm_parts(n[2], n[0]);
         } else {
-            k_from_planar<<<blocks, 256, 0, st>>>(a, z, n[0], rows, ldx);
+            transform(Ti[1], b, n[2], n[0], ldy, a, ldx, st);
+            if (norm_out) k_from_planar_norm<<<blocks, 256, 0, st>>>(a, z, n[0], rows, ldx, npart.as<double>());
+            else k_from_planar<<<blocks, 256, 0, st>>>(a, z, n[0], rows, ldx);
+            count_launch();
+        }
+        if (norm_out) {
+            k_sum_parts<<<1, 512, 0, st>>>(npart.as<double>(), parts, norm_out);
+            count_launch();
         }
         TDZ_CUDA(cudaGetLastError());
-        count_launch(2);
         ++applies;
         return;
     }

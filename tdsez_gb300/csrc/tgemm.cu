@@ -24,13 +24,17 @@
 // the error word, the consumers leave together, and TMEM is still freed.
 #include "tgemm.h"
 
+#include "cplx.cuh"
+
 #include <cudaTypedefs.h>
 
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdlib>
 #include <cstring>
 #include <mutex>
+#include <new>
 #include <string>
 #include <set>
 
@@ -43,7 +47,8 @@ constexpr int KC = 16;         // K per stage (64 bytes of FP32: one 64-byte swi
 constexpr int A_BYTES = TM * KC * 4;   // 8 KB
 constexpr long long kWaitCycles = 4000000000LL;   // about 2 s at 2 GHz
 
-__device__ int g_tgemm_error = 0;
+// pinned host word that a wait which ran out sets (the same for every device)
+__device__ int *g_tgemm_error = nullptr;
 
 __device__ __forceinline__ uint32_t smem_u32(const void *p) {
     return static_cast<uint32_t>(__cvta_generic_to_shared(p));
@@ -79,7 +84,7 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity) {
     const long long t0 = clock64();
     while (!mbar_try(bar, parity)) {
         if (clock64() - t0 > kWaitCycles) {
-            atomicExch(&g_tgemm_error, 1);
+            if (g_tgemm_error) *reinterpret_cast<volatile int *>(g_tgemm_error) = 1;
             return false;
         }
     }
@@ -503,6 +508,331 @@ __global__ void __launch_bounds__(320, 1)
         asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(TMEM_COLS) : "memory");
 }
 
+// ---- B-resident variant: BF16 x 3 slices
+// Both operands as sums of three BF16 slices (v = h + m + l, 24 significant
+// bits and FP32's exponent range); the product keeps the six slice pairs
+// above 2^-24: h h, h m, m h, m m, h l, l h. BF16 MMAs run at twice the TF32
+// rate, so this is three quarters of the TF32 hi/lo product's tensor time, and
+// the slices take 6 bytes per entry instead of 8: all of B (186 KB for
+// Np = Kp = 176) stays in shared memory for the whole launch. What bounded the
+// streaming kernel was B: 248 KB per 128-row tile through L2 against 83 KB of
+// A (57 us per transform at 111 818 rows of 163; this kernel 51 us).
+//   warps 0-15  in groups of four, as many as there are stages (at most four),
+//               the groups taking chunks in turn:
+//               load an A chunk (128 rows x 16) into registers, split it and
+//               store the slices to the stage ring. The proxy fence after the
+//               stores waits for the thread's loads too, so a group has no
+//               loads in flight across it; the other groups' cover the latency
+//               (one set of warps with a register prefetch: 68 us)
+//   warps 16-23 drain accumulator tile & 1 into the transposed output, two per
+//               TMEM lane quarter with half of the columns each, the next 16
+//               columns on their way while the last ones are stored (four warps
+//               and nothing in flight: 69 us; 43 us with the stores left out)
+//   warp 24     (one thread) loads B once by bulk copies, then issues the MMAs
+// Operand tiles are K-major rows of 16 BF16 (32 bytes), 32-byte swizzle: the
+// 16-byte halves of a row trade places when bit 2 of the row is set.
+constexpr int kB3Slice = TM * 32;            // one slice of an A chunk
+constexpr int kB3Stage = 3 * kB3Slice;       // 12 KB
+constexpr int kB3Groups = 4;                 // loader groups of 128 threads
+constexpr int kB3Epi = 8;                    // epilogue warps
+constexpr int kB3Threads = (4 * kB3Groups + kB3Epi + 1) * 32;
+constexpr size_t kB3Max = 232448;
+inline size_t b3_bytes(int Kp, int Np) { return (size_t)6 * Kp * Np; }
+// stages that fit beside B (0: B does not fit)
+inline int b3_stages(int Kp, int Np) {
+    const size_t fixed = 1024 + b3_bytes(Kp, Np) + 256;
+    if (fixed + 2 * kB3Stage > kB3Max) return 0;
+    return (int)std::min<size_t>(8, (kB3Max - fixed) / kB3Stage);
+}
+// byte offset of the 16-byte half h of row r in a K-major 32-byte-swizzled tile
+__host__ __device__ inline int b3_off(int r, int h) { return r * 32 + ((h ^ ((r >> 2) & 1)) << 4); }
+
+__device__ __forceinline__ uint64_t b3_desc(uint32_t addr) {
+    uint64_t d = 0;
+    d |= (uint64_t)((addr & 0x3FFFF) >> 4);
+    d |= (uint64_t)1 << 16;
+    d |= (uint64_t)(256 >> 4) << 32;                 // 8-row groups 256 bytes apart
+    d |= (uint64_t)1 << 46;
+    d |= (uint64_t)6 << 61;                          // 32-byte swizzle
+    return d;
+}
+// kind::f16: BF16 operands, FP32 accumulator, K-major, M = 128
+__host__ __device__ constexpr uint32_t b3_instr_desc(int n) {
+    return (1u << 4) | (1u << 7) | (1u << 10) | ((uint32_t)(n >> 3) << 17) | ((uint32_t)(TM >> 4) << 24);
+}
+__device__ __forceinline__ void mma_bf16(uint32_t tmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
+    asm volatile(
+        "{\n\t.reg .pred p;\n\t"
+        "setp.ne.b32 p, %4, 0;\n\t"
+        "tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n\t}" ::"r"(tmem),
+        "l"(a), "l"(b), "r"(idesc), "r"(acc)
+        : "memory");
+}
+// two FP32 values to packed BF16 (first in the low half) and their remainders
+__device__ __forceinline__ uint32_t bf16_split2(float &a, float &b) {
+    uint32_t p;
+    asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(p) : "f"(b), "f"(a));
+    a -= __uint_as_float(p << 16);
+    b -= __uint_as_float(p & 0xFFFF0000u);
+    return p;
+}
+
+struct B3Params {
+    const float *in;
+    const double2 *in64;   // IN64: complex rows of K natural-order FP64 entries
+    double *out64;         // OUT64: natural-order FP64, out64[((p N + n) R + r) 2 + part]
+    double *norm;          // OUT64: per epilogue warp the sum of squares written (kB3Epi per CTA), or null
+    const uint8_t *b;      // swizzled slices of B: [chunk][slice][Np x 32 bytes]
+    float *out;
+    int rows, R, K, N, Np, ldi, ldo, nch, tiles, ns;
+};
+
+template <bool IN64, bool OUT64>
+__global__ void __launch_bounds__(kB3Threads, 1) k_transform_b3(const B3Params prm) {
+    extern __shared__ uint8_t smem_raw[];
+    uint8_t *base = reinterpret_cast<uint8_t *>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
+    const int nch = prm.nch, NS = prm.ns, Np = prm.Np;
+    const int bchunk = 3 * Np * 32;
+    uint8_t *sB = base, *sA = base + (size_t)nch * bchunk;
+    uint64_t *bars = reinterpret_cast<uint64_t *>(sA + (size_t)NS * kB3Stage);   // full [8], done [8], accf [2], acce [2], B
+    uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(bars + 21);
+    const uint32_t full0 = smem_u32(&bars[0]), done0 = smem_u32(&bars[8]), accf0 = smem_u32(&bars[16]),
+                   acce0 = smem_u32(&bars[18]), bbar = smem_u32(&bars[20]);
+    const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+    const int my_tiles = prm.tiles > (int)blockIdx.x ? (prm.tiles - 1 - (int)blockIdx.x) / (int)gridDim.x + 1 : 0;
+    const int G = my_tiles * nch;
+    if (tid == 0) {
+        for (int s = 0; s < NS; ++s) {
+            mbar_init(full0 + 8 * s, 128);
+            mbar_init(done0 + 8 * s, 1);
+        }
+        for (int b = 0; b < 2; ++b) {
+            mbar_init(accf0 + 8 * b, 1);
+            mbar_init(acce0 + 8 * b, 32 * kB3Epi);
+        }
+        mbar_init(bbar, 1);
+        asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    if (warp == 0) {
+        asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
+                     "r"(512)
+                     : "memory");
+        asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    const uint32_t tmem = *tmem_slot;
+
+    if (warp < 4 * kB3Groups) {
+        const int lt = tid & 127;
+        // no more groups than stages: a group then waits for the MMAs of its own
+        // last chunk or an older one, never two phases of a barrier ahead
+        const int ng = min(kB3Groups, NS);
+        for (int g = (tid >> 7) < ng ? tid >> 7 : G; g < G; g += ng) {
+            const int tile = (int)blockIdx.x + (g / nch) * (int)gridDim.x, k0 = (g % nch) * 16, s = g % NS;
+            uint8_t *st = sA + (size_t)s * kB3Stage;
+            if constexpr (IN64) {
+                // complex rows lt / 4 and lt / 4 + 32, four entries each
+                const int qt = lt & 3, k = k0 + 4 * qt;
+                double2 v[2][4];
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const int row = tile * (TM / 2) + (lt >> 2) + 32 * m;
+#pragma unroll
+                    for (int j = 0; j < 4; ++j)
+                        v[m][j] = 2 * row < prm.rows && k + j < prm.K ? prm.in64[(size_t)row * prm.K + k + j]
+                                                                      : make_double2(0.0, 0.0);
+                }
+                if (g >= NS && !mbar_wait(done0 + 8 * s, ((g - NS) / NS) & 1)) break;
+#pragma unroll
+                for (int m = 0; m < 2; ++m) {
+                    const int r = (lt >> 2) + 32 * m;
+                    float re[4], im[4];
+#pragma unroll
+                    for (int j = 0; j < 4; ++j) {
+                        const dff x = dff_split(v[m][j].x), y = dff_split(v[m][j].y);
+                        re[j] = __fadd_rn(x.hi, x.lo);
+                        im[j] = __fadd_rn(y.hi, y.lo);
+                    }
+                    uint8_t *sr = st + b3_off(2 * r, qt >> 1) + 8 * (qt & 1);
+                    uint8_t *si = st + b3_off(2 * r + 1, qt >> 1) + 8 * (qt & 1);
+#pragma unroll
+                    for (int sl = 0; sl < 3; ++sl) {
+                        uint2 a, b;
+                        a.x = bf16_split2(re[0], re[1]);
+                        a.y = bf16_split2(re[2], re[3]);
+                        b.x = bf16_split2(im[0], im[1]);
+                        b.y = bf16_split2(im[2], im[3]);
+                        *reinterpret_cast<uint2 *>(sr + sl * kB3Slice) = a;
+                        *reinterpret_cast<uint2 *>(si + sl * kB3Slice) = b;
+                    }
+                }
+            } else {
+                // rows lt / 4 + 32 m, 16 bytes each (a warp reads whole 64-byte row pieces)
+                const int qt = lt & 3, k = k0 + 4 * qt;
+                float4 v[4];
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    const int row = tile * TM + (lt >> 2) + 32 * m;
+                    v[m] = make_float4(0.f, 0.f, 0.f, 0.f);
+                    if (row < prm.rows && k < prm.K) {
+                        v[m] = *reinterpret_cast<const float4 *>(prm.in + (size_t)row * prm.ldi + k);   // k + 3 < ldi
+                        if (k + 1 >= prm.K) v[m].y = 0.f;
+                        if (k + 2 >= prm.K) v[m].z = 0.f;
+                        if (k + 3 >= prm.K) v[m].w = 0.f;
+                    }
+                }
+                if (g >= NS && !mbar_wait(done0 + 8 * s, ((g - NS) / NS) & 1)) break;
+#pragma unroll
+                for (int m = 0; m < 4; ++m) {
+                    uint8_t *sr = st + b3_off((lt >> 2) + 32 * m, qt >> 1) + 8 * (qt & 1);
+#pragma unroll
+                    for (int sl = 0; sl < 3; ++sl) {
+                        uint2 w;
+                        w.x = bf16_split2(v[m].x, v[m].y);
+                        w.y = bf16_split2(v[m].z, v[m].w);
+                        *reinterpret_cast<uint2 *>(sr + sl * kB3Slice) = w;
+                    }
+                }
+            }
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+            mbar_arrive(full0 + 8 * s);
+        }
+    } else if (warp == 4 * kB3Groups + kB3Epi) {
+        // tile t of this CTA's A rows (contiguous in memory) into L2: chunks are
+        // 64-byte pieces of 128 rows, too small to fetch from HBM one at a time
+        auto prefetch = [&](int t) {
+            if (t >= my_tiles) return;
+            const long long r0 = ((long long)blockIdx.x + (long long)t * gridDim.x) * TM;
+            const int nr = (int)min((long long)TM, prm.rows - r0);
+            const char *p = IN64 ? reinterpret_cast<const char *>(prm.in64 + r0 / 2 * prm.K)
+                                 : reinterpret_cast<const char *>(prm.in + r0 * prm.ldi);
+            const uint32_t bytes = IN64 ? (uint32_t)(nr / 2) * prm.K * 16
+                                        : (uint32_t)((nr - 1) * prm.ldi + prm.K) * 4 / 16 * 16;
+            if (bytes)
+                asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
+        };
+        if (lane == 0 && G > 0) {
+            prefetch(0);
+            prefetch(1);
+            mbar_expect_tx(bbar, (uint32_t)(nch * bchunk));
+            for (int c = 0; c < nch; ++c)
+                asm volatile(
+                    "cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];" ::"r"(
+                        smem_u32(sB + (size_t)c * bchunk)),
+                    "l"(prm.b + (size_t)c * bchunk), "r"(bchunk), "r"(bbar)
+                    : "memory");
+            const uint32_t idesc = b3_instr_desc(Np);
+            bool ok = mbar_wait(bbar, 0);
+            int s = 0, ph = 0, c = 0, t = 0;
+            for (int g = 0; g < G && ok; ++g) {
+                const int b = t & 1;
+                if (c == 0 && t >= 2 && !mbar_wait(acce0 + 8 * b, ((t - 2) >> 1) & 1)) break;
+                if (!mbar_wait(full0 + 8 * s, ph)) break;
+                asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+                const uint32_t aa = smem_u32(sA + (size_t)s * kB3Stage), bb = smem_u32(sB + (size_t)c * bchunk);
+                const uint64_t ah = b3_desc(aa), am = b3_desc(aa + kB3Slice), al = b3_desc(aa + 2 * kB3Slice);
+                const uint64_t bh = b3_desc(bb), bm = b3_desc(bb + Np * 32), bl = b3_desc(bb + 2 * Np * 32);
+                const uint32_t d = tmem + (uint32_t)(b * 256);
+                mma_bf16(d, al, bh, idesc, c > 0 ? 1u : 0u);
+                mma_bf16(d, ah, bl, idesc, 1u);
+                mma_bf16(d, am, bm, idesc, 1u);
+                mma_bf16(d, am, bh, idesc, 1u);
+                mma_bf16(d, ah, bm, idesc, 1u);
+                mma_bf16(d, ah, bh, idesc, 1u);
+                mma_commit(done0 + 8 * s);
+                if (++s == NS) { s = 0; ph ^= 1; }
+                if (++c == nch) {
+                    mma_commit(accf0 + 8 * b);
+                    c = 0;
+                    ++t;
+                    prefetch(t + 1);
+                }
+            }
+        }
+    } else {
+        // ---- epilogue: TMEM -> registers -> global (transposed per plane)
+        const int q = warp & 3, hi = (warp - 4 * kB3Groups) >> 2;
+        const int nc16 = Np / 16, c_lo = (hi ? (nc16 + 1) / 2 : 0) * 16, c_hi = (hi ? nc16 : (nc16 + 1) / 2) * 16;
+        const size_t nstride = OUT64 ? (size_t)2 * prm.R : (size_t)2 * prm.ldo;
+        double norm = 0.0;
+        for (int t = 0; t < my_tiles; ++t) {
+            const int b = t & 1;
+            if (!mbar_wait(accf0 + 8 * b, (t >> 1) & 1)) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+            const int tile = (int)blockIdx.x + t * (int)gridDim.x;
+            const int row = tile * TM + q * 32 + lane;
+            const bool row_ok = row < prm.rows;
+            const int cr = row >> 1, part = row & 1;
+            const int p = row_ok ? cr / prm.R : 0, r = row_ok ? cr % prm.R : 0;
+            float *orow = OUT64 ? nullptr : prm.out + ((size_t)p * prm.N * 2 + part) * prm.ldo + r;
+            double *orow64 = OUT64 ? prm.out64 + ((size_t)p * prm.N * prm.R + r) * 2 + part : nullptr;
+            float sq[2] = {0.f, 0.f};   // at most 48 squares each: relative error below 3e-6
+            const uint32_t tbase = tmem + (uint32_t)(b * 256) + ((uint32_t)(q * 32) << 16);
+            auto load = [&](uint32_t (&v)[16], int c0) {
+                asm volatile(
+                    "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, "
+                    "%12, %13, %14, %15}, [%16];"
+                    : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]),
+                      "=r"(v[7]), "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]),
+                      "=r"(v[14]), "=r"(v[15])
+                    : "r"(tbase + (uint32_t)c0));
+            };
+            // waits for the loads in flight, whose registers are not touched before
+            auto arrived = [&](uint32_t (&v)[16]) {
+                asm volatile("tcgen05.wait::ld.sync.aligned;"
+                             : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]),
+                               "+r"(v[7]), "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]),
+                               "+r"(v[14]), "+r"(v[15])
+                             :
+                             : "memory");
+            };
+            auto store = [&](const uint32_t (&v)[16], int c0) {
+                if (!row_ok) return;
+                const int left = prm.N - c0;   // columns past N are padding
+#pragma unroll
+                for (int j = 0; j < 16; ++j) {
+                    if (j >= left) break;
+                    const float f = __uint_as_float(v[j]);
+                    if constexpr (OUT64) {
+                        orow64[(size_t)(c0 + j) * nstride] = f2d_exact(f);
+                        sq[j & 1] = fmaf(f, f, sq[j & 1]);
+                    } else {
+                        orow[(size_t)(c0 + j) * nstride] = f;
+                    }
+                }
+            };
+            uint32_t v[2][16];
+            if (c_lo < c_hi) load(v[0], c_lo);
+#pragma unroll 1
+            for (int c0 = c_lo; c0 < c_hi; c0 += 32) {
+                arrived(v[0]);
+                if (c0 + 16 < c_hi) load(v[1], c0 + 16);
+                store(v[0], c0);
+                if (c0 + 16 < c_hi) {
+                    arrived(v[1]);
+                    if (c0 + 32 < c_hi) load(v[0], c0 + 32);
+                    store(v[1], c0 + 16);
+                }
+            }
+            asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+            mbar_arrive(acce0 + 8 * b);
+            if constexpr (OUT64)
+                if (prm.norm) norm += (double)sq[0] + (double)sq[1];
+        }
+        if constexpr (OUT64)
+            if (prm.norm) {
+                for (int o = 16; o > 0; o >>= 1) norm += __shfl_down_sync(0xffffffffu, norm, o);
+                if (lane == 0) prm.norm[kB3Epi * blockIdx.x + warp - 4 * kB3Groups] = norm;
+            }
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    if (warp == 0)
+        asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+}
+
 PFN_cuTensorMapEncodeTiled_v12000 encode_fn() {
     static PFN_cuTensorMapEncodeTiled_v12000 fn = nullptr;
     static std::once_flag once;
@@ -545,19 +875,67 @@ float tf32_round_host(double v) {
 // 256-row tiles where two sub-tiles' stages fit in shared memory (Np <= 192), else 128
 template <int NP> constexpr int sub_tiles() { return TGShape<NP, 2>::fits ? 2 : 1; }
 
-// the warp-specialised kernel unless TDZ_TRANSFORM=split asks for the
-// single-accumulator-pair one
-bool use_ws() {
-    static const bool ws = [] {
+// TDZ_TRANSFORM picks a kernel: "split" the single-accumulator-pair one, "ws"
+// the streaming warp-specialised one; else the B-resident kernel where all of
+// B fits in shared memory beside two stages (6 Kp Np bytes: up to 176 x 176)
+// and the streaming one beyond
+int variant() {
+    static const int v = [] {
         const char *e = std::getenv("TDZ_TRANSFORM");
-        return !(e && std::string(e) == "split");
+        return !e ? 0 : std::string(e) == "split" ? 2 : std::string(e) == "ws" ? 1 : 0;
     }();
-    return ws;
+    return v;
+}
+
+// the B-resident kernel: in / out FP32 planar, or in64 / out64 FP64 natural order
+void launch_b3(const TransformMat &T, const float *in, const double2 *in64, int planes, int R, int ldi, float *out,
+               int ldo, double2 *out64, double *norm, cudaStream_t st) {
+    // opt-in to the largest size once per device (the batch API steps runs from several host threads)
+    {
+        static std::mutex mu;
+        static std::set<int> done;
+        int dev = 0;
+        TDZ_CUDA(cudaGetDevice(&dev));
+        std::lock_guard<std::mutex> lk(mu);
+        if (!done.count(dev)) {
+            for (auto k : {k_transform_b3<false, false>, k_transform_b3<true, false>, k_transform_b3<false, true>})
+                TDZ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kB3Max));
+            done.insert(dev);
+        }
+    }
+    TDZ_CHECK((reinterpret_cast<uintptr_t>(in) & 15) == 0, TDZ_ERR_ARG, "transform operand not 16-byte aligned");
+    TDZ_CHECK(ldi % 4 == 0, TDZ_ERR_ARG, "transform row pitch not a multiple of 16 bytes");
+    const long long rows = 2LL * planes * R;
+    TDZ_CHECK(rows < (1LL << 31), TDZ_ERR_ARG, "transform too large");
+    B3Params prm{};
+    prm.in = in;
+    prm.in64 = in64;
+    prm.b = T.slices.as<uint8_t>();
+    prm.out = out;
+    prm.out64 = reinterpret_cast<double *>(out64);
+    prm.norm = norm;
+    prm.rows = (int)rows;
+    prm.R = R;
+    prm.K = T.K;
+    prm.N = T.N;
+    prm.Np = T.Np;
+    prm.ldi = ldi;
+    prm.ldo = ldo;
+    prm.nch = T.Kp / KC;
+    prm.tiles = (prm.rows + TM - 1) / TM;
+    prm.ns = b3_stages(T.Kp, T.Np);
+    const size_t smem = 1024 + b3_bytes(T.Kp, T.Np) + (size_t)prm.ns * kB3Stage + 256;
+    const int grid = std::min(prm.tiles, sm_count());
+    if (in64) k_transform_b3<true, false><<<grid, kB3Threads, smem, st>>>(prm);
+    else if (out64) k_transform_b3<false, true><<<grid, kB3Threads, smem, st>>>(prm);
+    else k_transform_b3<false, false><<<grid, kB3Threads, smem, st>>>(prm);
+    TDZ_CUDA(cudaGetLastError());
+    count_launch();
 }
 
 template <int NP>
 void launch(const TransformMat &T, const float *in, int ldi, TGParams prm, cudaStream_t st) {
-    const bool ws = use_ws();
+    const bool ws = variant() != 2;
     constexpr int MS = sub_tiles<NP>();
     const size_t smem = ws ? WSShape<NP>::SMEM : TGShape<NP, MS>::SMEM;
     // opt-in to the tile's shared memory once per device (guarded: the batch
@@ -587,6 +965,27 @@ void launch(const TransformMat &T, const float *in, int ldi, TGParams prm, cudaS
 
 }  // namespace
 
+namespace {
+// the process's error word; its address goes to each device before its first transform
+std::atomic<int> *error_word() {
+    static std::atomic<int> *word = [] {
+        void *p = nullptr;
+        TDZ_CUDA(cudaHostAlloc(&p, sizeof(int), cudaHostAllocMapped | cudaHostAllocPortable));
+        return new (p) std::atomic<int>(0);
+    }();
+    static std::mutex mu;
+    static std::set<int> done;
+    int dev = 0;
+    TDZ_CUDA(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    if (!done.count(dev)) {
+        TDZ_CUDA(cudaMemcpyToSymbol(g_tgemm_error, &word, sizeof(void *)));
+        done.insert(dev);
+    }
+    return word;
+}
+}  // namespace
+
 bool transform_supported(int N) { return N >= 1 && N <= 256; }
 
 void TransformMat::build(const std::vector<double> &B, int K_, int N_) {
@@ -596,6 +995,7 @@ void TransformMat::build(const std::vector<double> &B, int K_, int N_) {
     TDZ_CHECK((int)B.size() == K * N, TDZ_ERR_ARG, "transform matrix size");
     Kp = (K + KC - 1) / KC * KC;
     Np = (N + 15) / 16 * 16;
+    error_word();
     std::vector<float> h((size_t)2 * Np * Kp, 0.f);
     for (int n = 0; n < N; ++n)
         for (int k = 0; k < K; ++k) {
@@ -605,17 +1005,41 @@ void TransformMat::build(const std::vector<double> &B, int K_, int N_) {
             h[(size_t)(Np + n) * Kp + k] = tf32_round_host(v - (double)hi);
         }
     upload(hilo, h);
+    if (b3_stages(Kp, Np) > 0) {   // BF16 slices in the B-resident kernel's shared-memory order
+        std::vector<uint16_t> b((size_t)3 * Kp * Np, 0);
+        for (int n = 0; n < N; ++n)
+            for (int k = 0; k < K; ++k) {
+                double v = B[(size_t)k * N + n];
+                for (int sl = 0; sl < 3; ++sl) {
+                    float f = (float)v;
+                    uint32_t u;
+                    std::memcpy(&u, &f, 4);
+                    u = (u + 0x7FFFu + ((u >> 16) & 1u)) & 0xFFFF0000u;   // nearest BF16, ties to even
+                    std::memcpy(&f, &u, 4);
+                    v -= (double)f;
+                    const size_t off = ((size_t)(k / KC) * 3 + sl) * Np * 32 + b3_off(n, (k % KC) / 8) + (k % 8) * 2;
+                    b[off / 2] = (uint16_t)(u >> 16);
+                }
+            }
+        upload(slices, b);
+    }
     make_map(&map, hilo.ptr, Kp, 2 * (uint64_t)Np, Kp, (uint32_t)Np);
 }
 
-int take_transform_error() {
-    int h = 0;
-    TDZ_CUDA(cudaMemcpyFromSymbol(&h, g_tgemm_error, sizeof(int)));
-    if (h) {
-        const int z = 0;
-        TDZ_CUDA(cudaMemcpyToSymbol(g_tgemm_error, &z, sizeof(int)));
-    }
-    return h;
+int take_transform_error() { return error_word()->exchange(0); }
+
+bool transform_natural(const TransformMat &T) { return variant() == 0 && T.slices.ptr; }
+int transform_norm_parts(int planes, int R) {
+    return kB3Epi * (int)std::min<long long>((2LL * planes * R + TM - 1) / TM, sm_count());
+}
+void transform_from64(const TransformMat &T, const double2 *in, int planes, int R, float *out, int ldo, cudaStream_t st) {
+    TDZ_CHECK(transform_natural(T) && ldo >= R, TDZ_ERR_INTERNAL, "natural-order transform");
+    launch_b3(T, nullptr, in, planes, R, 4, out, ldo, nullptr, nullptr, st);
+}
+void transform_to64(const TransformMat &T, const float *in, int planes, int R, int ldi, double2 *out, double *norm,
+                    cudaStream_t st) {
+    TDZ_CHECK(transform_natural(T) && ldi >= T.K, TDZ_ERR_INTERNAL, "natural-order transform");
+    launch_b3(T, in, nullptr, planes, R, ldi, nullptr, 0, out, norm, st);
 }
 
 void transform(const TransformMat &T, const float *in, int planes, int R, int ldi, float *out, int ldo,
@@ -630,6 +1054,10 @@ void transform(const TransformMat &T, const float *in, int planes, int R, int ld
     prm.N = T.N;
     prm.ldo = ldo;
     prm.nchunks = T.Kp / KC;
+    if (transform_natural(T)) {
+        launch_b3(T, in, nullptr, planes, R, ldi, out, ldo, nullptr, nullptr, st);
+        return;
+    }
     switch (T.Np) {
     case 16: launch<16>(T, in, ldi, prm, st); break;
     case 32: launch<32>(T, in, ldi, prm, st); break;

@@ -1,5 +1,6 @@
 // Batched complex-by-real transforms on the 5th-generation tensor cores
-// (tcgen05, TF32 with a hi/lo split of both operands, FP32 accuracy). Internal.
+// (tcgen05; both operands as three BF16 slices, or as TF32 hi/lo pairs where B
+// is too large to stay in shared memory; FP32 accuracy). Internal.
 //
 //   out[p][n][c][r] = sum_k in[p][r][c][k] B[k][n]      (p < planes, r < R, c = re/im)
 //
@@ -25,6 +26,7 @@ namespace tdz {
 struct TransformMat {
     int K = 0, N = 0, Kp = 0, Np = 0;
     DevBuf hilo;
+    DevBuf slices;     // the three BF16 slices of B for the B-resident kernel (empty when B does not fit)
     CUtensorMap map{};
     // B is K x N, row-major, FP64
     void build(const std::vector<double> &B, int K, int N);
@@ -33,11 +35,24 @@ struct TransformMat {
 // true when the tensor-core transform handles an N x N matrix of this size
 bool transform_supported(int N);
 
-// Device error word of the transform kernels (0 = no error): a bounded wait
-// that ran out sets it; read and cleared by take_transform_error().
+// Error word of the transform kernels (0 = no error): a bounded wait that ran
+// out sets it; read and cleared here, after the caller has synchronised the
+// transforms' stream.
 int take_transform_error();
 
 void transform(const TransformMat &T, const float *in, int planes, int R, int ldi, float *out, int ldo,
                cudaStream_t st);
+
+// The first and the last transform of a chain on natural-order FP64 vectors
+// (B-resident kernel only: transform_natural), so that no layout pass is
+// needed around the chain:
+//   from64: in[(p R + r) K + k] complex FP64 (rounded to FP32), out planar
+//   to64:   in planar, out[(p N + n) R + r] complex FP64 (widened exactly);
+//           with norm (device, transform_norm_parts doubles) partial sums of |out|^2
+bool transform_natural(const TransformMat &T);
+int transform_norm_parts(int planes, int R);
+void transform_from64(const TransformMat &T, const double2 *in, int planes, int R, float *out, int ldo, cudaStream_t st);
+void transform_to64(const TransformMat &T, const float *in, int planes, int R, int ldi, double2 *out, double *norm,
+                    cudaStream_t st);
 
 }  // namespace tdz
