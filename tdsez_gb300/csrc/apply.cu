@@ -192,10 +192,10 @@ void launch_1d(const ApplyParams<T> &prm, cudaStream_t st) {
 
 // sum of the fused-reduction partials, one CTA, fixed order
 constexpr int kRedThreads = 512;
-__global__ void __launch_bounds__(kRedThreads) k_apply_red_finish(const double2 *part, double2 *out) {
+__global__ void __launch_bounds__(kRedThreads) k_apply_red_finish(const double2 *part, int n, double2 *out) {
     double2 t = make_double2(0.0, 0.0);
-#pragma unroll
-    for (int i = threadIdx.x; i < kApplyRedCap; i += kRedThreads) {
+#pragma unroll 4
+    for (int i = threadIdx.x; i < n; i += kRedThreads) {
         const double2 v = part[i];
         t.x += v.x;
         t.y += v.y;
@@ -204,8 +204,8 @@ __global__ void __launch_bounds__(kRedThreads) k_apply_red_finish(const double2 
     if (threadIdx.x == 0) *out = t;
 }
 
-void apply_red_finish(const double2 *part, double2 *out, cudaStream_t st) {
-    k_apply_red_finish<<<1, kRedThreads, 0, st>>>(part, out);
+void apply_red_finish(const double2 *part, int n, double2 *out, cudaStream_t st) {
+    k_apply_red_finish<<<1, kRedThreads, 0, st>>>(part, n, out);
     TDZ_CUDA(cudaGetLastError());
     count_launch();
 }
@@ -220,6 +220,7 @@ void launch_apply(const Operator &op, const Plan &pl, int prec, const void *x, v
         prm.red = ex.red;
         prm.dotv = ex.dotv;
         prm.red_mode = ex.red_mode;
+        prm.red_count = ex.red_count;
         prm.err = apply_error_word();
         return prm;
     };

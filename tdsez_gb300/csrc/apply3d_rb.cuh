@@ -603,6 +603,7 @@ inline void run3d_rb(const ApplyParams<T> &prm0, cudaStream_t st) {
         prm.zchunk = seg;
         prm.zchunk_planes = std::min(seg, n2) + 2 * P;
         const unsigned grid = (unsigned)((total + seg - 1) / seg);
+        if (prm.red_mode) *prm.red_count = (int)grid;
         const size_t smem = Sh::smem(prm.zchunk_planes);
         TDZ_CHECK(smem <= kMaxDyn, TDZ_ERR_UNSUPPORTED, "outer axis too long for the 3D apply");
         kern<<<grid, dim3(txw, NTY), smem, st>>>(prm, map);

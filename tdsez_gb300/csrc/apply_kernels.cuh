@@ -55,6 +55,7 @@ template <class T> struct ApplyParams {
     const void *dotv;
     int red_mode;
     int *err;                   // error word of bounded waits (device, library-owned)
+    int *red_count;             // host: number of partial sums the launch writes (not read by kernels)
 };
 
 
@@ -589,6 +590,7 @@ inline void run3d(const ApplyParams<T> &prm0, cudaStream_t st) {
         prm.zchunk = seg;
         prm.zchunk_planes = std::min(seg, n2) + 2 * P;
         const unsigned grid = (unsigned)((total + seg - 1) / seg);
+        if (prm.red_mode) *prm.red_count = (int)grid;
         TDZ_CHECK(smem_for(std::min(seg, n2)) <= kMaxDyn, TDZ_ERR_UNSUPPORTED, "outer axis too long for the 3D apply");
         kern<<<grid, dim3(txw, TY), smem_for(std::min(seg, n2)), st>>>(prm);
     };

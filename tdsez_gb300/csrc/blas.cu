@@ -454,12 +454,7 @@ void Reducer::init() {
     const int nb = red_blocks();
     partial.alloc(sizeof(double2) * (kMaxDot + 1) * nb);
     result.alloc(sizeof(double2) * (kMaxDot + 1));
-    if (!host) TDZ_CUDA(cudaMallocHost(reinterpret_cast<void **>(&host), sizeof(double2) * (kMaxDot + 1)));
     blocks = nb;   // last: a Reducer with blocks != 0 has all its buffers
-}
-
-Reducer::~Reducer() {
-    if (host) cudaFreeHost(host);
 }
 
 void mdot(Reducer &r, const void *const *V, int k, const void *w, size_t n, int prec, cd *out, cudaStream_t st) {
@@ -473,10 +468,10 @@ void mdot(Reducer &r, const void *const *V, int k, const void *w, size_t n, int 
         else mdot_dispatch<float>(kk, pp, w, n, r.partial.as<double2>(), nb, st);
         k_finish<<<kk, kThreads, 0, st>>>(r.partial.as<double2>(), nb, r.result.as<double2>());
         TDZ_CUDA(cudaGetLastError());
-    count_launch();
-        TDZ_CUDA(cudaMemcpyAsync(r.host, r.result.ptr, sizeof(double2) * kk, cudaMemcpyDeviceToHost, st));
+        count_launch();
         TDZ_CUDA(cudaStreamSynchronize(st));
-        for (int i = 0; i < kk; ++i) out[c0 + i] = cd(r.host[i].x, r.host[i].y);
+        const volatile double *h = r.result.as<double>();
+        for (int i = 0; i < kk; ++i) out[c0 + i] = cd(h[2 * i], h[2 * i + 1]);
     }
 }
 
@@ -554,12 +549,12 @@ void gs_update(Reducer &r, void *w, int k, const void *const *V, const cd *a, si
     k_finish<<<nres, kThreads, 0, st>>>(part, nb, r.result.as<double2>());
     TDZ_CUDA(cudaGetLastError());
     count_launch(2);
-    TDZ_CUDA(cudaMemcpyAsync(r.host, r.result.ptr, sizeof(double2) * nres, cudaMemcpyDeviceToHost, st));
     TDZ_CUDA(cudaStreamSynchronize(st));
+    const volatile double *h = r.result.as<double>();
     if (dots)
-        for (int i = 0; i < k; ++i) dots[i] = cd(r.host[i].x, r.host[i].y);
+        for (int i = 0; i < k; ++i) dots[i] = cd(h[2 * i], h[2 * i + 1]);
     if (norm) {
-        const double v = r.host[nres - 1].x;
+        const double v = h[2 * (nres - 1)];
         *norm = std::isfinite(v) ? std::sqrt(std::max(0.0, v)) : std::numeric_limits<double>::quiet_NaN();
     }
 }

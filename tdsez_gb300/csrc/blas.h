@@ -29,12 +29,9 @@ void add_cast(double2 *y, cd a, const float2 *x, size_t n, cudaStream_t st);
 // Reduction workspace: per-block partial sums and device results.
 struct Reducer {
     DevBuf partial;   // [kMaxDot + 1][blocks] double2
-    DevBuf result;    // [kMaxDot + 1] double2
-    DevBuf hostbuf;   // pinned host mirror of result
-    double2 *host = nullptr;
+    HostBuf result;   // [kMaxDot + 1] double2, written by the last kernel of a reduction
     int blocks = 0;
     void init();
-    ~Reducer();
 };
 
 // out[i] = <V_i, w> = sum conj(V_i) w for i < k (any k; chunks of kMaxDot),

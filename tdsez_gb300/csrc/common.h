@@ -77,6 +77,26 @@ struct DevBuf {
     template <class T> T *as() const { return static_cast<T *>(ptr); }
 };
 
+// Pinned host memory that kernels write directly: results the host needs after
+// the next synchronisation of their stream, without a copy of their own.
+struct HostBuf {
+    void *ptr = nullptr;
+    HostBuf() = default;
+    HostBuf(const HostBuf &) = delete;
+    HostBuf &operator=(const HostBuf &) = delete;
+    ~HostBuf() { release(); }
+    void alloc(size_t b) {
+        release();
+        TDZ_CUDA(cudaHostAlloc(&ptr, b, cudaHostAllocMapped | cudaHostAllocPortable));
+    }
+    void release() {
+        if (ptr) cudaFreeHost(ptr);
+        ptr = nullptr;
+    }
+    // read by the host after a synchronisation (volatile: kernels write it)
+    template <class T> T *as() const { return static_cast<T *>(ptr); }
+};
+
 template <class T> inline void upload(DevBuf &b, const std::vector<T> &v) {
     b.alloc(v.size() * sizeof(T));
     if (!v.empty()) TDZ_CUDA(cudaMemcpy(b.ptr, v.data(), v.size() * sizeof(T), cudaMemcpyHostToDevice));

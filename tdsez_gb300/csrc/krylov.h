@@ -46,7 +46,7 @@ struct FGMRES {
     Precond *pc = nullptr;
     std::vector<DevBuf> V, Z;
     DevBuf w;
-    DevBuf znd;                 // ||z_j||^2 of relaxed columns from the preconditioner's output pass
+    HostBuf znd;                // ||z_j||^2 of relaxed columns from the preconditioner's output pass
     blas::Reducer red;
     SolveStats last;
     long long applies = 0;
@@ -71,11 +71,13 @@ struct FGMRES {
 
     void setup(Operator *op_, int restart_, Precond *pc_);
     // Solve A x = b (A = the operator's current stage, FP64), x holds the guess.
-    // bnorm: ||b|| when the caller has it (< 0: computed here). cn_psi: when
+    // bnorm2: ||b||^2 (real part) when the caller has it on the way, valid after
+    // the next synchronisation of st (null: computed here). cn_psi: when
     // the solve converges after one iteration, its last update is fused with
     // the Crank-Nicolson state update psi = 2 x - psi (*cn_done = true; x is
     // then left at its initial guess); otherwise x is the solution as usual.
-    SolveStats solve(const double2 *b, double2 *x, double rtol, int maxit, cudaStream_t st, double bnorm = -1.0,
+    SolveStats solve(const double2 *b, double2 *x, double rtol, int maxit, cudaStream_t st,
+                     const double2 *bnorm2 = nullptr,
                      double2 *cn_psi = nullptr, bool *cn_done = nullptr);
 };
 

@@ -287,21 +287,21 @@ bool Operator::fused_reductions() const { return sp->dim == 3 && !quad.on; }
 
 namespace {
 // one fused-reduction result to the host (synchronises the stream)
-cd take_reduction(Operator &op, cudaStream_t st) {
-    apply_red_finish(op.red_part.as<double2>(), op.red_res.as<double2>(), st);
-    double2 v;
-    TDZ_CUDA(cudaMemcpyAsync(&v, op.red_res.ptr, sizeof(double2), cudaMemcpyDeviceToHost, st));
+cd take_reduction(Operator &op, int parts, cudaStream_t st) {
+    apply_red_finish(op.red_part.as<double2>(), parts, op.red_res.as<double2>(), st);
     TDZ_CUDA(cudaStreamSynchronize(st));
-    return cd(v.x, v.y);
+    const volatile double *v = op.red_res.as<double>();
+    return cd(v[0], v[1]);
 }
 void ensure_red(Operator &op) {
     if (op.red_part.ptr) return;
     op.red_part.alloc(sizeof(double2) * kApplyRedCap);
-    op.red_res.alloc(sizeof(double2));
+    op.red_res.alloc(2 * sizeof(double2));
 }
 }  // namespace
 
-void Operator::residual(int which, int prec, const void *x, const void *b, void *y, cudaStream_t st, double *norm) {
+void Operator::residual(int which, int prec, const void *x, const void *b, void *y, cudaStream_t st, double *norm,
+                        const double2 **pending) {
     TDZ_CHECK(prec == TDZ_FP32 || prec == TDZ_FP64 || prec == TDZ_FP64_DF || (prec == kPrecF32M64 && f32_on_f64()),
               TDZ_ERR_ARG, "precision must be TDZ_FP32, TDZ_FP64, TDZ_FP64_DF or (3D, no soft-core term) TDZ_FP64_F32");
     TDZ_CHECK(x && y, TDZ_ERR_ARG, "null vector");
@@ -310,10 +310,12 @@ void Operator::residual(int which, int prec, const void *x, const void *b, void 
     Plan &pl = plan(which);
     ApplyExtra ex;
     ex.sub = b;
-    const bool fused = norm && fused_reductions();
+    const bool fused = (norm || pending) && fused_reductions();
+    TDZ_CHECK(!pending || (fused && !norm), TDZ_ERR_INTERNAL, "pending norm of an unfused apply");
+    int parts = 0;
     if (fused) {
         ensure_red(*this);
-        TDZ_CUDA(cudaMemsetAsync(red_part.ptr, 0, sizeof(double2) * kApplyRedCap, st));
+        ex.red_count = &parts;
         ex.red = red_part.as<double2>();
         ex.red_mode = 1;
     }
@@ -324,9 +326,13 @@ void Operator::residual(int which, int prec, const void *x, const void *b, void 
         quad.apply(b ? -coef : coef, prec, x, y, st);
     }
     ++launches;
+    if (pending) {
+        apply_red_finish(red_part.as<double2>(), parts, red_res.as<double2>() + 1, st);
+        *pending = red_res.as<double2>() + 1;
+    }
     if (norm) {
         if (fused) {
-            const double v = take_reduction(*this, st).real();
+            const double v = take_reduction(*this, parts, st).real();
             *norm = std::isfinite(v) ? std::sqrt(std::max(0.0, v)) : std::numeric_limits<double>::quiet_NaN();
         } else {
             *norm = blas::nrm2(red, y, (size_t)sp->ndof(), prec == TDZ_FP32 ? TDZ_FP32 : TDZ_FP64, st);
@@ -348,14 +354,15 @@ void Operator::apply_dot(int which, int prec, const void *x, void *y, const void
     if (which == TDZ_STAGE) TDZ_CHECK(stage_set, TDZ_ERR_STATE, "stage coefficients not set");
     Plan &pl = plan(which);
     ensure_red(*this);
-    TDZ_CUDA(cudaMemsetAsync(red_part.ptr, 0, sizeof(double2) * kApplyRedCap, st));
+    int parts = 0;
     ApplyExtra ex;
+    ex.red_count = &parts;
     ex.red = red_part.as<double2>();
     ex.dotv = v;
     ex.red_mode = 2;
     launch_apply(*this, pl, prec, x, y, st, ex);
     ++launches;
-    *dot = take_reduction(*this, st);
+    *dot = take_reduction(*this, parts, st);
 }
 
 void Operator::observables(const double2 *psi, std::vector<cd> &out, cudaStream_t st) {

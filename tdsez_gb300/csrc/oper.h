@@ -82,11 +82,15 @@ struct Operator {
     // y = b - op x in one pass (b and y FP64 for TDZ_FP64 / TDZ_FP64_DF);
     // b may be null (y = op x). With norm: *norm = ||y|| (fused into the
     // store for 3D operators without the quadrature term; synchronises)
+    // With pending (fused_reductions() operators): no synchronisation; *pending
+    // points at the sum of squares, valid after the next synchronisation of
+    // the stream and until the next pending call
     void residual(int which, int prec, const void *x, const void *b, void *y, cudaStream_t st,
-                  double *norm = nullptr);
+                  double *norm = nullptr, const double2 **pending = nullptr);
     // y = op x and *dot = <v, y> = sum conj(v) y (FP64 vectors; synchronises)
     void apply_dot(int which, int prec, const void *x, void *y, const void *v, cd *dot, cudaStream_t st);
-    DevBuf red_part, red_res;      // fused-reduction partials and result
+    DevBuf red_part;               // fused-reduction partials
+    HostBuf red_res;               // and results: [0] of a call that returns one, [1] pending (below)
     blas::Reducer red;             // unfused reductions (allocated on first use, then reused)
     bool fused_reductions() const;
     // upper bound on || |A| ||_2 for operator `which` at the current stage:
@@ -114,13 +118,14 @@ void set_forced_shape(int txw, int run);
 // non-null (a residual); for 3D, per-CTA partial sums of |y|^2 (red_mode 1)
 // or of conj(dotv) y (red_mode 2) into red[0 .. kApplyRedCap).
 constexpr int kApplyRedCap = 4096;   // partial-sum slots (CTAs of one 3D launch)
-// red[0 .. kApplyRedCap) summed into *out (device), fixed order
-void apply_red_finish(const double2 *part, double2 *out, cudaStream_t st);
+// part[0 .. n) summed into *out (device or pinned host), fixed order
+void apply_red_finish(const double2 *part, int n, double2 *out, cudaStream_t st);
 struct ApplyExtra {
     const void *sub = nullptr;
     double2 *red = nullptr;
     const void *dotv = nullptr;
     int red_mode = 0;
+    int *red_count = nullptr;   // receives the number of partial sums (red_mode != 0)
 };
 void launch_apply(const Operator &op, const Plan &pl, int prec, const void *x, void *y, cudaStream_t st,
                   const ApplyExtra &ex = ApplyExtra{});

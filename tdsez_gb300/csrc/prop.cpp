@@ -73,9 +73,9 @@ void Solver::setup(Operator *op_, const SolverOptions &o, cudaStream_t st) {
     ksp.aprec = o.outer;
 }
 
-SolveStats Solver::solve(const double2 *b, double2 *x, cudaStream_t st, double bnorm, double2 *cn_psi,
+SolveStats Solver::solve(const double2 *b, double2 *x, cudaStream_t st, const double2 *bnorm2, double2 *cn_psi,
                          bool *cn_done) {
-    SolveStats s = ksp.solve(b, x, opt.rtol, opt.maxit, st, bnorm, cn_psi, cn_done);
+    SolveStats s = ksp.solve(b, x, opt.rtol, opt.maxit, st, bnorm2, cn_psi, cn_done);
     if (opt.pc == 3 && static_cast<PcFDM *>(pc.get())->tensor)
         TDZ_CHECK(take_transform_error() == 0, TDZ_ERR_CUDA, "tensor-core transform: a bounded wait ran out");
     ++solves;
@@ -127,9 +127,9 @@ void Propagator::record(int slot, const double2 *y, const double2 *x, cudaStream
     hist_count[slot] = std::min(hist_count[slot] + 1, guess_order);
 }
 
-void Propagator::stage_solve(int k, const double2 *b, double2 *x, cudaStream_t st, double bnorm, double2 *cn_psi,
+void Propagator::stage_solve(int k, const double2 *b, double2 *x, cudaStream_t st, const double2 *bnorm2, double2 *cn_psi,
                              bool *cn_done) {
-    SolveStats s = solver[k].solve(b, x, st, bnorm, cn_psi, cn_done);
+    SolveStats s = solver[k].solve(b, x, st, bnorm2, cn_psi, cn_done);
     last = s;
     ++solves;
     its += s.its;
@@ -144,8 +144,9 @@ void Propagator::stage_solve(int k, const double2 *b, double2 *x, cudaStream_t s
 
 void Propagator::cn_step(double2 *psi, double h, const std::vector<cd> &c, cudaStream_t st) {
     op->set_stage(1.0, cd(0.0, 0.5 * h), c);
-    double bn = -1.0;
-    op->residual(TDZ_MASS, aprec, psi, nullptr, rhs.ptr, st, op->fused_reductions() ? &bn : nullptr);   // M psi
+    // M psi; ||M psi||^2 is read with the solve's first residual norm
+    const double2 *bn = nullptr;
+    op->residual(TDZ_MASS, aprec, psi, nullptr, rhs.ptr, st, nullptr, op->fused_reductions() ? &bn : nullptr);
     double2 *X = tmp.as<double2>();
     if (guess_order < 0) {
         solver[0].pc->apply(rhs.as<double2>(), X, st);           // x0 = P^-1 b
