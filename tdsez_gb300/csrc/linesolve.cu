@@ -88,7 +88,7 @@ template <class T> struct TileArgs {
     // epilogue of a Chebyshev step (ch_x set): d = a z + b d, x = (set ? d : x + d)
     typename CT<T>::type *ch_d, *ch_x;
     T ar, ai, br, bi;
-    int ch_set;
+    int ch_set, ch_keep;
 };
 
 template <class T> __device__ __forceinline__ void cp_async_c(void *dst, const void *src) {
@@ -230,6 +230,7 @@ __global__ void __launch_bounds__(32 * kTileWarps<T>) k_line_tile(const TileArgs
                 g.dst[e] = z;
                 continue;
             }
+            if (g.ch_keep) g.dst[e] = z;
             C o;
             o.x = g.ar * z.x - g.ai * z.y;
             o.y = g.ar * z.y + g.ai * z.x;
@@ -406,6 +407,7 @@ bool run_axis(const BandChol &F, int axis, const typename CT<T>::type *src, type
             g.br = (T)ch->b.real();
             g.bi = (T)ch->b.imag();
             g.ch_set = ch->set ? 1 : 0;
+            g.ch_keep = ch->keep ? 1 : 0;
             fused = true;
         }
         // warps per CTA: the fewest waves of tiles (shared memory decides how many

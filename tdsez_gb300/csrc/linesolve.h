@@ -18,16 +18,16 @@ struct BandChol {
 };
 
 // Epilogue of a Chebyshev step on the solution z: d = a z + b d, x = d (set)
-// or x + d. z itself need not be stored.
+// or x + d. z itself is stored only with keep.
 struct ChebStep {
     cd a, b;
     void *d, *x;
-    bool set;
+    bool set, keep;
 };
 
 // dst = (A_axis^-1 along one axis) src for an array of shape (n2, n1, n0), x
 // fastest; dst may be src. With ch the epilogue takes the place of the store
-// of dst where the kernel can (returns true); dst then holds nothing useful.
+// of dst where the kernel can (returns true); dst then holds z only with keep.
 bool line_solve(const BandChol &F, int axis, const void *src, void *dst, int n0, int n1, int n2, int prec,
                 cudaStream_t st, const ChebStep *ch = nullptr);
 

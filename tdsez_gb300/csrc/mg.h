@@ -11,6 +11,7 @@
 // Kronecker line solves); coarsest level: Chebyshev over the whole segment.
 #pragma once
 
+#include <array>
 #include <memory>
 #include <vector>
 
@@ -32,11 +33,31 @@ struct RowSparse {
     void upload();
 };
 
+// Chebyshev steps with dense per-axis matrices M_d^-1 B (small 3D FP32 levels,
+// mg_dense.cu).
+struct DenseLevel {
+    bool ok = false;                      // matrices built
+    bool ready = false;                   // combined for the current stage
+    std::array<cd, 5> at{};               // the stage scalars it was combined for
+    bool has_c = false;
+    int n[3] = {1, 1, 1}, pd = 0, py = 0, pz = 0;
+    DevBuf base[3];                       // per axis M_d^-1 B of every base band, [band][n][n] FP32
+    DevBuf rx, ry, rz, cz;                // the stage's combinations (transposed, padded)
+    static bool pays(const int *n, size_t ndof);
+    void build(const Operator &op, const int *n);
+    // matrices of the operator's current stage; false when the stage is outside
+    // the form (complex ratios to g)
+    bool prepare(const Operator &op, cudaStream_t st);
+    // z -= M^-1 A d, d = a z + b d, x += d (u: scratch)
+    void step(const Operator &op, void *z, void *d, void *x, void *u, cd a, cd b, cudaStream_t st) const;
+};
+
 struct MGLevel {
     Space space;                          // sizes of the level
     std::unique_ptr<Operator> op;         // level operator (bands = Galerkin products)
     Operator *opp = nullptr;              // op.get() or the fine operator
     KronSolve minv;
+    DenseLevel dense;
     RowSparse P[3], R[3];                 // to this level from the next coarser: prolongation, restriction
     int n[3] = {1, 1, 1};
     size_t ndof = 0;

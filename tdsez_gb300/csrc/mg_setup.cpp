@@ -244,6 +244,9 @@ void Multigrid::setup(Operator *fine_, const MGOptions &o, cudaStream_t st) {
         const size_t es = prec == TDZ_FP64 ? sizeof(double2) : sizeof(float2);
         for (DevBuf *b : {&m.x, &m.b, &m.r, &m.d, &m.z, &m.t1, &m.t2}) b->alloc(m.ndof * es);
     }
+    if (prec == TDZ_FP32)
+        for (auto &m : lv)
+            if (DenseLevel::pays(m.n, m.ndof)) m.dense.build(*m.opp, m.n);
     red.init();
     estimate_bounds(st);
     if (opt.learned) learned_setup();
@@ -344,20 +347,26 @@ void chebyshev(MGLevel &m, int prec, double mu_a, double mu_b, double w, int ste
         op.residual(TDZ_STAGE, prec, m.x.ptr, m.b.ptr, m.r.ptr, st);
         r = m.r.ptr;
     }
-    // A step is one apply (r -= A d in its store) and the line solves of M^-1 r,
-    // whose last axis forms d and x from z while it stores (ChebStep).
     const bool degenerate = std::abs(delta) <= 1e-12 * std::abs(theta);   // damped Richardson, one step
     const cd sigma1 = degenerate ? cd(1.0) : theta / delta;
     cd rho = 1.0 / sigma1;
-    const ChebStep first{1.0 / theta, 0.0, m.d.ptr, m.x.ptr, x_zero};
+    const bool dense = m.dense.ready && m.dense.at == op.sigma && steps > 1 && !degenerate;
+    ChebStep first{1.0 / theta, 0.0, m.d.ptr, m.x.ptr, x_zero, dense};
     m.minv.apply(r, m.z.ptr, prec, st, &first);
     if (degenerate) return;
     for (int k = 1; k < steps; ++k) {
-        op.residual(TDZ_STAGE, prec, m.d.ptr, r, m.r.ptr, st);
-        r = m.r.ptr;
         const cd rn = 1.0 / (2.0 * sigma1 - rho);
-        const ChebStep next{2.0 * rn / delta, rn * rho, m.d.ptr, m.x.ptr, false};
-        m.minv.apply(r, m.z.ptr, prec, st, &next);
+        if (dense) {
+            // small level: z = M^-1 r updated by dense axis matrices (mg_dense.cu)
+            m.dense.step(op, m.z.ptr, m.d.ptr, m.x.ptr, m.t1.ptr, 2.0 * rn / delta, rn * rho, st);
+        } else {
+            // one apply (r -= A d in its store) and the line solves of M^-1 r, whose
+            // last axis forms d and x from z while it stores (ChebStep)
+            op.residual(TDZ_STAGE, prec, m.d.ptr, r, m.r.ptr, st);
+            r = m.r.ptr;
+            const ChebStep next{2.0 * rn / delta, rn * rho, m.d.ptr, m.x.ptr, false, false};
+            m.minv.apply(r, m.z.ptr, prec, st, &next);
+        }
         rho = rn;
     }
 }
@@ -419,6 +428,7 @@ void Multigrid::vcycle(int l, cudaStream_t st) {
 void Multigrid::apply(const double2 *r, double2 *z, cudaStream_t st) {
     // coarse levels follow the current stage scalars of the fine operator
     for (size_t l = 1; l < lv.size(); ++l) lv[l].opp->sigma = fine->sigma;
+    for (auto &m : lv) m.dense.prepare(*m.opp, st);
     MGLevel &f = lv[0];
     blas::cast(r, TDZ_FP64, f.b.ptr, prec, f.ndof, st);
     vcycle(0, st);
