@@ -297,6 +297,7 @@ struct ZSolveParams {
     const float *lxi, *lyi; // their imaginary parts (complex axis pencils), else null
     int n0, n1, n2;
     CombP<float> Bc, Cc;    // A_z(s) = Bc + s Cc
+    float4 *fac;            // stored factor (k_zfac): [half][row][line][pairs of entries], or null
 };
 
 // ---- line solves along the outer axis: banded complex L D L^T (no pivoting),
@@ -375,6 +376,68 @@ __device__ __forceinline__ float2 csubf(float2 a, float2 b) { return make_float2
 __device__ __forceinline__ void csubmul(float2 &acc, float2 a, float2 b) {
     acc.x = fmaf(a.y, b.y, fmaf(-a.x, b.x, acc.x));
     acc.y = fmaf(-a.y, b.x, fmaf(-a.x, b.y, acc.y));
+}
+
+// the 2P x 2P system at the cut: U1 T1 + W1 T2 = c1, U2 T2 + W2 T1 = c2 (U unit
+// upper triangular, its diagonal not stored)
+template <int P>
+__device__ __forceinline__ void twist_solve(const float2 (&U1)[P][P], const float2 (&W1)[P][P], const float2 (&c1)[P],
+                                            const float2 (&U2)[P][P], const float2 (&W2)[P][P], const float2 (&c2)[P],
+                                            float2 (&T1)[P], float2 (&T2)[P]) {
+    // z1 = U1^-1 c1, M1 = U1^-1 W1 (unit upper triangular)
+    float2 z1[P], M1[P][P];
+#pragma unroll
+    for (int r = P - 1; r >= 0; --r) {
+        z1[r] = c1[r];
+#pragma unroll
+        for (int k = 0; k < P; ++k) M1[r][k] = W1[r][k];
+#pragma unroll
+        for (int q = r + 1; q < P; ++q) {
+            z1[r] = csubf(z1[r], cmulf(U1[r][q], z1[q]));
+#pragma unroll
+            for (int k = 0; k < P; ++k) M1[r][k] = csubf(M1[r][k], cmulf(U1[r][q], M1[q][k]));
+        }
+    }
+    // S = U2 + I - W2 M1 (U2 holds the strict upper part), g = c2 - W2 z1
+    float2 S[P][P], g[P];
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+        g[r] = c2[r];
+#pragma unroll
+        for (int k = 0; k < P; ++k) S[r][k] = k == r ? make_float2(1.f, 0.f) : U2[r][k];
+#pragma unroll
+        for (int q = 0; q < P; ++q) {
+            g[r] = csubf(g[r], cmulf(W2[r][q], z1[q]));
+#pragma unroll
+            for (int k = 0; k < P; ++k) S[r][k] = csubf(S[r][k], cmulf(W2[r][q], M1[q][k]));
+        }
+    }
+    // S T2 = g: Gaussian elimination without pivoting, then T1 = z1 - M1 T2
+#pragma unroll
+    for (int c = 0; c < P; ++c) {
+        const float2 inv = crecf(S[c][c]);
+#pragma unroll
+        for (int r = c + 1; r < P; ++r) {
+            const float2 f = cmulf(S[r][c], inv);
+#pragma unroll
+            for (int k = c + 1; k < P; ++k) S[r][k] = csubf(S[r][k], cmulf(f, S[c][k]));
+            g[r] = csubf(g[r], cmulf(f, g[c]));
+        }
+        S[c][c] = inv;
+    }
+#pragma unroll
+    for (int r = P - 1; r >= 0; --r) {
+        float2 v = g[r];
+#pragma unroll
+        for (int k = r + 1; k < P; ++k) v = csubf(v, cmulf(S[r][k], T2[k]));
+        T2[r] = cmulf(v, S[r][r]);
+    }
+#pragma unroll
+    for (int r = 0; r < P; ++r) {
+        T1[r] = z1[r];
+#pragma unroll
+        for (int k = 0; k < P; ++k) T1[r] = csubf(T1[r], cmulf(M1[r][k], T2[k]));
+    }
 }
 
 template <int P, bool CI>
@@ -513,60 +576,7 @@ __global__ void __launch_bounds__(2 * kZLines, P <= 3 ? 3 : 2) k_zsolve(const ZS
         tail(li, U1, W1, c1);
         tail(li + kZLines, U2, W2, c2);
         __syncthreads();   // the exchange buffer is this thread's u block from here on
-        // z1 = U1^-1 c1, M1 = U1^-1 W1 (unit upper triangular)
-        float2 z1[P], M1[P][P];
-#pragma unroll
-        for (int r = P - 1; r >= 0; --r) {
-            z1[r] = c1[r];
-#pragma unroll
-            for (int k = 0; k < P; ++k) M1[r][k] = W1[r][k];
-#pragma unroll
-            for (int q = r + 1; q < P; ++q) {
-                z1[r] = csubf(z1[r], cmulf(U1[r][q], z1[q]));
-#pragma unroll
-                for (int k = 0; k < P; ++k) M1[r][k] = csubf(M1[r][k], cmulf(U1[r][q], M1[q][k]));
-            }
-        }
-        // S = U2 + I - W2 M1 (U2 holds the strict upper part), g = c2 - W2 z1
-        float2 S[P][P], g[P];
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-            g[r] = c2[r];
-#pragma unroll
-            for (int k = 0; k < P; ++k) S[r][k] = k == r ? make_float2(1.f, 0.f) : U2[r][k];
-#pragma unroll
-            for (int q = 0; q < P; ++q) {
-                g[r] = csubf(g[r], cmulf(W2[r][q], z1[q]));
-#pragma unroll
-                for (int k = 0; k < P; ++k) S[r][k] = csubf(S[r][k], cmulf(W2[r][q], M1[q][k]));
-            }
-        }
-        // S T2 = g: Gaussian elimination without pivoting, then T1 = z1 - M1 T2
-#pragma unroll
-        for (int c = 0; c < P; ++c) {
-            const float2 inv = crecf(S[c][c]);
-#pragma unroll
-            for (int r = c + 1; r < P; ++r) {
-                const float2 f = cmulf(S[r][c], inv);
-#pragma unroll
-                for (int k = c + 1; k < P; ++k) S[r][k] = csubf(S[r][k], cmulf(f, S[c][k]));
-                g[r] = csubf(g[r], cmulf(f, g[c]));
-            }
-            S[c][c] = inv;
-        }
-#pragma unroll
-        for (int r = P - 1; r >= 0; --r) {
-            float2 v = g[r];
-#pragma unroll
-            for (int k = r + 1; k < P; ++k) v = csubf(v, cmulf(S[r][k], T2[k]));
-            T2[r] = cmulf(v, S[r][r]);
-        }
-#pragma unroll
-        for (int r = 0; r < P; ++r) {
-            T1[r] = z1[r];
-#pragma unroll
-            for (int k = 0; k < P; ++k) T1[r] = csubf(T1[r], cmulf(M1[r][k], T2[k]));
-        }
+        twist_solve<P>(U1, W1, c1, U2, W2, c2, T1, T2);
     }
 
     // backward pass of this half; local row rows + c is the partner's tail row P-1-c
@@ -627,7 +637,249 @@ __global__ void __launch_bounds__(2 * kZLines, P <= 3 ? 3 : 2) k_zsolve(const ZS
     }
 }
 
-template <int P, bool CI> void launch_zsolve_t(const ZSolveParams &zp, cudaStream_t st) {
+// ---- stored factor, for small problems
+// The line matrices change only with the stage coefficients, and a stage solve
+// applies the preconditioner several times. Where the whole factor stays in
+// L2, k_zfac stores the reciprocal pivot and the unit factor row of every row
+// once per stage, and k_zsub only substitutes: P complex multiply-subtracts per
+// row and pass against the 14 (P = 4) of an elimination plus its repetition.
+// With few lines both are bound by one warp's issue rate and dependent
+// products, so a row's instructions are what counts: its factor is one padded
+// record per line, fetched by 16-byte asynchronous copies into a ring of
+// kRing rows with static slots, and L^-1 r stays in shared memory. 260 lines of
+// 260 rows, P = 4: 59 us per application (k_zbands and k_zsolve) before,
+// 30 us now; with one 8-byte copy per entry and computed addresses 65 us.
+constexpr int kZSubLines = 32;
+template <int P> struct ZFac {
+    static constexpr int FP = (P + 2) / 2;                      // float4 per record (1/u(k,k), unit row, padding)
+    static constexpr int kRing = P == 3 || P == 5 ? 15 : 16;    // a multiple of P
+    static_assert(kRing % P == 0, "static ring slots");
+    static_assert(P * (P + 1) <= kRing * 2 * FP, "the ring doubles as the exchange buffer");
+};
+template <int P> size_t zsub_smem(int n2) {
+    const size_t rows = (size_t)z_blocks(n2, ZBlk<P>::B) * ZBlk<P>::B;
+    return (ZFac<P>::kRing * (2 * ZFac<P>::FP + 1) + rows) * 2 * kZSubLines * sizeof(float2);
+}
+__device__ __forceinline__ void cp_async16(float4 *dst, const float4 *src) {
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async8(void *dst, const void *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async4(float *dst, const float *src) {
+    asm volatile("cp.async.ca.shared.global [%0], [%1], 4;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src)
+                 : "memory");
+}
+__device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;" ::"n"(N) : "memory");
+}
+
+template <int P, bool CI> __global__ void __launch_bounds__(2 * kZSubLines) k_zfac(const ZSolveParams prm) {
+    constexpr int B = ZBlk<P>::B;
+    const int n = prm.n2, rows = z_blocks(n, B) * B;
+    const int half = threadIdx.x / kZSubLines, nl = prm.n0 * prm.n1;
+    const int l = blockIdx.x * kZSubLines + threadIdx.x % kZSubLines;
+    if (l >= nl) return;
+    const int i = l % prm.n0, j = l / prm.n0;
+    const float s = prm.lx[i] + (prm.ly ? prm.ly[j] : 0.f);
+    const float si = CI ? prm.lxi[i] + (prm.lyi ? prm.lyi[j] : 0.f) : 0.f;
+    const float4 *zt = prm.zb + (size_t)half * rows * (P + 1);
+    constexpr int FP = ZFac<P>::FP;
+    float4 *out = prm.fac + ((size_t)half * rows * nl + l) * FP;
+    float2 U[P][P], F[P][P];   // u(k, k+q) and u(k, k+q) / u(k, k) of the last P rows
+#pragma unroll
+    for (int d = 0; d < P; ++d)
+#pragma unroll
+        for (int q = 0; q < P; ++q) U[d][q] = F[d][q] = make_float2(0.f, 0.f);
+    float4 z[P + 1];
+#pragma unroll
+    for (int q = 0; q <= P; ++q) z[q] = zt[q];
+    for (int k0 = 0; k0 < rows; k0 += P) {
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+            const int k = k0 + r;
+            float2 a[P + 1];
+#pragma unroll
+            for (int q = 0; q <= P; ++q) {
+                a[q] = CI ? make_float2(fmaf(-si, z[q].w, fmaf(s, z[q].z, z[q].x)), fmaf(si, z[q].z, fmaf(s, z[q].w, z[q].y)))
+                          : make_float2(fmaf(s, z[q].z, z[q].x), fmaf(s, z[q].w, z[q].y));
+                if (k + 1 < rows) z[q] = zt[(size_t)(k + 1) * (P + 1) + q];
+            }
+#pragma unroll
+            for (int d = P; d >= 1; --d) {
+                const int o = (r + P - d) % P;
+#pragma unroll
+                for (int q = 0; q + d <= P; ++q) csubmul(a[q], F[o][d - 1], U[o][d + q - 1]);
+            }
+            float2 rec[2 * FP];
+            rec[0] = crecf(a[0]);
+            rec[2 * FP - 1] = make_float2(0.f, 0.f);
+#pragma unroll
+            for (int q = 0; q < P; ++q) {
+                U[r][q] = a[q + 1];
+                rec[q + 1] = F[r][q] = cmulf(a[q + 1], rec[0]);
+            }
+#pragma unroll
+            for (int h = 0; h < FP; ++h)
+                out[(size_t)k * nl * FP + h] = make_float4(rec[2 * h].x, rec[2 * h].y, rec[2 * h + 1].x, rec[2 * h + 1].y);
+        }
+    }
+}
+
+// IL: the lines' real and imaginary parts are neighbours (cs = 1)
+template <int P, bool IL> __global__ void __launch_bounds__(2 * kZSubLines) k_zsub(const ZSolveParams prm) {
+    constexpr int B = ZBlk<P>::B, T = 2 * kZSubLines, FP = ZFac<P>::FP, D = ZFac<P>::kRing;
+    extern __shared__ float4 zs_smem[];
+    const int n = prm.n2, rows = z_blocks(n, B) * B;
+    float4 *rf = zs_smem + threadIdx.x;                                           // [slot][FP][thread]
+    float2 *rx = reinterpret_cast<float2 *>(zs_smem + D * FP * T) + threadIdx.x;  // [slot][thread]
+    float2 *sy = rx + D * T;                                                      // [row][thread]: L^-1 r
+    const int half = threadIdx.x / kZSubLines, li = threadIdx.x % kZSubLines, nl = prm.n0 * prm.n1;
+    const int lraw = blockIdx.x * kZSubLines + li;
+    const bool valid = lraw < nl;
+    const int l = valid ? lraw : nl - 1;
+    const int h0 = z_half(n), pad = rows - (half ? n - h0 : h0);
+    const int i = l % prm.n0, j = l / prm.n0, cs = prm.cs;
+    const long long ks = half ? -(long long)prm.ks : (long long)prm.ks;
+    float *xl = prm.x + (size_t)j * prm.js + (size_t)i * prm.is + (half ? (long long)(n - 1) * (long long)prm.ks : 0) -
+                (long long)pad * ks;
+    const float4 *fac = prm.fac + ((size_t)half * rows * nl + l) * FP;
+    const long long fs = (long long)nl * FP;
+    // the next row's record into a slot (past the last row only the group is counted)
+    const float4 *pf = fac;
+    const float *px = xl;
+    int left = rows;
+    auto issue = [&](int slot) {
+        if (left > 0) {
+#pragma unroll
+            for (int h = 0; h < FP; ++h) cp_async16(rf + (slot * FP + h) * T, pf + h);
+            if (left <= rows - pad) {
+                if constexpr (IL) {
+                    cp_async8(rx + slot * T, px);
+                } else {
+                    cp_async4(&rx[slot * T].x, px);
+                    cp_async4(&rx[slot * T].y, px + cs);
+                }
+            } else {
+                rx[slot * T] = make_float2(0.f, 0.f);   // identity row
+            }
+            pf += fs;
+            px += ks;
+            --left;
+        }
+        cp_async_commit();
+    };
+    auto record = [&](int slot, float2 (&f)[2 * FP]) {
+#pragma unroll
+        for (int h = 0; h < FP; ++h) {
+            const float4 v = rf[(slot * FP + h) * T];
+            f[2 * h] = make_float2(v.x, v.y);
+            f[2 * h + 1] = make_float2(v.z, v.w);
+        }
+    };
+    // forward: t holds what the last P rows subtract from the next ones
+    float2 t[P], fl[P][2 * FP], yl[P];   // and the last P rows' records and results
+#pragma unroll
+    for (int d = 0; d < P; ++d) t[d] = make_float2(0.f, 0.f);
+#pragma unroll
+    for (int u = 0; u < D; ++u) issue(u);
+    for (int k0 = 0, s0 = 0; k0 < rows; k0 += P, s0 = s0 + P == D ? 0 : s0 + P) {
+#pragma unroll
+        for (int r = 0; r < P; ++r) {
+            cp_async_wait<D - 1>();
+            record(s0 + r, fl[r]);
+            const float2 y = csubf(rx[(s0 + r) * T], t[r]);
+            issue(s0 + r);
+            yl[r] = y;
+            sy[(size_t)(k0 + r) * T] = y;
+            const float2 ny = make_float2(-y.x, -y.y);
+#pragma unroll
+            for (int d = 1; d < P; ++d) csubmul(t[(r + d) % P], fl[r][d], ny);
+            t[r] = cmulf(fl[r][P], y);
+        }
+    }
+    cp_async_wait<0>();
+    // the system at the cut (see k_zsolve), here with unit rows as stored
+    __syncthreads();
+    float2 *ex = reinterpret_cast<float2 *>(zs_smem);   // the ring is free: [e][thread]
+#pragma unroll
+    for (int d = 0; d < P; ++d) {
+        const int o = P - 1 - d;
+#pragma unroll
+        for (int q = 1; q <= P; ++q) ex[(size_t)(d * P + q - 1) * T + threadIdx.x] = fl[o][q];
+        ex[(size_t)(P * P + d) * T + threadIdx.x] = cmulf(fl[o][0], yl[o]);
+    }
+    __syncthreads();
+    float2 T1[P], T2[P];
+    {
+        float2 U1[P][P], W1[P][P], c1[P], U2[P][P], W2[P][P], c2[P];
+        auto tail = [&](int col, float2 (&Um)[P][P], float2 (&W)[P][P], float2 (&c)[P]) {
+#pragma unroll
+            for (int r = 0; r < P; ++r) {
+                const int d = P - 1 - r;
+                auto st = [&](int q) { return ex[(size_t)(d * P + q - 1) * T + col]; };
+#pragma unroll
+                for (int k = 0; k < P; ++k) {
+                    Um[r][k] = k > r ? st(k - r) : make_float2(0.f, 0.f);
+                    W[r][k] = k >= P - 1 - r ? st(2 * P - 1 - r - k) : make_float2(0.f, 0.f);
+                }
+                c[r] = ex[(size_t)(P * P + d) * T + col];
+            }
+        };
+        tail(li, U1, W1, c1);
+        tail(li + kZSubLines, U2, W2, c2);
+        twist_solve<P>(U1, W1, c1, U2, W2, c2, T1, T2);
+    }
+    __syncthreads();   // the ring is in use again from here on
+    // backward: local row rows + c is the partner's tail row P-1-c
+    float2 xw[P];      // x of row k+1 .. k+P, row k+q in slot (k+q) % P; row rows + c in slot c (P divides rows)
+#pragma unroll
+    for (int c = 0; c < P; ++c) xw[c] = half ? T1[P - 1 - c] : T2[P - 1 - c];
+    pf = fac + (size_t)(rows - 1) * fs;
+    left = rows;
+    auto issue_back = [&](int slot) {
+        if (left > 0) {
+#pragma unroll
+            for (int h = 0; h < FP; ++h) cp_async16(rf + (slot * FP + h) * T, pf + h);
+            pf -= fs;
+            --left;
+        }
+        cp_async_commit();
+    };
+#pragma unroll
+    for (int u = 0; u < D; ++u) issue_back(u);
+    float *out = xl + (long long)(rows - 1) * ks;
+    for (int k0 = rows - P, s0 = 0; k0 >= 0; k0 -= P, s0 = s0 + P == D ? 0 : s0 + P) {
+#pragma unroll
+        for (int r = P - 1; r >= 0; --r) {
+            const int slot = s0 + P - 1 - r;
+            cp_async_wait<D - 1>();
+            float2 f[2 * FP];
+            record(slot, f);
+            issue_back(slot);
+            float2 v = cmulf(sy[(size_t)(k0 + r) * T], f[0]);
+#pragma unroll
+            for (int q = P; q >= 1; --q) csubmul(v, f[q], xw[(r + q) % P]);
+            xw[r] = v;
+            if (valid && k0 + r >= pad) {
+                if constexpr (IL) {
+                    *reinterpret_cast<float2 *>(out) = v;
+                } else {
+                    out[0] = v.x;
+                    out[cs] = v.y;
+                }
+            }
+            out -= ks;
+        }
+    }
+    cp_async_wait<0>();
+}
+
+// fresh: the stored factor is not the current stage's
+template <int P, bool CI> void launch_zsolve_t(const ZSolveParams &zp, bool fresh, cudaStream_t st) {
     constexpr size_t kMax = 220 * 1024;
     // the dynamic shared-memory limit is a property of the kernel, not of a
     // launch: set it once to the largest size any line length may use, so
@@ -635,22 +887,37 @@ template <int P, bool CI> void launch_zsolve_t(const ZSolveParams &zp, cudaStrea
     // lower it under each other's launches
     static const bool attr = [] {
         TDZ_CUDA(cudaFuncSetAttribute(k_zsolve<P, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
+        TDZ_CUDA(cudaFuncSetAttribute(k_zsub<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
+        TDZ_CUDA(cudaFuncSetAttribute(k_zsub<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
         return true;
     }();
     (void)attr;
     const int nl = zp.n0 * zp.n1;
+    if (zp.fac) {
+        const int blocks = (nl + kZSubLines - 1) / kZSubLines;
+        if (fresh) {
+            const int entries = 2 * z_blocks(zp.n2, ZBlk<P>::B) * ZBlk<P>::B * (P + 1);
+            k_zbands<P><<<(entries + 127) / 128, 128, 0, st>>>(zp);
+            k_zfac<P, CI><<<blocks, 2 * kZSubLines, 0, st>>>(zp);
+            count_launch(2);
+        }
+        (zp.cs == 1 ? k_zsub<P, true> : k_zsub<P, false>)<<<blocks, 2 * kZSubLines, zsub_smem<P>(zp.n2), st>>>(zp);
+        count_launch();
+        return;
+    }
     const size_t smem = zsolve_smem<P>(zp.n2);
     TDZ_CHECK(smem <= kMax, TDZ_ERR_UNSUPPORTED, "outer axis too long for the FDM line solve");
     const int entries = 2 * z_blocks(zp.n2, ZBlk<P>::B) * ZBlk<P>::B * (P + 1);
     k_zbands<P><<<(entries + 127) / 128, 128, 0, st>>>(zp);
     k_zsolve<P, CI><<<(nl + kZLines - 1) / kZLines, 2 * kZLines, smem, st>>>(zp);
+    count_launch(2);
 }
 
 // complex eigenvalues (complex axis pencils) take the variant with the
 // imaginary part of the line shift
-template <int P> void launch_zsolve(const ZSolveParams &zp, cudaStream_t st) {
-    if (zp.lxi) launch_zsolve_t<P, true>(zp, st);
-    else launch_zsolve_t<P, false>(zp, st);
+template <int P> void launch_zsolve(const ZSolveParams &zp, bool fresh, cudaStream_t st) {
+    if (zp.lxi) launch_zsolve_t<P, true>(zp, fresh, st);
+    else launch_zsolve_t<P, false>(zp, fresh, st);
 }
 
 // scratch of the line solves: saved states (float2 entries) and band rows (float4 entries)
@@ -663,6 +930,22 @@ size_t zsolve_state_size(int P, int n2, size_t lines) {
     case 3: return state_entries<3>(n2, lines);
     case 4: return state_entries<4>(n2, lines);
     default: return state_entries<5>(n2, lines);
+    }
+}
+// stored factor (float4 entries), 0 where it is not used: beyond 64 MB it would
+// not stay in L2, and streaming it (88 bytes per coefficient and application
+// at P = 3) costs more than redoing the elimination (97 us against about 120
+// on 163 x 163 lines of 343 rows)
+template <int P> size_t factor_entries(int n2, size_t lines) {
+    const size_t e = (size_t)2 * z_blocks(n2, ZBlk<P>::B) * ZBlk<P>::B * ZFac<P>::FP * lines;
+    return e * sizeof(float4) <= ((size_t)64 << 20) && zsub_smem<P>(n2) <= 220 * 1024 ? e : 0;
+}
+size_t zsolve_factor_size(int P, int n2, size_t lines) {
+    switch (P) {
+    case 2: return factor_entries<2>(n2, lines);
+    case 3: return factor_entries<3>(n2, lines);
+    case 4: return factor_entries<4>(n2, lines);
+    default: return factor_entries<5>(n2, lines);
     }
 }
 size_t zsolve_band_size(int P, int n2) {
@@ -814,6 +1097,8 @@ void PcFDM::setup(Operator *op_, int prec) {
     }
     ufac.alloc(zsolve_state_size(P, n[dim - 1], N / n[dim - 1]) * sizeof(float2));
     zb.alloc(zsolve_band_size(P, n[dim - 1]) * sizeof(float4));
+    zfac.alloc(zsolve_factor_size(P, n[dim - 1], N / n[dim - 1]) * sizeof(float4));
+    zfac_valid = false;
     if (tensor) {
         npart.alloc((size_t)16 * sm_count() * sizeof(double));
         ldx = (n[0] + 3) / 4 * 4;
@@ -1026,15 +1311,42 @@ void line_solve64(const PcFDM &f, double2 *x, cudaStream_t st) {
     count_launch();
 }
 
-void line_solve(int P, const ZSolveParams &zp, cudaStream_t st) {
-    switch (P) {
-    case 2: launch_zsolve<2>(zp, st); break;
-    case 3: launch_zsolve<3>(zp, st); break;
-    case 4: launch_zsolve<4>(zp, st); break;
-    case 5: launch_zsolve<5>(zp, st); break;
+// The stored factor is kept while the stage coefficients of the line matrices
+// stay the same values. A captured call must stand on its own at every replay
+// and must not overwrite it: it takes the kernel without a stored factor.
+void line_solve(PcFDM &f, ZSolveParams &zp, cudaStream_t st) {
+    bool fresh = false;
+    if (f.zfac.ptr) {
+        cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+        const bool plain = cudaStreamIsCapturing(st, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+        if (!plain) {
+            cudaGetLastError();
+        } else {
+            zp.fac = f.zfac.as<float4>();
+            auto key = [](const CombP<float> &c, std::vector<float> &out) {
+                out.push_back((float)c.n);
+                for (int i = 0; i < c.n; ++i) {
+                    out.push_back((float)c.base[i]);
+                    out.push_back(c.re[i]);
+                    out.push_back(c.im[i]);
+                }
+            };
+            std::vector<float> now;
+            key(zp.Bc, now);
+            key(zp.Cc, now);
+            fresh = !f.zfac_valid || now != f.zfac_key;
+            if (fresh) f.zfac_valid = false;   // until its launches have gone out
+            f.zfac_key = std::move(now);
+        }
+    }
+    switch (f.P) {
+    case 2: launch_zsolve<2>(zp, fresh, st); break;
+    case 3: launch_zsolve<3>(zp, fresh, st); break;
+    case 4: launch_zsolve<4>(zp, fresh, st); break;
+    case 5: launch_zsolve<5>(zp, fresh, st); break;
     }
     TDZ_CUDA(cudaGetLastError());
-    count_launch(2);
+    if (zp.fac) f.zfac_valid = true;
 }
 
 }  // namespace
@@ -1068,7 +1380,7 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
         zp.js = 2 * ldx;
         zp.is = 1;
         zp.cs = ldx;
-        line_solve(P, zp, st);
+        line_solve(*this, zp, st);
         transform(Ti[0], a, n[2], n[1], ldx, b, ldy, st);
         int parts = blocks;
         if (transform_natural(Ti[1])) {
@@ -1146,7 +1458,7 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
     zp.js = 2 * n[0];
     zp.is = 2;
     zp.cs = 1;
-    line_solve(P, zp, st);
+    line_solve(*this, zp, st);
     // inverse transforms: along y with V, along x with V^T
     if (dim == 3) {
         along_y(V[1], cur, oth);
@@ -1155,7 +1467,6 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
     along_x(VT[0], cur, oth);
     TDZ_CUDA(cudaGetLastError());
     count_launch(dim == 3 ? 4 : 2);
-    blas::cast(oth, TDZ_FP32, z, TDZ_FP64, N, st);
     ++applies;
 }
 

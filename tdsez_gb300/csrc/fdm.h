@@ -41,6 +41,9 @@ struct PcFDM : Precond {
     // dropped, or the dropped terms' stage scalars are zero now
     bool exact_now() const;
     DevBuf zb;                 // FP32 upper band rows (Bc, Cc) of the line matrices in elimination order
+    DevBuf zfac;               // stored line factor of small problems (empty: eliminated in every application)
+    std::vector<float> zfac_key;   // the coefficients it was computed for
+    bool zfac_valid = false;
     DevBuf b1, b2, ufac;       // FP32 work vectors and the saved elimination states of the line solves
     bool exact = true;         // false: inner one-axis terms were dropped (stiffness-only pencil, or a
                                // field along an inner axis)
