@@ -131,18 +131,31 @@ template <> __device__ __forceinline__ double2 gzero<double2>() { return make_do
 // (16 TT)^2 tile, TT x TT outputs per thread. The next K chunk is requested
 // into registers before the current one is used and shared memory is double
 // buffered, so a chunk costs one barrier and its load latency overlaps the
-// products. TT = 2 where TT = 4 would leave SMs idle: a 260 x 260 x 260
-// complex transform (the 2D runs) has 25 tiles of 64 x 64 and 81 of 32 x 32
-// (79 us before, one buffer and 25 tiles; 21 us now).
+// products. TT = 2 where TT = 4 would leave SMs idle, in FP32 with KS = 2 groups
+// of 256 threads that take every other K chunk and add up at the end. MA and MC
+// are the types in memory: the first and the last transform of an FP32
+// application read and write the FP64 vectors themselves. A 260 x 260 x 260
+// complex transform (the 2D runs) has 25 tiles of 64 x 64 and 81 of 32 x 32: 79
+// us with one buffer and 25 tiles, 21 us with 81 and 3 us for the cast beside
+// it; with two groups 24 us from FP64 and 15 us to FP64, no cast.
 // K chunk: half as long for the FP64 64 x 64 tiles, whose buffers would pass 48 KB
 template <class C2, int TT> constexpr int kGemmK = sizeof(C2) == 16 && TT == 4 ? 8 : 16;
-template <class TA, class TB, class C2, int TT>
-__global__ void __launch_bounds__(256) k_gemm(const TA *__restrict__ A, const TB *__restrict__ B, C2 *__restrict__ Cm,
-                                              int M, int N, int K, size_t bplane, size_t cplane) {
+template <class D, class S> __device__ __forceinline__ D gconv(const S &v) { return v; }
+template <> __device__ __forceinline__ float2 gconv<float2, double2>(const double2 &v) {
+    const dff x = dff_split(v.x), y = dff_split(v.y);
+    return make_float2(__fadd_rn(x.hi, x.lo), __fadd_rn(y.hi, y.lo));
+}
+template <> __device__ __forceinline__ double2 gconv<double2, float2>(const float2 &v) {
+    return make_double2(f2d_exact(v.x), f2d_exact(v.y));
+}
+template <class MA, class TA, class TB, class C2, class MC, int TT, int KS>
+__global__ void __launch_bounds__(256 * KS) k_gemm(const MA *__restrict__ A, const TB *__restrict__ B,
+                                                   MC *__restrict__ Cm, int M, int N, int K, size_t bplane,
+                                                   size_t cplane) {
     constexpr int BT = 16 * TT, BK = kGemmK<C2, TT>, L = BT * BK / 256;
-    __shared__ TA As[2][BK][BT + 1];
-    __shared__ TB Bs[2][BK][BT + 1];
-    const int tid = threadIdx.x, tx = tid % 16, ty = tid / 16;
+    __shared__ TA As[KS][2][BK][BT + 1];
+    __shared__ TB Bs[KS][2][BK][BT + 1];
+    const int tid = threadIdx.x % 256, grp = threadIdx.x / 256, tx = tid % 16, ty = tid / 16;
     const int m0 = blockIdx.y * BT, n0 = blockIdx.x * BT;
     B += blockIdx.z * bplane;
     Cm += blockIdx.z * cplane;
@@ -158,7 +171,7 @@ __global__ void __launch_bounds__(256) k_gemm(const TA *__restrict__ A, const TB
         for (int q = 0; q < L; ++q) {
             const int i = tid + 256 * q;
             const int gm = m0 + i / BK, ka = k0 + i % BK, kb = k0 + i / BT, gn = n0 + i % BT;
-            pa[q] = gm < M && ka < K ? A[(size_t)gm * K + ka] : gzero<TA>();
+            pa[q] = gm < M && ka < K ? gconv<TA, MA>(A[(size_t)gm * K + ka]) : gzero<TA>();
             pb[q] = kb < K && gn < N ? B[(size_t)kb * N + gn] : gzero<TB>();
         }
     };
@@ -166,25 +179,25 @@ __global__ void __launch_bounds__(256) k_gemm(const TA *__restrict__ A, const TB
 #pragma unroll
         for (int q = 0; q < L; ++q) {
             const int i = tid + 256 * q;
-            As[s][i % BK][i / BK] = pa[q];
-            Bs[s][i / BT][i % BT] = pb[q];
+            As[grp][s][i % BK][i / BK] = pa[q];
+            Bs[grp][s][i / BT][i % BT] = pb[q];
         }
     };
-    fetch(0);
+    fetch(grp * BK);
     put(0);
     __syncthreads();
     int s = 0;
-    for (int k0 = 0; k0 < K; k0 += BK, s ^= 1) {
-        const bool more = k0 + BK < K;
-        if (more) fetch(k0 + BK);
+    for (int k0 = 0; k0 < K; k0 += KS * BK, s ^= 1) {   // chunk k0 + grp BK of each group
+        const bool more = k0 + KS * BK < K;
+        if (more) fetch(k0 + (KS + grp) * BK);
 #pragma unroll
         for (int k = 0; k < BK; ++k) {
             TA a[TT];
             TB b[TT];
 #pragma unroll
-            for (int r = 0; r < TT; ++r) a[r] = As[s][k][ty * TT + r];
+            for (int r = 0; r < TT; ++r) a[r] = As[grp][s][k][ty * TT + r];
 #pragma unroll
-            for (int c = 0; c < TT; ++c) b[c] = Bs[s][k][tx + 16 * c];
+            for (int c = 0; c < TT; ++c) b[c] = Bs[grp][s][k][tx + 16 * c];
 #pragma unroll
             for (int r = 0; r < TT; ++r)
 #pragma unroll
@@ -193,34 +206,55 @@ __global__ void __launch_bounds__(256) k_gemm(const TA *__restrict__ A, const TB
         if (more) put(s ^ 1);   // last read before the previous barrier
         __syncthreads();
     }
+    if constexpr (KS == 2) {
+        __shared__ C2 part[TT * TT][256];
+        if (grp == 1)
+#pragma unroll
+            for (int r = 0; r < TT; ++r)
+#pragma unroll
+                for (int c = 0; c < TT; ++c) part[r * TT + c][tid] = acc[r][c];
+        __syncthreads();
+        if (grp == 1) return;
+#pragma unroll
+        for (int r = 0; r < TT; ++r)
+#pragma unroll
+            for (int c = 0; c < TT; ++c) {
+                const C2 v = part[r * TT + c][tid];
+                acc[r][c].x += v.x;
+                acc[r][c].y += v.y;
+            }
+    }
 #pragma unroll
     for (int r = 0; r < TT; ++r)
 #pragma unroll
         for (int c = 0; c < TT; ++c) {
             const int gm = m0 + ty * TT + r, gn = n0 + tx + 16 * c;
-            if (gm < M && gn < N) Cm[(size_t)gm * N + gn] = acc[r][c];
+            if (gm < M && gn < N) Cm[(size_t)gm * N + gn] = gconv<MC, C2>(acc[r][c]);
         }
 }
 
-template <class TA, class TB, class C2>
-void gemm(const TA *A, const TB *B, C2 *Cm, int M, int N, int K, int planes, size_t bplane, size_t cplane,
+template <class MA, class TA, class TB, class C2, class MC>
+void gemm(const MA *A, const TB *B, MC *Cm, int M, int N, int K, int planes, size_t bplane, size_t cplane,
           cudaStream_t st) {
+    constexpr int KS = sizeof(C2) == 8 ? 2 : 1;
     const long long big = (long long)((M + 63) / 64) * ((N + 63) / 64) * planes;
     if (big >= 2LL * sm_count())
-        k_gemm<TA, TB, C2, 4><<<dim3((N + 63) / 64, (M + 63) / 64, planes), 256, 0, st>>>(A, B, Cm, M, N, K, bplane, cplane);
+        k_gemm<MA, TA, TB, C2, MC, 4, 1>
+            <<<dim3((N + 63) / 64, (M + 63) / 64, planes), 256, 0, st>>>(A, B, Cm, M, N, K, bplane, cplane);
     else
-        k_gemm<TA, TB, C2, 2><<<dim3((N + 31) / 32, (M + 31) / 32, planes), 256, 0, st>>>(A, B, Cm, M, N, K, bplane, cplane);
+        k_gemm<MA, TA, TB, C2, MC, 2, KS>
+            <<<dim3((N + 31) / 32, (M + 31) / 32, planes), 256 * KS, 0, st>>>(A, B, Cm, M, N, K, bplane, cplane);
 }
 // along x: rows of n0 entries times an n0 x n0 matrix
-template <class TM, class C2>
-void gemm_x(const DevBuf &Mx, const C2 *in, C2 *out, int rows, int n0, cudaStream_t st) {
-    gemm<C2, TM, C2>(in, Mx.as<TM>(), out, rows, n0, n0, 1, 0, 0, st);
+template <class TM, class C2, class MI, class MO>
+void gemm_x(const DevBuf &Mx, const MI *in, MO *out, int rows, int n0, cudaStream_t st) {
+    gemm<MI, C2, TM, C2, MO>(in, Mx.as<TM>(), out, rows, n0, n0, 1, 0, 0, st);
 }
 // along y: an n1 x n1 matrix times every n1 x n0 plane
 template <class TM, class C2>
 void gemm_y(const DevBuf &My, const C2 *in, C2 *out, int n0, int n1, int planes, cudaStream_t st) {
     const size_t plane = (size_t)n0 * n1;
-    gemm<TM, C2, C2>(My.as<TM>(), in, out, n1, n0, n1, planes, plane, plane, st);
+    gemm<TM, TM, C2, C2, C2>(My.as<TM>(), in, out, n1, n0, n1, planes, plane, plane, st);
 }
 
 __device__ __forceinline__ float2 cmulf(float2 a, float2 b) {
@@ -1405,8 +1439,8 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
         // FP64 preconditioner (SIMT transforms, FP64 line solves)
         double2 *y1 = b1.as<double2>(), *y2 = b2.as<double2>();
         auto x64 = [&](const DevBuf &Mx, const double2 *in, double2 *out) {
-            if (cplx) gemm_x<double2>(Mx, in, out, grows, n[0], st);
-            else gemm_x<double>(Mx, in, out, grows, n[0], st);
+            if (cplx) gemm_x<double2, double2>(Mx, in, out, grows, n[0], st);
+            else gemm_x<double, double2>(Mx, in, out, grows, n[0], st);
         };
         auto y64 = [&](const DevBuf &My, const double2 *in, double2 *out) {
             if (cplx) gemm_y<double2>(My, in, out, n[0], n[1], n[2], st);
@@ -1431,19 +1465,18 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
         return;
     }
     float2 *x1 = b1.as<float2>(), *x2 = b2.as<float2>();
-    blas::cast(r, TDZ_FP64, x1, TDZ_FP32, N, st);
     // transforms along x (rows of n0) and along y (planes of n1 x n0) with a
     // real or complex FP32 matrix
-    auto along_x = [&](const DevBuf &Mx, const float2 *in, float2 *out) {
-        if (cplx) gemm_x<float2>(Mx, in, out, grows, n[0], st);
-        else gemm_x<float>(Mx, in, out, grows, n[0], st);
+    auto along_x = [&](const DevBuf &Mx, const auto *in, auto *out) {
+        if (cplx) gemm_x<float2, float2>(Mx, in, out, grows, n[0], st);
+        else gemm_x<float, float2>(Mx, in, out, grows, n[0], st);
     };
     auto along_y = [&](const DevBuf &My, const float2 *in, float2 *out) {
         if (cplx) gemm_y<float2>(My, in, out, n[0], n[1], n[2], st);
         else gemm_y<float>(My, in, out, n[0], n[1], n[2], st);
     };
     // forward transforms: along x with V (t_i = sum_i' V[i'][i] r_i'), along y with V^T
-    along_x(V[0], x1, x2);
+    along_x(V[0], r, x2);   // FP64 in
     float2 *cur = x2, *oth = x1;
     if (dim == 3) {
         along_y(VT[1], x2, x1);
@@ -1464,7 +1497,7 @@ void PcFDM::apply(const double2 *r, double2 *z, cudaStream_t st) {
         along_y(V[1], cur, oth);
         std::swap(cur, oth);
     }
-    along_x(VT[0], cur, oth);
+    along_x(VT[0], cur, z);   // FP64 out
     TDZ_CUDA(cudaGetLastError());
     count_launch(dim == 3 ? 4 : 2);
     ++applies;
