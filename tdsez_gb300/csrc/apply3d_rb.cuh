@@ -49,7 +49,7 @@ template <class MC> struct IsF64Mem { static constexpr bool v = std::is_same<MC,
 // FP64 -> FP32 keeping the leading 24 significand bits (truncation, relative
 // error below 2^-23) with integer operations; |v| < 2^-100 gives 0, values
 // beyond the FP32 range a non-finite result
-__device__ __forceinline__ float d2f_trunc(double v) {   // the high part of dff_split
+__device__ __forceinline__ float d2f_trunc(double v) {   // dff_split without the rounding
     const unsigned int h32 = (unsigned int)__double2hiint(v), l32 = (unsigned int)__double2loint(v);
     const unsigned int sign = h32 & 0x80000000u;
     const unsigned int hb = ((__funnelshift_l(l32, h32, 3) ^ 0x40000000u) & 0x7FFFFFFFu) | sign;
@@ -295,7 +295,7 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
         const int buf = it & 1;
         C uM[XR], uT[XR], uS[XR];
 #pragma unroll
-        for (int k = 0; k < XR; ++k) { uM[k] = czero<C>(); uT[k] = czero<C>(); uS[k] = czero<C>(); }
+        for (int k = 0; k < XR; ++k) { uM[k] = czero<C>(); uT[k] = czero<C>(); uS[k] = czero<C>(); }   // past the tile
 #pragma unroll
         for (int j = 0; j < BW; ++j) {
 #pragma unroll
@@ -303,6 +303,12 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
                 const int q = ty + k * NTY;
                 if (k == XR - 1 && q >= RY) break;
                 const C v = in[q * RX + tx + j];
+                if (j == 0) {
+                    rset(uM[k], xm[j], v);
+                    if constexpr (HB) cset(uT[k], xt[j], v);
+                    if constexpr (HC) rset(uS[k], xs[j], v);
+                    continue;
+                }
                 rfma(uM[k], xm[j], v);
                 if constexpr (HB) cfma(uT[k], xt[j], v);
                 if constexpr (HC) rfma(uS[k], xs[j], v);
@@ -318,17 +324,15 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
         }
     };
     // y and z stages of plane it; output plane zs + it - P + o of row r
-    // accumulates in acc[r][(ring + o) % BW]
+    // accumulates in acc[r][o], which the plane loop shifts
     C acc[R][BW];
 #pragma unroll
     for (int r = 0; r < R; ++r)
 #pragma unroll
         for (int s = 0; s < BW; ++s) acc[r][s] = czero<C>();
-    auto yzstage = [&](int it, int ring) {
+    auto yzstage = [&](int it) {
         const int buf = it & 1;
         C wA[R], wB[R], wC[R];
-#pragma unroll
-        for (int r = 0; r < R; ++r) { wA[r] = czero<C>(); wB[r] = czero<C>(); wC[r] = czero<C>(); }
 #pragma unroll
         for (int qq = 0; qq < R + 2 * P; ++qq) {
             const int q = ty * R + qq;
@@ -344,16 +348,19 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
                 T ym;
                 if constexpr (Sh::kYReg) ym = ymr[r][j];
                 else ym = sYm[j][row];
-                rfma(wA[r], ym, um);
+                if (j == 0) rset(wA[r], ym, um);
+                else rfma(wA[r], ym, um);
                 if constexpr (HB) {
-                    rfma(wB[r], ym, ut);
+                    if (j == 0) rset(wB[r], ym, ut);
+                    else rfma(wB[r], ym, ut);
                     cfma(wB[r], sYt[j][row], um);
                 }
                 if constexpr (HC) {
                     T ysv;
                     if constexpr (Sh::kYReg) ysv = ysr[r][j];
                     else ysv = sYs[j][row];
-                    rfma(wC[r], ym, us);
+                    if (j == 0) rset(wC[r], ym, us);
+                    else rfma(wC[r], ym, us);
                     rfma(wC[r], ysv, um);
                 }
             }
@@ -374,10 +381,16 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
             if constexpr (HB) zm = sZM[(size_t)it * BW + o];
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-                C &a = acc[r][(ring + o) % BW];
-                if constexpr (KA == 1) rfma(a, cre(za), wA[r]);
-                else if constexpr (KA == 2) ifma(a, cim(za), wA[r]);
-                else cfma(a, za, wA[r]);
+                C &a = acc[r][o];
+                if (o == 2 * P) {   // the output plane's first input plane
+                    if constexpr (KA == 1) rset(a, cre(za), wA[r]);
+                    else if constexpr (KA == 2) iset(a, cim(za), wA[r]);
+                    else cset(a, za, wA[r]);
+                } else {
+                    if constexpr (KA == 1) rfma(a, cre(za), wA[r]);
+                    else if constexpr (KA == 2) ifma(a, cim(za), wA[r]);
+                    else cfma(a, za, wA[r]);
+                }
                 if constexpr (HB) rfma(a, zm, wB[r]);
                 if constexpr (HC) {
                     if constexpr (KC == 1) rfma(a, cre(zc), wC[r]);
@@ -387,12 +400,12 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
             }
         }
     };
-    auto step = [&](int it, int ring) {
+    auto step = [&](int it) {
         arrive(it + 1);
         __syncthreads();
         issue(it + 3);
         if (it + 1 < hi) xstage(it + 1);
-        yzstage(it, ring);
+        yzstage(it);
     };
     // prologue: planes lo, lo+1, lo+2 requested, plane lo staged and contracted along x
     if (lo < hi) {
@@ -418,12 +431,8 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
             }
         }
     };
-    auto finish = [&](int it, int slot, const MC (&sv)[R]) {
-        if (it < 2 * P) {   // a halo output plane of the run: not stored, its slot is reused
-#pragma unroll
-            for (int r = 0; r < R; ++r) acc[r][slot] = czero<C>();
-            return;
-        }
+    auto finish = [&](int it, const MC (&sv)[R]) {
+        if (it < 2 * P) return;   // a halo output plane of the run: not stored
         const int m = zs + it - P;
 #pragma unroll
         for (int r = 0; r < R; ++r) {
@@ -435,13 +444,13 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
                     if constexpr (std::is_same<T, float>::value && IsF64Mem<MC>::v) {
                         // FP32 arithmetic on FP64 vectors: b - A x formed in FP64 (exact
                         // operands, one rounding), so the stored residual keeps b's bits
-                        const double2 o = rb_store<MC, C>(acc[r][slot]);
+                        const double2 o = rb_store<MC, C>(acc[r][0]);
                         v = make_double2(sv[r].x - o.x, sv[r].y - o.y);
                     } else {
-                        v = rb_store<MC, C>(rb_sub<C, MC>(sv[r], acc[r][slot]));
+                        v = rb_store<MC, C>(rb_sub<C, MC>(sv[r], acc[r][0]));
                     }
                 } else {
-                    v = rb_store<MC, C>(acc[r][slot]);
+                    v = rb_store<MC, C>(acc[r][0]);
                 }
                 Y[e] = v;
                 if (prm.red_mode) {
@@ -449,7 +458,7 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
                         if (!prm.sub) {
                             // FP32 arithmetic: the run's partial sum in FP32 (its own error is
                             // below the apply's), off GB300's FP64 pipe
-                            const float2 a = acc[r][slot];
+                            const float2 a = acc[r][0];
                             if (prm.red_mode == 1) {
                                 facc.x = fmaf(a.x, a.x, fmaf(a.y, a.y, facc.x));
                             } else {
@@ -457,7 +466,6 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
                                 facc.x = fmaf(d.x, a.x, fmaf(d.y, a.y, facc.x));
                                 facc.y = fmaf(d.x, a.y, fmaf(-d.y, a.x, facc.y));
                             }
-                            acc[r][slot] = czero<C>();
                             continue;
                         }
                     }
@@ -470,7 +478,6 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
                     }
                 }
             }
-            acc[r][slot] = czero<C>();
         }
     };
 
@@ -484,8 +491,8 @@ __device__ __noinline__ double2 rb_run(const ApplyParams<T> &prm, const CUtensor
     for (int it = 0; it < nplanes; ++it) {
         MC sv[R];
         side_load(it, sv);
-        if (it >= lo && it < hi) step(it, 0);
-        finish(it, 0, sv);
+        if (it >= lo && it < hi) step(it);
+        finish(it, sv);
 #pragma unroll
         for (int r = 0; r < R; ++r) {
 #pragma unroll

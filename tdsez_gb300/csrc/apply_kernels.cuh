@@ -385,13 +385,19 @@ template <class T, int P, bool HB, bool HC> struct Shape2D {
 
 // sum_j a_j v_j, the a_j complex or all imaginary (the uniform branch outside the loop)
 template <int BW, class C> __device__ __forceinline__ C dot_kind(const C (&a)[BW], const C *v, int stride, int kind) {
-    C s = czero<C>();
+    C s;
     if (kind == 2) {
 #pragma unroll
-        for (int j = 0; j < BW; ++j) ifma(s, cim(a[j]), v[j * stride]);
+        for (int j = 0; j < BW; ++j) {
+            if (j == 0) iset(s, cim(a[j]), v[j * stride]);
+            else ifma(s, cim(a[j]), v[j * stride]);
+        }
     } else {
 #pragma unroll
-        for (int j = 0; j < BW; ++j) cfma(s, a[j], v[j * stride]);
+        for (int j = 0; j < BW; ++j) {
+            if (j == 0) cset(s, a[j], v[j * stride]);
+            else cfma(s, a[j], v[j * stride]);
+        }
     }
     return s;
 }
@@ -441,12 +447,18 @@ __global__ void __launch_bounds__(kTX2 *kTY2) k_apply2d(const __grid_constant__ 
             const C *v = sIn + r * RX + tx;
             C uM = czero<C>();
 #pragma unroll
-            for (int j = 0; j < BW; ++j) rfma(uM, xm[j], v[j]);
+            for (int j = 0; j < BW; ++j) {
+                if (j == 0) rset(uM, xm[j], v[j]);
+                else rfma(uM, xm[j], v[j]);
+            }
             sU[r * kTX2 + tx] = cnorm(uM);
             if constexpr (HC) {
                 C uS = czero<C>();
 #pragma unroll
-                for (int j = 0; j < BW; ++j) rfma(uS, xs[j], v[j]);
+                for (int j = 0; j < BW; ++j) {
+                    if (j == 0) rset(uS, xs[j], v[j]);
+                    else rfma(uS, xs[j], v[j]);
+                }
                 sU[(US * RY + r) * kTX2 + tx] = cnorm(uS);
             }
             if constexpr (HB) sU[(UT * RY + r) * kTX2 + tx] = cnorm(dot_kind<BW, C>(xt, v, 1, prm.xt_kind));
@@ -458,7 +470,8 @@ __global__ void __launch_bounds__(kTX2 *kTY2) k_apply2d(const __grid_constant__ 
     const C *u = sU + ty * kTX2 + tx;
 #pragma unroll
     for (int j = 0; j < BW; ++j) {
-        kfma(out, sZA[ty * BW + j], u[j * kTX2], prm.za_kind);
+        if (j == 0) kset(out, sZA[ty * BW + j], u[j * kTX2], prm.za_kind);
+        else kfma(out, sZA[ty * BW + j], u[j * kTX2], prm.za_kind);
         if constexpr (HB) rfma(out, sZM[ty * BW + j], u[(UT * RY + j) * kTX2]);
         if constexpr (HC) kfma(out, sZC[ty * BW + j], u[(US * RY + j) * kTX2], prm.zc_kind);
     }
