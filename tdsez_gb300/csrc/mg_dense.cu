@@ -12,8 +12,8 @@
 // spends its time on:
 //   k_dense_xy   u = (R_x + R_y) d, one z plane per CTA
 //   k_dense_z    z -= alpha d + g (R_z d + C_z u); d = a z + b d; x += d,
-//                16 columns per CTA, their whole length in shared memory, the
-//                matrices streamed through it 16 rows at a time
+//                a few columns per CTA, their whole length in shared memory,
+//                and the matrices streamed through it
 // Products are packed FP32 on both components; the z matrices are stored as
 // equal pairs, so a coefficient needs no move to become an operand. Used for
 // 3D FP32 levels whose estimated step is shorter (dense_pays) and whose stage
@@ -22,7 +22,7 @@
 //
 // 51 x 51 x 109 level, degree 3: a step of 4 launches and 56 us becomes 2
 // launches and 51 us (20 and 31, with cold caches); on the small levels
-// the launches count, 40 us and more against 24 (27 x 27 x 64) and 17 (15 x 15 x 39).
+// the launches count, 40 us and more against 19 (27 x 27 x 64) and 14 (15 x 15 x 39).
 #include <algorithm>
 #include <cmath>
 
@@ -33,7 +33,7 @@ namespace tdz {
 
 namespace {
 
-constexpr int kZCols = 16, kRows = 8;   // columns per CTA and rows per thread of k_dense_z
+constexpr int kRows = 8;   // rows per thread
 inline int up8(int n) { return (n + 7) / 8 * 8; }
 
 struct CombineParams {
@@ -115,30 +115,33 @@ __global__ void __launch_bounds__(256) k_dense_xy(const float *__restrict__ rx, 
 
 struct DenseStep {
     const float2 *rz, *cz;      // [n2][pz] equal pairs, transposed; cz null: identity
-    int n2, pz;
+    int n2, pz, chunk;
     size_t cols;                // n0 n1
     const float2 *u;
     float2 *z, *d, *x;
     float2 alpha, g, a, b;
 };
 
-constexpr int kZChunk = 16;   // matrix rows per stage of k_dense_z
-
-__global__ void k_dense_z(const DenseStep s) {
+// ZC columns per CTA, KR rows per thread, the matrices in stages of s.chunk
+// rows: 16 columns, 8 rows and stages of 16 where they make enough CTAs, else 8
+// columns, 4 rows and both matrices requested whole at the start, since there a
+// thread's chain of stages and products is all the time (27 x 27 x 64: 15.6 us,
+// now 10.9 us; 15 x 15 x 39: 12.4 and 8.6 us; 9 x 9 x 28: 9.9 and 7.4 us).
+template <int ZC, int KR> __global__ void k_dense_z(const DenseStep s) {
     extern __shared__ __align__(16) unsigned char dz_raw[];
     const int nm = s.cz ? 2 : 1;
-    float2 *sD = reinterpret_cast<float2 *>(dz_raw);   // [n2][16]
-    float2 *sU = sD + (size_t)s.n2 * kZCols;
-    float2 *sM = sU + (size_t)s.n2 * kZCols;           // two stages of [matrix][kZChunk][pz]
-    const size_t c0 = (size_t)blockIdx.x * kZCols;
-    const int nc = (int)min((size_t)kZCols, s.cols - c0);
-    // rows k0 .. k0 + 15 of both matrices into stage (k0 / 16) & 1
+    float2 *sD = reinterpret_cast<float2 *>(dz_raw);   // [n2][ZC]
+    float2 *sU = sD + (size_t)s.n2 * ZC;
+    float2 *sM = sU + (size_t)s.n2 * ZC;           // stages of [matrix][chunk][pz]
+    const size_t c0 = (size_t)blockIdx.x * ZC;
+    const int nc = (int)min((size_t)ZC, s.cols - c0);
+    // rows k0 .. k0 + chunk - 1 of both matrices into stage (k0 / chunk) & 1
     auto issue = [&](int k0) {
-        const int rows = min(kZChunk, s.n2 - k0), per = rows * s.pz / 2;   // 16-byte pieces per matrix
+        const int rows = min(s.chunk, s.n2 - k0), per = rows * s.pz / 2;   // 16-byte pieces per matrix
         for (int e = threadIdx.x; e < nm * per; e += blockDim.x) {
             const int m = e / per, p = e % per;
             const float4 *src = reinterpret_cast<const float4 *>((m ? s.cz : s.rz) + (size_t)k0 * s.pz) + p;
-            float4 *dst = reinterpret_cast<float4 *>(sM + ((size_t)((k0 / kZChunk) & 1) * nm + m) * kZChunk * s.pz) + p;
+            float4 *dst = reinterpret_cast<float4 *>(sM + ((size_t)((k0 / s.chunk) & 1) * nm + m) * s.chunk * s.pz) + p;
             asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
                          "l"(src)
                          : "memory");
@@ -146,38 +149,38 @@ __global__ void k_dense_z(const DenseStep s) {
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     issue(0);
-    for (int e = threadIdx.x; e < s.n2 * kZCols; e += blockDim.x) {
-        const int k = e / kZCols, c = e % kZCols;
+    for (int e = threadIdx.x; e < s.n2 * ZC; e += blockDim.x) {
+        const int k = e / ZC, c = e % ZC;
         const size_t i = (size_t)k * s.cols + c0 + min(c, nc - 1);
         sD[e] = s.d[i];
         sU[e] = s.u[i];
     }
-    const int c = threadIdx.x % kZCols, z0 = (threadIdx.x / kZCols) * kRows;
+    const int c = threadIdx.x % ZC, z0 = (threadIdx.x / ZC) * KR;
     // the vectors of this thread's rows, requested before the products
-    float2 zv[kRows], xv[kRows];
+    float2 zv[KR], xv[KR];
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) {
+    for (int j = 0; j < KR; ++j) {
         const size_t i = (size_t)min(z0 + j, s.n2 - 1) * s.cols + c0 + min(c, nc - 1);
         zv[j] = s.z[i];
         xv[j] = s.x[i];
     }
-    float2 acc[kRows];
+    float2 acc[KR];
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) acc[j] = make_float2(0.f, 0.f);
-    for (int k0 = 0; k0 < s.n2; k0 += kZChunk) {
+    for (int j = 0; j < KR; ++j) acc[j] = make_float2(0.f, 0.f);
+    for (int k0 = 0; k0 < s.n2; k0 += s.chunk) {
         asm volatile("cp.async.wait_group 0;" ::: "memory");
         __syncthreads();   // this stage has arrived; the other one is no longer read
-        if (k0 + kZChunk < s.n2) issue(k0 + kZChunk);
-        const int rows = min(kZChunk, s.n2 - k0);
+        if (k0 + s.chunk < s.n2) issue(k0 + s.chunk);
+        const int rows = min(s.chunk, s.n2 - k0);
         for (int m = 0; m < nm; ++m) {
-            const float2 *mat = sM + ((size_t)((k0 / kZChunk) & 1) * nm + m) * kZChunk * s.pz + z0;
-            const float2 *v = (m ? sU : sD) + (size_t)k0 * kZCols + c;
+            const float2 *mat = sM + ((size_t)((k0 / s.chunk) & 1) * nm + m) * s.chunk * s.pz + z0;
+            const float2 *v = (m ? sU : sD) + (size_t)k0 * ZC + c;
 #pragma unroll 4
             for (int k = 0; k < rows; ++k) {
                 const float4 *q = reinterpret_cast<const float4 *>(mat + (size_t)k * s.pz);
-                const float2 w = v[k * kZCols];
+                const float2 w = v[k * ZC];
 #pragma unroll
-                for (int j = 0; j < kRows / 2; ++j) {
+                for (int j = 0; j < KR / 2; ++j) {
                     const float4 p = q[j];
                     acc[2 * j] = __ffma2_rn(make_float2(p.x, p.y), w, acc[2 * j]);
                     acc[2 * j + 1] = __ffma2_rn(make_float2(p.z, p.w), w, acc[2 * j + 1]);
@@ -187,12 +190,12 @@ __global__ void k_dense_z(const DenseStep s) {
     }
     if (c >= nc) return;
 #pragma unroll
-    for (int j = 0; j < kRows; ++j) {
+    for (int j = 0; j < KR; ++j) {
         const int k = z0 + j;
         if (k >= s.n2) break;
         const size_t i = (size_t)k * s.cols + c0 + c;
-        if (!s.cz) acc[j] = __fadd2_rn(acc[j], sU[k * kZCols + c]);
-        const float2 dv = sD[k * kZCols + c];
+        if (!s.cz) acc[j] = __fadd2_rn(acc[j], sU[k * ZC + c]);
+        const float2 dv = sD[k * ZC + c];
         float2 t = zv[j];   // z - alpha d - g acc
         cfma(t, make_float2(-s.alpha.x, -s.alpha.y), dv);
         cfma(t, make_float2(-s.g.x, -s.g.y), acc[j]);
@@ -210,7 +213,9 @@ size_t xy_smem(int n0, int n1) {
     const size_t pd = (n0 + 1) / 2 * 2, px = n0, py = up8(n1);
     return (size_t)n1 * pd * 8 + (pd * px + 3) / 4 * 16 + (size_t)n1 * py * 4;
 }
-size_t z_smem(int n2) { return (size_t)2 * n2 * kZCols * 8 + (size_t)4 * kZChunk * up8(n2) * 8; }
+size_t z_smem(int n2, int zc, int chunk) {
+    return (size_t)2 * n2 * zc * 8 + (size_t)(chunk == n2 ? 2 : 4) * chunk * up8(n2) * 8;
+}
 
 }  // namespace
 
@@ -222,7 +227,7 @@ size_t z_smem(int n2) { return (size_t)2 * n2 * kZCols * 8 + (size_t)4 * kZChunk
 bool DenseLevel::pays(const int *n, size_t ndof) {
     const double dense = 6.0 + 0.08e-6 * 2.0 * ndof * (n[0] + n[1] + 2 * n[2]);
     const double general = 35.0 + 43e-6 * ndof;
-    return dense < general && xy_smem(n[0], n[1]) <= kDenseSmem && z_smem(n[2]) <= kDenseSmem && n[2] <= 512;
+    return dense < general && xy_smem(n[0], n[1]) <= kDenseSmem && z_smem(n[2], 16, 16) <= kDenseSmem && n[2] <= 512;
 }
 
 void DenseLevel::build(const Operator &op, const int *n_) {
@@ -321,7 +326,8 @@ bool DenseLevel::prepare(const Operator &op, cudaStream_t st) {
 void DenseLevel::step(const Operator &op, void *z, void *d, void *x, void *u, cd a, cd b, cudaStream_t st) const {
     static const bool attr = [] {   // once, to the largest size any level may use
         TDZ_CUDA(cudaFuncSetAttribute(k_dense_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
-        TDZ_CUDA(cudaFuncSetAttribute(k_dense_z, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
+        TDZ_CUDA(cudaFuncSetAttribute(k_dense_z<16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
+        TDZ_CUDA(cudaFuncSetAttribute(k_dense_z<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
         return true;
     }();
     (void)attr;
@@ -342,7 +348,13 @@ void DenseLevel::step(const Operator &op, void *z, void *d, void *x, void *u, cd
     s.g = f2(op.sigma[1]);
     s.a = f2(a);
     s.b = f2(b);
-    k_dense_z<<<(unsigned)((s.cols + kZCols - 1) / kZCols), kZCols * (pz / kRows), z_smem(n[2]), st>>>(s);
+    if (s.cols > (size_t)8 * sm_count() || z_smem(n[2], 8, n[2]) > kDenseSmem) {
+        s.chunk = 16;
+        k_dense_z<16, 8><<<(unsigned)((s.cols + 15) / 16), 16 * (pz / 8), z_smem(n[2], 16, 16), st>>>(s);
+    } else {
+        s.chunk = n[2];
+        k_dense_z<8, 4><<<(unsigned)((s.cols + 7) / 8), 8 * (pz / 4), z_smem(n[2], 8, n[2]), st>>>(s);
+    }
     TDZ_CUDA(cudaGetLastError());
     count_launch(2);
 }
