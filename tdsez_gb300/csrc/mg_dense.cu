@@ -21,8 +21,8 @@
 // general step runs.
 //
 // 51 x 51 x 109 level, degree 3: a step of 4 launches and 56 us becomes 2
-// launches and 51 us (20 and 31, with cold caches); on the small levels
-// the launches count, 40 us and more against 19 (27 x 27 x 64) and 14 (15 x 15 x 39).
+// launches and 33 us; on the small levels the launches count, 40 us and more
+// against 14 (27 x 27 x 64) and 11 (15 x 15 x 39).
 #include <algorithm>
 #include <cmath>
 
@@ -63,7 +63,7 @@ __global__ void k_dense_combine(const CombineSet set) {
 __device__ __forceinline__ float2 pmac(float a, float2 v, float2 acc) { return __ffma2_rn(make_float2(a, a), v, acc); }
 
 // u[y][x] = sum_k Rx[x][k] d[y][k] + sum_k Ry[y][k] d[k][x] of plane blockIdx.x
-__global__ void __launch_bounds__(256) k_dense_xy(const float *__restrict__ rx, const float *__restrict__ ry, int n0,
+__global__ void __launch_bounds__(512) k_dense_xy(const float *__restrict__ rx, const float *__restrict__ ry, int n0,
                                                   int n1, int px, int pd, int py, const float2 *__restrict__ d,
                                                   float2 *__restrict__ u) {
     extern __shared__ __align__(16) unsigned char dx_raw[];
@@ -71,15 +71,15 @@ __global__ void __launch_bounds__(256) k_dense_xy(const float *__restrict__ rx, 
     float *sX = reinterpret_cast<float *>(sP + (size_t)n1 * pd);   // [pd][px]: Rx transposed, zero rows past n0
     float *sY = sX + ((size_t)pd * px + 3) / 4 * 4;              // [n1][py]: Ry transposed (16-byte rows)
     const size_t plane = (size_t)blockIdx.x * n0 * n1;
-    for (int e = threadIdx.x; e < n1 * pd; e += 256) {
-        const int y = e / pd, x = e % pd;
-        sP[e] = x < n0 ? d[plane + (size_t)y * n0 + x] : make_float2(0.f, 0.f);
-    }
-    for (int e = threadIdx.x; e < pd * px; e += 256) sX[e] = e / px < n0 ? rx[e] : 0.f;
-    for (int e = threadIdx.x; e < n1 * py; e += 256) sY[e] = ry[e];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, nw = blockDim.x >> 5, nt = blockDim.x;
+    for (int y = warp; y < n1; y += nw)   // a row per warp: no division
+        for (int x = lane; x < pd; x += 32)
+            sP[y * pd + x] = x < n0 ? d[plane + (size_t)y * n0 + x] : make_float2(0.f, 0.f);
+    for (int e = threadIdx.x; e < pd * px; e += nt) sX[e] = e < n0 * px ? rx[e] : 0.f;
+    for (int e = threadIdx.x; e < n1 * py; e += nt) sY[e] = ry[e];
     __syncthreads();
-    const int lane = threadIdx.x & 31, tx = (n0 + 31) / 32, ty = py / kRows;
-    for (int t = threadIdx.x >> 5; t < tx * ty; t += 8) {
+    const int tx = (n0 + 31) / 32, ty = py / kRows;
+    for (int t = warp; t < tx * ty; t += nw) {
         const int x = (t % tx) * 32 + lane, xc = min(x, n0 - 1), y0 = (t / tx) * kRows;
         float2 acc[kRows];
         const float2 *row[kRows];
@@ -115,47 +115,51 @@ __global__ void __launch_bounds__(256) k_dense_xy(const float *__restrict__ rx, 
 
 struct DenseStep {
     const float2 *rz, *cz;      // [n2][pz] equal pairs, transposed; cz null: identity
-    int n2, pz, chunk;
+    int n2, pz, zc, chunk;
     size_t cols;                // n0 n1
     const float2 *u;
     float2 *z, *d, *x;
     float2 alpha, g, a, b;
 };
 
-// ZC columns per CTA, KR rows per thread, the matrices in stages of s.chunk
-// rows: 16 columns, 8 rows and stages of 16 where they make enough CTAs, else 8
-// columns, 4 rows and both matrices requested whole at the start, since there a
-// thread's chain of stages and products is all the time (27 x 27 x 64: 15.6 us,
-// now 10.9 us; 15 x 15 x 39: 12.4 and 8.6 us; 9 x 9 x 28: 9.9 and 7.4 us).
-template <int ZC, int KR> __global__ void k_dense_z(const DenseStep s) {
+// s.zc columns per CTA, KR rows per thread, the matrices in stages of s.chunk
+// rows. Where they make a CTA for each SM: 8 rows, stages of 16 rows, and as many
+// columns as give every SM the same number of CTAs (51 x 51 x 109: 16 columns, 163
+// CTAs, 26.5 us; 18 columns, 145 CTAs, 19.8 us). Else 8 columns, 4 rows and both
+// matrices requested whole at the start, since there a thread's chain of stages
+// and products is all the time (with 16 columns, 8 rows and stages: 27 x 27 x 64
+// 15.6 us, now 7.2 us; 15 x 15 x 39 12.4 and 6.0 us; 9 x 9 x 28 9.9 and 5.0 us).
+// More warps with fewer rows hide no more (4 rows: 27.6 us), and larger tiles per
+// thread (4 x 4) leave too few warps (35 us).
+template <int KR> __global__ void k_dense_z(const DenseStep s) {
     extern __shared__ __align__(16) unsigned char dz_raw[];
-    const int nm = s.cz ? 2 : 1;
-    float2 *sD = reinterpret_cast<float2 *>(dz_raw);   // [n2][ZC]
-    float2 *sU = sD + (size_t)s.n2 * ZC;
-    float2 *sM = sU + (size_t)s.n2 * ZC;           // stages of [matrix][chunk][pz]
-    const size_t c0 = (size_t)blockIdx.x * ZC;
-    const int nc = (int)min((size_t)ZC, s.cols - c0);
+    const int nm = s.cz ? 2 : 1, zc = s.zc;
+    float2 *sD = reinterpret_cast<float2 *>(dz_raw);   // [n2][zc]
+    float2 *sU = sD + (size_t)s.n2 * zc;
+    float2 *sM = sU + (size_t)s.n2 * zc;           // stages of [matrix][chunk][pz]
+    const size_t c0 = (size_t)blockIdx.x * zc;
+    const int nc = (int)min((size_t)zc, s.cols - c0);
     // rows k0 .. k0 + chunk - 1 of both matrices into stage (k0 / chunk) & 1
     auto issue = [&](int k0) {
-        const int rows = min(s.chunk, s.n2 - k0), per = rows * s.pz / 2;   // 16-byte pieces per matrix
-        for (int e = threadIdx.x; e < nm * per; e += blockDim.x) {
-            const int m = e / per, p = e % per;
-            const float4 *src = reinterpret_cast<const float4 *>((m ? s.cz : s.rz) + (size_t)k0 * s.pz) + p;
-            float4 *dst = reinterpret_cast<float4 *>(sM + ((size_t)((k0 / s.chunk) & 1) * nm + m) * s.chunk * s.pz) + p;
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst)),
-                         "l"(src)
-                         : "memory");
+        const int per = min(s.chunk, s.n2 - k0) * s.pz / 2;   // 16-byte pieces per matrix
+        for (int m = 0; m < nm; ++m) {
+            const float4 *src = reinterpret_cast<const float4 *>((m ? s.cz : s.rz) + (size_t)k0 * s.pz);
+            float4 *dst = reinterpret_cast<float4 *>(sM + ((size_t)(k0 / s.chunk & 1) * nm + m) * s.chunk * s.pz);
+            for (int p = threadIdx.x; p < per; p += blockDim.x)
+                asm volatile(
+                    "cp.async.cg.shared.global [%0], [%1], 16;" ::"r"((unsigned)__cvta_generic_to_shared(dst + p)),
+                    "l"(src + p)
+                    : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
     };
     issue(0);
-    for (int e = threadIdx.x; e < s.n2 * ZC; e += blockDim.x) {
-        const int k = e / ZC, c = e % ZC;
+    const int c = threadIdx.x % zc, g = threadIdx.x / zc, z0 = g * KR;
+    for (int k = g; k < s.n2; k += s.pz / KR) {
         const size_t i = (size_t)k * s.cols + c0 + min(c, nc - 1);
-        sD[e] = s.d[i];
-        sU[e] = s.u[i];
+        sD[k * zc + c] = s.d[i];
+        sU[k * zc + c] = s.u[i];
     }
-    const int c = threadIdx.x % ZC, z0 = (threadIdx.x / ZC) * KR;
     // the vectors of this thread's rows, requested before the products
     float2 zv[KR], xv[KR];
 #pragma unroll
@@ -174,11 +178,11 @@ template <int ZC, int KR> __global__ void k_dense_z(const DenseStep s) {
         const int rows = min(s.chunk, s.n2 - k0);
         for (int m = 0; m < nm; ++m) {
             const float2 *mat = sM + ((size_t)((k0 / s.chunk) & 1) * nm + m) * s.chunk * s.pz + z0;
-            const float2 *v = (m ? sU : sD) + (size_t)k0 * ZC + c;
+            const float2 *v = (m ? sU : sD) + (size_t)k0 * zc + c;
 #pragma unroll 4
             for (int k = 0; k < rows; ++k) {
                 const float4 *q = reinterpret_cast<const float4 *>(mat + (size_t)k * s.pz);
-                const float2 w = v[k * ZC];
+                const float2 w = v[k * zc];
 #pragma unroll
                 for (int j = 0; j < KR / 2; ++j) {
                     const float4 p = q[j];
@@ -194,8 +198,8 @@ template <int ZC, int KR> __global__ void k_dense_z(const DenseStep s) {
         const int k = z0 + j;
         if (k >= s.n2) break;
         const size_t i = (size_t)k * s.cols + c0 + c;
-        if (!s.cz) acc[j] = __fadd2_rn(acc[j], sU[k * ZC + c]);
-        const float2 dv = sD[k * ZC + c];
+        if (!s.cz) acc[j] = __fadd2_rn(acc[j], sU[k * zc + c]);
+        const float2 dv = sD[k * zc + c];
         float2 t = zv[j];   // z - alpha d - g acc
         cfma(t, make_float2(-s.alpha.x, -s.alpha.y), dv);
         cfma(t, make_float2(-s.g.x, -s.g.y), acc[j]);
@@ -223,7 +227,7 @@ size_t z_smem(int n2, int zc, int chunk) {
 // per coefficient at a third of the FP32 rate; general, four launches of
 // latency-bound kernels plus 43 ps per coefficient (the banded apply's 17 and
 // the line solves' 26 on large grids). Both sides measured at 51 x 51 x 109
-// (51 against 56) and on the benchmark's 163 x 163 x 333 level (general).
+// (33 against 56) and on the benchmark's 163 x 163 x 333 level (general).
 bool DenseLevel::pays(const int *n, size_t ndof) {
     const double dense = 6.0 + 0.08e-6 * 2.0 * ndof * (n[0] + n[1] + 2 * n[2]);
     const double general = 35.0 + 43e-6 * ndof;
@@ -326,13 +330,15 @@ bool DenseLevel::prepare(const Operator &op, cudaStream_t st) {
 void DenseLevel::step(const Operator &op, void *z, void *d, void *x, void *u, cd a, cd b, cudaStream_t st) const {
     static const bool attr = [] {   // once, to the largest size any level may use
         TDZ_CUDA(cudaFuncSetAttribute(k_dense_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
-        TDZ_CUDA(cudaFuncSetAttribute(k_dense_z<16, 8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
-        TDZ_CUDA(cudaFuncSetAttribute(k_dense_z<8, 4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
+        TDZ_CUDA(cudaFuncSetAttribute(k_dense_z<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
+        TDZ_CUDA(cudaFuncSetAttribute(k_dense_z<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
         return true;
     }();
     (void)attr;
-    k_dense_xy<<<n[2], 256, xy_smem(n[0], n[1]), st>>>(rx.as<float>(), ry.as<float>(), n[0], n[1], n[0], pd, py,
-                                                       static_cast<const float2 *>(d), static_cast<float2 *>(u));
+    const int tasks = (n[0] + 31) / 32 * (py / kRows), rounds = (tasks + 15) / 16;   // one per warp and round
+    k_dense_xy<<<n[2], 32 * std::max(8, (tasks + rounds - 1) / rounds), xy_smem(n[0], n[1]), st>>>(
+        rx.as<float>(), ry.as<float>(), n[0], n[1], n[0], pd, py, static_cast<const float2 *>(d),
+        static_cast<float2 *>(u));
     auto f2 = [](cd v) { return make_float2((float)v.real(), (float)v.imag()); };
     DenseStep s{};
     s.rz = rz.as<float2>();
@@ -349,11 +355,15 @@ void DenseLevel::step(const Operator &op, void *z, void *d, void *x, void *u, cd
     s.a = f2(a);
     s.b = f2(b);
     if (s.cols > (size_t)8 * sm_count() || z_smem(n[2], 8, n[2]) > kDenseSmem) {
+        const size_t most = z_smem(n[2], 20, 16) <= kDenseSmem ? 20 : 16, sms = sm_count();
+        const size_t ctas = (s.cols + sms * most - 1) / (sms * most) * sms;
+        s.zc = (int)std::max<size_t>(8, (s.cols + ctas - 1) / ctas);
         s.chunk = 16;
-        k_dense_z<16, 8><<<(unsigned)((s.cols + 15) / 16), 16 * (pz / 8), z_smem(n[2], 16, 16), st>>>(s);
+        k_dense_z<8><<<(unsigned)((s.cols + s.zc - 1) / s.zc), s.zc * (pz / 8), z_smem(n[2], s.zc, 16), st>>>(s);
     } else {
+        s.zc = 8;
         s.chunk = n[2];
-        k_dense_z<8, 4><<<(unsigned)((s.cols + 7) / 8), 8 * (pz / 4), z_smem(n[2], 8, n[2]), st>>>(s);
+        k_dense_z<4><<<(unsigned)((s.cols + 7) / 8), 8 * (pz / 4), z_smem(n[2], 8, n[2]), st>>>(s);
     }
     TDZ_CUDA(cudaGetLastError());
     count_launch(2);
