@@ -54,10 +54,8 @@ __device__ __forceinline__ float d2f_trunc(double v) {   // dff_split without th
     const unsigned int sign = h32 & 0x80000000u;
     const unsigned int hb = ((__funnelshift_l(l32, h32, 3) ^ 0x40000000u) & 0x7FFFFFFFu) | sign;
     const unsigned int above = (h32 & 0x7FFFFFFFu) - ((1023u - 100u) << 20);
-    if (above < (228u << 20)) return __uint_as_float(hb);
-    if ((int)above < 0) return __uint_as_float(sign);
-    const bool nan = (h32 & 0x7FF00000u) == 0x7FF00000u && ((h32 & 0xFFFFFu) | l32);
-    return __uint_as_float(sign | (nan ? 0x7FC00000u : 0x7F800000u));
+    const unsigned int other = (int)above < 0 ? sign : hb | 0x7F800000u;
+    return __uint_as_float(above < (228u << 20) ? hb : other);   // a select, as in dff_split
 }
 
 // memory complex -> arithmetic complex

@@ -142,8 +142,7 @@ template <> __device__ __forceinline__ double2 gzero<double2>() { return make_do
 template <class C2, int TT> constexpr int kGemmK = sizeof(C2) == 16 && TT == 4 ? 8 : 16;
 template <class D, class S> __device__ __forceinline__ D gconv(const S &v) { return v; }
 template <> __device__ __forceinline__ float2 gconv<float2, double2>(const double2 &v) {
-    const dff x = dff_split(v.x), y = dff_split(v.y);
-    return make_float2(__fadd_rn(x.hi, x.lo), __fadd_rn(y.hi, y.lo));
+    return make_float2(dff_split(v.x).hi, dff_split(v.y).hi);
 }
 template <> __device__ __forceinline__ double2 gconv<double2, float2>(const float2 &v) {
     return make_double2(f2d_exact(v.x), f2d_exact(v.y));
@@ -272,9 +271,8 @@ __global__ void k_to_planar(const double2 *__restrict__ r, float *__restrict__ a
         const size_t row = e / n0;
         const int x = (int)(e % n0);
         const double2 v = r[e];   // FP64 -> FP32 without the (slow) FP64 pipe
-        const dff re = dff_split(v.x), im = dff_split(v.y);
-        a[(row * 2) * ld + x] = __fadd_rn(re.hi, re.lo);
-        a[(row * 2 + 1) * ld + x] = __fadd_rn(im.hi, im.lo);
+        a[(row * 2) * ld + x] = dff_split(v.x).hi;
+        a[(row * 2 + 1) * ld + x] = dff_split(v.y).hi;
     }
 }
 

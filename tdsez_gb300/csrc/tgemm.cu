@@ -651,9 +651,8 @@ __global__ void __launch_bounds__(kB3Threads, 1) k_transform_b3(const B3Params p
                     float re[4], im[4];
 #pragma unroll
                     for (int j = 0; j < 4; ++j) {
-                        const dff x = dff_split(v[m][j].x), y = dff_split(v[m][j].y);
-                        re[j] = __fadd_rn(x.hi, x.lo);
-                        im[j] = __fadd_rn(y.hi, y.lo);
+                        re[j] = dff_split(v[m][j].x).hi;   // rounded to FP32
+                        im[j] = dff_split(v[m][j].y).hi;
                     }
                     uint8_t *sr = st + b3_off(2 * r, qt >> 1) + 8 * (qt & 1);
                     uint8_t *si = st + b3_off(2 * r + 1, qt >> 1) + 8 * (qt & 1);
