@@ -365,8 +365,8 @@ def run_tdz(args):
                         "double-float applies); no learned component",
         "precision_note": "FP64 storage; outer residual and right-hand-side applies in double-float arithmetic "
                           "(~48 bits, 1e-14 relative) rather than native FP64; Arnoldi apply in FP32 arithmetic "
-                          "certified by the bound gamma |||A||| ||z||; preconditioner in FP32 with TF32 hi/lo "
-                          "tensor-core transforms (no BF16x3)",
+                          "certified by the bound gamma |||A||| ||z||; preconditioner in FP32 with BF16 x 3 "
+                          "tensor-core transforms (24-bit operands)",
         "vs_plain_mg": (value / plain["steps_per_s"]) if plain else None,
         "mixed_mg": mixed_mg,
         "mixed_mg_exact_coarse": exact_coarse,
@@ -385,10 +385,10 @@ def run_tdz(args):
                      "frac": bytes64 / tdf / 1e9 / pk.get("hbm_gbs", 6800.0), "traffic": DF_APPLY_TRAFFIC,
                      "peak_source": "measured" if "hbm_gbs" in pk else "fallback",
                      "launch_us": tdf * 1e6, "bytes_per_launch": bytes64,
-                     "limiter": "FP32 pipes: 12 FP32 instructions per double-float FMA (ncu: 70% issue, "
-                                "55% FMA pipe)",
+                     "limiter": "fixed latencies at 12 to 16 warps per SM; 10 FP32 instructions per "
+                                "double-float FMA (ncu: 41% issue, 47% FMA pipe)",
                      "fp32_apply": {"kernel": "k_apply3d_rb<float> (multigrid smoother and residual; latency-bound, "
-                                              "ncu: 57% issue, 24% warps active)",
+                                              "ncu: 58% issue, 24% warps active)",
                                     "achieved": ach32, "frac": ach32 / pk.get("hbm_gbs", 6800.0),
                                     "launch_us": t32 * 1e6, "bytes_per_launch": bytes32},
                      "fp64_apply": {"kernel": "k_apply3d<double> (native FP64, not used by the step)",
