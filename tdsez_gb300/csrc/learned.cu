@@ -135,7 +135,7 @@ float Multigrid::train_recorded(int epochs, float lr, uint64_t seed, cudaStream_
 float Multigrid::train_coarse(int pairs, int epochs, float lr, uint64_t seed, cudaStream_t st) {
     TDZ_CHECK(lrn.on, TDZ_ERR_STATE, "the learned coarse correction needs mg_learned and FP32 levels");
     TDZ_CHECK(pairs >= lrn.batch && epochs >= 1, TDZ_ERR_ARG, "need at least one batch of pairs and one epoch");
-    for (size_t l = 1; l < lv.size(); ++l) lv[l].opp->sigma = fine->sigma;
+    begin(st);
     MGLevel &m = lv.back();
     const int n = (int)m.ndof;
     const size_t per = 2 * (size_t)n;
@@ -186,7 +186,7 @@ float Multigrid::train_coarse(int pairs, int epochs, float lr, uint64_t seed, cu
 
 std::pair<double, double> Multigrid::coarse_gain(int trials, uint64_t seed, cudaStream_t st) {
     TDZ_CHECK(lrn.on && lrn.trained, TDZ_ERR_STATE, "the learned coarse correction is not trained");
-    for (size_t l = 1; l < lv.size(); ++l) lv[l].opp->sigma = fine->sigma;
+    begin(st);
     MGLevel &m = lv.back();
     std::mt19937_64 rng(seed);
     DevBuf b(m.ndof * sizeof(float2)), e(m.ndof * sizeof(float2)), c(m.ndof * sizeof(float2));

@@ -11,7 +11,6 @@
 // Kronecker line solves); coarsest level: Chebyshev over the whole segment.
 #pragma once
 
-#include <array>
 #include <memory>
 #include <vector>
 
@@ -37,8 +36,7 @@ struct RowSparse {
 // mg_dense.cu).
 struct DenseLevel {
     bool ok = false;                      // matrices built
-    bool ready = false;                   // combined for the current stage
-    std::array<cd, 5> at{};               // the stage scalars it was combined for
+    bool ready = false;                   // combined by the last prepare()
     bool has_c = false;
     int n[3] = {1, 1, 1}, pd = 0, py = 0, pz = 0;
     DevBuf base[3];                       // per axis M_d^-1 B of every base band, [band][n][n] FP32
@@ -115,6 +113,12 @@ struct Multigrid : Precond {
 
     void setup(Operator *fine_, const MGOptions &o, cudaStream_t st);
     void estimate_bounds(cudaStream_t st);
+    // every entry point that runs chebyshev() starts here: the levels take the
+    // fine operator's stage scalars and their dense matrices are combined for
+    // them on the entry's own stream. Nothing is trusted from an earlier call: a
+    // captured one combines when its graph runs, not when it is recorded, and
+    // again at every replay.
+    void begin(cudaStream_t st);
     void vcycle(int l, cudaStream_t st);  // lv[l].b -> lv[l].x
     // learned coarse correction (learned.cu)
     void learned_setup();

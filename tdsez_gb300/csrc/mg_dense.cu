@@ -323,7 +323,6 @@ bool DenseLevel::prepare(const Operator &op, cudaStream_t st) {
     TDZ_CUDA(cudaGetLastError());
     count_launch();
     ready = true;
-    at = op.sigma;
     return true;
 }
 

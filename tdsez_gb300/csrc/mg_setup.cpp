@@ -350,7 +350,7 @@ void chebyshev(MGLevel &m, int prec, double mu_a, double mu_b, double w, int ste
     const bool degenerate = std::abs(delta) <= 1e-12 * std::abs(theta);   // damped Richardson, one step
     const cd sigma1 = degenerate ? cd(1.0) : theta / delta;
     cd rho = 1.0 / sigma1;
-    const bool dense = m.dense.ready && m.dense.at == op.sigma && steps > 1 && !degenerate;
+    const bool dense = m.dense.ready && steps > 1 && !degenerate;
     ChebStep first{1.0 / theta, 0.0, m.d.ptr, m.x.ptr, x_zero, dense};
     m.minv.apply(r, m.z.ptr, prec, st, &first);
     if (degenerate) return;
@@ -425,10 +425,13 @@ void Multigrid::vcycle(int l, cudaStream_t st) {
     chebyshev(m, prec, lo, m.mu_hi, m.w_max, opt.smooth, false, st);
 }
 
-void Multigrid::apply(const double2 *r, double2 *z, cudaStream_t st) {
-    // coarse levels follow the current stage scalars of the fine operator
+void Multigrid::begin(cudaStream_t st) {
     for (size_t l = 1; l < lv.size(); ++l) lv[l].opp->sigma = fine->sigma;
     for (auto &m : lv) m.dense.prepare(*m.opp, st);
+}
+
+void Multigrid::apply(const double2 *r, double2 *z, cudaStream_t st) {
+    begin(st);
     MGLevel &f = lv[0];
     blas::cast(r, TDZ_FP64, f.b.ptr, prec, f.ndof, st);
     vcycle(0, st);
