@@ -94,48 +94,69 @@ __device__ __forceinline__ cdff ld_df(const double2 &v) { return load_c<cdff>(v)
 __device__ __forceinline__ double2 st_df(const cdff &c) { return store_c<double2>(c); }
 __host__ __device__ inline cdff mk_df(dff re, dff im) { return make_cdff(re, im); }
 
-// a + b, renormalised (both components)
-__device__ __forceinline__ cdff add_df(const cdff &a, const cdff &b) {
-    const float2 s = __fadd2_rn(a.hi, b.hi), bv = sub2(s, a.hi);
-    const float2 err = __fadd2_rn(sub2(a.hi, sub2(s, bv)), sub2(b.hi, bv));
-    cdff r;
-    r.hi = s;
-    r.lo = __fadd2_rn(__fadd2_rn(a.lo, b.lo), err);
-    return cnorm(r);
+// Sums of N values of each lane over the warp, in FP64 (the sums over threads
+// keep FP64's bits whatever arithmetic the products took): at every step the
+// lanes of a pair keep one half of the values each, so that a step halves the
+// additions instead of repeating all of them (10 values: 12 additions per lane
+// against 50), since GB300 issues an FP64 instruction of a warp in 16 clocks of
+// the whole SM. Five dots of 67 600 entries: 15 us, 17 us with every value added
+// up in double-float on the FP32 pipes, which loses the bits past 48. Every value
+// is the sum of the same pairs as in a tree of shfl_down, to the bit. On return
+// a[0] is the sum of value `at` where `own` (one lane per value).
+template <int OFF, int N, int NV>
+__device__ __forceinline__ void warp_sums(double (&a)[NV], int lane, int &at, int &left, bool &own) {
+    if constexpr (OFF > 0) {
+        const bool up = lane & OFF;
+        if constexpr (N == 1) {
+            a[0] += __shfl_xor_sync(0xffffffffu, a[0], OFF);
+            own = own && !up;
+            warp_sums<OFF / 2, 1>(a, lane, at, left, own);
+        } else {
+            constexpr int H = (N + 1) / 2;   // the upper half may have one value less: a zero in its place
+#pragma unroll
+            for (int i = 0; i < H; ++i) {
+                const double lo = a[i], hi = i + H < N ? a[i + H] : 0.0;
+                a[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, OFF);
+            }
+            at += up ? H : 0;
+            left = up ? left - H : min(left, H);
+            warp_sums<OFF / 2, H>(a, lane, at, left, own);
+        }
+    } else {
+        own = own && left > 0;
+    }
 }
-// CTA sums of R double-float accumulators into partial[i][block]: within a
-// warp in double-float on the FP32 pipes, across warps in FP64. (FP64 shuffles
-// for every warp cost more than the sums themselves: GB300 issues an FP64
-// instruction of a warp in 16 clocks of the whole SM, and 1216 CTAs with five
-// results spent 27 us in this tail alone.)
-template <int R> __device__ __forceinline__ void cta_partials(cdff (&acc)[R], double2 *partial) {
-    __shared__ double2 red[kThreads / 32][R];
+// CTA sums of R complex values into partial[i][block], in FP64 (fixed order)
+template <int R> __device__ __forceinline__ void cta_partials(double (&v)[2 * R], double2 *partial) {
+    __shared__ double red[kThreads / 32][2 * R];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    int at = 0, left = 2 * R;
+    bool own = true;
+    warp_sums<16, 2 * R>(v, lane, at, left, own);
+    if (own) red[warp][at] = v[0];
+    __syncthreads();
+    if (threadIdx.x < 2 * R) {
+        double t = 0.0;
+#pragma unroll
+        for (int w = 0; w < kThreads / 32; ++w) t += red[w][threadIdx.x];
+        reinterpret_cast<double *>(partial + (size_t)(threadIdx.x / 2) * gridDim.x + blockIdx.x)[threadIdx.x & 1] = t;
+    }
+}
+// the same of R double-float accumulators, whose parts are added up in FP64
+// before any sum over threads
+template <int R> __device__ __forceinline__ void cta_partials(const cdff (&acc)[R], double2 *partial) {
+    double v[2 * R];
 #pragma unroll
     for (int i = 0; i < R; ++i) {
-        cdff v = cnorm(acc[i]);
-#pragma unroll
-        for (int off = 16; off > 0; off >>= 1) {
-            cdff o;
-            o.hi.x = __shfl_down_sync(0xffffffffu, v.hi.x, off);
-            o.hi.y = __shfl_down_sync(0xffffffffu, v.hi.y, off);
-            o.lo.x = __shfl_down_sync(0xffffffffu, v.lo.x, off);
-            o.lo.y = __shfl_down_sync(0xffffffffu, v.lo.y, off);
-            v = add_df(v, o);
-        }
-        if (lane == 0) red[warp][i] = make_double2(dff_to_double(v.re()), dff_to_double(v.im()));
+        v[2 * i] = dff_to_double(acc[i].re());
+        v[2 * i + 1] = dff_to_double(acc[i].im());
     }
-    __syncthreads();
-    if (threadIdx.x < R) {
-        double re = 0.0, im = 0.0;
-#pragma unroll
-        for (int w = 0; w < kThreads / 32; ++w) { re += red[w][threadIdx.x].x; im += red[w][threadIdx.x].y; }
-        partial[(size_t)threadIdx.x * gridDim.x + blockIdx.x] = make_double2(re, im);
-    }
+    cta_partials<R>(v, partial);
 }
 
+// (three CTAs per SM as far as the registers go, two beyond)
 template <int K>
-__global__ void __launch_bounds__(kThreads) k_mdot_df(PtrPack V, const double2 *w, size_t n, double2 *partial) {
+__global__ void __launch_bounds__(kThreads, K <= 13 ? 3 : 2) k_mdot_df(PtrPack V, const double2 *w, size_t n, double2 *partial) {
     cdff acc[K];
 #pragma unroll
     for (int i = 0; i < K; ++i) acc[i] = czero<cdff>();
@@ -264,12 +285,18 @@ __global__ void __launch_bounds__(kThreads) k_gs_df(double2 *w, PtrPack V, CoefD
         }
         if constexpr (MODE != 0) fma2(acc[R - 1], x.hi, x.lo, x.hi, x.lo);
     }
+    double r[2 * R];
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+        r[2 * i] = dff_to_double(acc[i].re());
+        r[2 * i + 1] = dff_to_double(acc[i].im());
+    }
     // |w|^2: the sums of the squares of the real and of the imaginary parts
     if constexpr (MODE != 0) {
-        const cdff t = cnorm(acc[R - 1]);
-        acc[R - 1] = add_df(make_cdff(t.re(), dff(0.f)), make_cdff(t.im(), dff(0.f)));
+        r[2 * R - 2] += r[2 * R - 1];
+        r[2 * R - 1] = 0.0;
     }
-    cta_partials<R>(acc, partial);
+    cta_partials<R>(r, partial);
 }
 
 // per-block partial sums of conj(V_i) w, i < k; partial layout [i][block]
