@@ -101,16 +101,16 @@ __host__ __device__ inline cdff mk_df(dff re, dff im) { return make_cdff(re, im)
 // against 50), since GB300 issues an FP64 instruction of a warp in 16 clocks of
 // the whole SM. Five dots of 67 600 entries: 15 us, 17 us with every value added
 // up in double-float on the FP32 pipes, which loses the bits past 48. Every value
-// is the sum of the same pairs as in a tree of shfl_down, to the bit. On return
-// a[0] is the sum of value `at` where `own` (one lane per value).
+// is the sum of the same pairs as in a tree of shfl_down, to the bit. The sums
+// go to out[at], ...: the lane's share of them, `left` values (at most N, more
+// than one only for more than 32 values), from one lane each.
 template <int OFF, int N, int NV>
-__device__ __forceinline__ void warp_sums(double (&a)[NV], int lane, int &at, int &left, bool &own) {
+__device__ __forceinline__ void warp_sums(double (&a)[NV], int lane, int at, int left, bool own, double *out) {
     if constexpr (OFF > 0) {
         const bool up = lane & OFF;
         if constexpr (N == 1) {
             a[0] += __shfl_xor_sync(0xffffffffu, a[0], OFF);
-            own = own && !up;
-            warp_sums<OFF / 2, 1>(a, lane, at, left, own);
+            warp_sums<OFF / 2, 1>(a, lane, at, left, own && !up, out);
         } else {
             constexpr int H = (N + 1) / 2;   // the upper half may have one value less: a zero in its place
 #pragma unroll
@@ -118,22 +118,18 @@ __device__ __forceinline__ void warp_sums(double (&a)[NV], int lane, int &at, in
                 const double lo = a[i], hi = i + H < N ? a[i + H] : 0.0;
                 a[i] = (up ? hi : lo) + __shfl_xor_sync(0xffffffffu, up ? lo : hi, OFF);
             }
-            at += up ? H : 0;
-            left = up ? left - H : min(left, H);
-            warp_sums<OFF / 2, H>(a, lane, at, left, own);
+            warp_sums<OFF / 2, H>(a, lane, up ? at + H : at, up ? left - H : min(left, H), own, out);
         }
     } else {
-        own = own && left > 0;
+#pragma unroll
+        for (int i = 0; i < N; ++i)
+            if (own && i < left) out[at + i] = a[i];
     }
 }
 // CTA sums of R complex values into partial[i][block], in FP64 (fixed order)
 template <int R> __device__ __forceinline__ void cta_partials(double (&v)[2 * R], double2 *partial) {
     __shared__ double red[kThreads / 32][2 * R];
-    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    int at = 0, left = 2 * R;
-    bool own = true;
-    warp_sums<16, 2 * R>(v, lane, at, left, own);
-    if (own) red[warp][at] = v[0];
+    warp_sums<16, 2 * R>(v, threadIdx.x & 31, 0, 2 * R, true, red[threadIdx.x >> 5]);
     __syncthreads();
     if (threadIdx.x < 2 * R) {
         double t = 0.0;
