@@ -365,15 +365,15 @@ __global__ void __launch_bounds__(TX *TY) k_apply3d(const __grid_constant__ Appl
     }
 }
 
-// ---------------------------------------------------------------- 2D kernel
-// A CTA owns a kTX2 x kTY2 output tile: the halo tile of the input in shared
-// memory, the x stage of its kTY2 + 2P rows, then the y stage, one output per
-// thread; two barriers in all. A 2D operator is small (a few hundred thousand
-// coefficients at most in practice), so what counts is the latency of one
-// tile and having enough tiles: streaming row by row through a register ring
-// recomputed no halo rows but left a 260 x 260 grid 48 CTAs of 24 dependent
-// row steps (double-float, degree 4: 224 us; this kernel 19 us on its 297
-// tiles, the x stage computed twice over).
+// ---------------------------------------------------------------- 2D kernels
+// Small grids, and double-float on every grid. A CTA owns a kTX2 x kTY2 output
+// tile: the halo tile of the input in shared memory, the x stage of its
+// kTY2 + 2P rows, then the y stage, one output per thread; two barriers in all.
+// What counts there is the latency of one tile and having enough tiles:
+// streaming row by row (k_apply2d_ring below) recomputes no halo rows but
+// leaves a 260 x 260 grid 48 CTAs of 24 dependent row steps (double-float,
+// degree 4: 224 us; this kernel 19 us on its 297 tiles, the x stage computed
+// twice over).
 constexpr int kTX2 = 32, kTY2 = 8;
 template <class T, int P, bool HB, bool HC> struct Shape2D {
     using C = typename CT<T>::type;
@@ -383,10 +383,16 @@ template <class T, int P, bool HB, bool HC> struct Shape2D {
                                    (HB ? sizeof(T) * BW * kTY2 : 0);
 };
 
-// sum_j a_j v_j, the a_j complex or all imaginary (the uniform branch outside the loop)
+// sum_j a_j v_j, the a_j complex, all real or all imaginary (the uniform branch outside the loop)
 template <int BW, class C> __device__ __forceinline__ C dot_kind(const C (&a)[BW], const C *v, int stride, int kind) {
     C s;
-    if (kind == 2) {
+    if (kind == 1) {
+#pragma unroll
+        for (int j = 0; j < BW; ++j) {
+            if (j == 0) rset(s, cre(a[j]), v[j * stride]);
+            else rfma(s, cre(a[j]), v[j * stride]);
+        }
+    } else if (kind == 2) {
 #pragma unroll
         for (int j = 0; j < BW; ++j) {
             if (j == 0) iset(s, cim(a[j]), v[j * stride]);
@@ -477,6 +483,90 @@ __global__ void __launch_bounds__(kTX2 *kTY2) k_apply2d(const __grid_constant__ 
     }
     const size_t e = (size_t)gy * n0 + gx;
     Y[e] = out_value<T, MC>(prm, e, out);
+}
+
+// Large grids, FP32 and FP64: the x stage on a row tile, the outer stage along y
+// in a register ring, so that no x stage is computed twice and the y stage
+// reads no shared memory. Worth it once its CTAs, each a chain of dependent
+// rows, fill the chip (ring2d below).
+constexpr int kTX2R = 128;
+// resident CTAs asked of the compiler: FP64 as many registers as it likes; FP32 its
+// own choice, but for degree 3 with the inner-axis stream, where that ends one CTA
+// short of eight (1448^2: 68 us, with eight 44 us)
+template <class T, int P, bool HB, bool HC> constexpr int kRingMin =
+    sizeof(T) == 8 ? 1 : P == 3 && HB && !HC ? 8 : 0;
+template <class T, int P, bool HB, bool HC>
+__global__ void __launch_bounds__(kTX2R, kRingMin<T, P, HB, HC>) k_apply2d_ring(const __grid_constant__ ApplyParams<T> prm) {
+    using C = typename CT<T>::type;
+    using MC = typename MemC<T>::type;
+    constexpr int BW = 2 * P + 1, TX = kTX2R, RX = TX + 2 * P;
+    __shared__ C sIn[RX];
+    __shared__ C sZA[BW], sZC[BW];
+    __shared__ T sZM[BW];
+    const int tx = threadIdx.x;
+    const int n0 = prm.n0, n1 = prm.n1;
+    const int x0 = blockIdx.x * TX, gx = x0 + tx;
+    const int z0 = blockIdx.y * prm.zchunk;
+    const int z1 = min(n1, z0 + prm.zchunk);
+    if (z0 >= z1) return;
+    const MC *__restrict__ X = static_cast<const MC *>(prm.x);
+    MC *__restrict__ Y = static_cast<MC *>(prm.y);
+    T xm[BW], xs[HC ? BW : 1];
+    C xt[HB ? BW : 1];
+#pragma unroll
+    for (int j = 0; j < BW; ++j) {
+        const bool in = gx < n0;
+        xm[j] = in ? prm.b0[((size_t)kM * n0 + gx) * BW + j] : T(0);
+        if constexpr (HC) xs[j] = in ? prm.b0[((size_t)kS * n0 + gx) * BW + j] : T(0);
+        if constexpr (HB) xt[j] = in ? comb_at<T, C>(prm.xT, prm.b0, n0, BW, gx, j) : czero<C>();
+    }
+    C acc[BW];
+#pragma unroll
+    for (int s = 0; s < BW; ++s) acc[s] = czero<C>();
+    const int zs = z0 - P;
+    const int nplanes = (z1 - z0) + 2 * P;
+    for (int base = 0; base < nplanes; base += BW) {
+#pragma unroll
+        for (int ph = 0; ph < BW; ++ph) {
+            const int it = base + ph;
+            if (it >= nplanes) break;
+            const int zin = zs + it;
+            if (zin >= 0 && zin < n1) {
+                __syncthreads();
+                for (int c = tx; c < RX; c += TX) {
+                    const int xx = x0 - P + c;
+                    sIn[c] = (xx >= 0 && xx < n0) ? load_c<C>(X[(size_t)zin * n0 + xx]) : czero<C>();
+                }
+                if (tx < BW) {
+                    sZA[tx] = comb_at<T, C>(prm.zA, prm.b1, n1, BW, zin, tx);
+                    if constexpr (HB) sZM[tx] = prm.b1[((size_t)kM * n1 + zin) * BW + tx];
+                    if constexpr (HC) sZC[tx] = comb_at<T, C>(prm.zC, prm.b1, n1, BW, zin, tx);
+                }
+                __syncthreads();
+                C uM = czero<C>(), uT = czero<C>(), uS = czero<C>();
+#pragma unroll
+                for (int j = 0; j < BW; ++j) {
+                    const C v = sIn[tx + j];
+                    rfma(uM, xm[j], v);
+                    if constexpr (HB) cfma(uT, xt[j], v);
+                    if constexpr (HC) rfma(uS, xs[j], v);
+                }
+#pragma unroll
+                for (int o = 0; o < BW; ++o) {
+                    C &a = acc[(ph - P + o + 2 * BW) % BW];
+                    kfma(a, sZA[o], uM, prm.za_kind);
+                    if constexpr (HB) rfma(a, sZM[o], uT);
+                    if constexpr (HC) kfma(a, sZC[o], uS, prm.zc_kind);
+                }
+            }
+            C &out = acc[(ph - P + 2 * BW) % BW];
+            if (it >= 2 * P) {
+                const int m = zin - P;
+                if (gx < n0) Y[(size_t)m * n0 + gx] = out_value<T, MC>(prm, (size_t)m * n0 + gx, out);
+            }
+            out = czero<C>();
+        }
+    }
 }
 
 // ---------------------------------------------------------------- 1D kernel
@@ -651,8 +741,56 @@ inline void run3d(const ApplyParams<T> &prm0, cudaStream_t st) {
     launch(txw, zchunk);
 }
 
+// The row-streaming kernel instead of the tiles (T = float or double): grids
+// beyond a line in coefficients whose last 128-column tile is mostly filled.
+// Both in us, tiles and streaming, on both sides of the line:
+//   FP32, inner-axis stream, degree 3: 1024^2 33 and 36, 1200^2 42 and 38,
+//   2048^2 105 and 66; without it, mass: 1448^2 29 and 33, 2048^2 52 and 51;
+//   FP64: the second x stage of the tiles counts the more the higher the degree
+//   and the more products it has. Degree 4: CN stage 900^2 246 and 283, 1200^2 421
+//   and 393; with complex coefficients (absorbing layers) 600^2 152 and 172, 750^2
+//   224 and 190; real ones 1200^2 326 and 331, 1448^2 476 and 442; mass 1448^2 212
+//   and 217, 2900^2 803 and 650; the stage of a layered mass, whose second stream
+//   costs the streaming kernel as much, 2048^2 1369 and 1457, 2900^2 2690 and
+//   2587 (degrees 2 and 3: tiles at every size).
+template <class T> inline bool ring2d(const ApplyParams<T> &prm, int P, bool hb, bool hc) {
+    if ((prm.n0 + kTX2R - 1) / kTX2R * kTX2R > 1.3 * prm.n0) return false;
+    double line;   // million coefficients
+    if (std::is_same<T, float>::value) line = !hb ? 2.6 : hc && P == 5 ? 2.0 : 1.25;
+    else if (hb) line = (prm.xt_kind == 0 ? 2.0 : prm.xt_kind == 2 && !hc ? 4.2 : 7.0) / P;
+    else if (hc && prm.zc_kind == 1) line = 5.0 / P;
+    else if (hc) line = P >= 4 ? 22.0 / P : 1e9;
+    else line = 40.0 / (P * P);
+    return 1e-6 * prm.n0 * prm.n1 > line;
+}
+
 template <class T, int P, bool HB, bool HC>
-inline void run2d(const ApplyParams<T> &prm, cudaStream_t st) {
+inline void run2d(const ApplyParams<T> &prm0, cudaStream_t st) {
+    if constexpr (!std::is_same<T, dff>::value) {
+        if (ring2d(prm0, P, HB, HC)) {
+            // one to four waves of CTAs, whichever takes the fewest rows one after the other, the
+            // 2p halo rows of a chunk included; chunks no shorter than 4p rows
+            auto kern = k_apply2d_ring<T, P, HB, HC>;
+            static const int per_sm = [&] {
+                int k = 0;
+                TDZ_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&k, kern, kTX2R, 0));
+                return std::max(1, k);
+            }();
+            ApplyParams<T> prm = prm0;
+            const int tiles = (prm.n0 + kTX2R - 1) / kTX2R;
+            const int slots = per_sm * sm_count();
+            long long cost = -1;
+            int chunks = 1;
+            for (int w = 1; w <= 4; ++w) {
+                const int c = std::max(1, std::min(w * slots / tiles, prm.n1 / (4 * P)));
+                const long long t = (long long)((tiles * c + slots - 1) / slots) * ((prm.n1 + c - 1) / c + 2 * P);
+                if (cost < 0 || t < cost) { cost = t; chunks = c; }
+            }
+            prm.zchunk = (prm.n1 + chunks - 1) / chunks;
+            kern<<<dim3(tiles, (prm.n1 + prm.zchunk - 1) / prm.zchunk), kTX2R, 0, st>>>(prm);
+            return;
+        }
+    }
     auto kern = k_apply2d<T, P, HB, HC>;
     constexpr size_t smem = Shape2D<T, P, HB, HC>::smem;
     static const bool attr = [&] {
@@ -660,9 +798,9 @@ inline void run2d(const ApplyParams<T> &prm, cudaStream_t st) {
         return true;
     }();
     (void)attr;
-    const long long tiles = (long long)((prm.n0 + kTX2 - 1) / kTX2) * ((prm.n1 + kTY2 - 1) / kTY2);
+    const long long tiles = (long long)((prm0.n0 + kTX2 - 1) / kTX2) * ((prm0.n1 + kTY2 - 1) / kTY2);
     TDZ_CHECK(tiles < (1LL << 31), TDZ_ERR_UNSUPPORTED, "too many tiles for the 2D apply");
-    kern<<<(unsigned)tiles, dim3(kTX2, kTY2), smem, st>>>(prm);
+    kern<<<(unsigned)tiles, dim3(kTX2, kTY2), smem, st>>>(prm0);
 }
 
 // per-degree entry points (apply_p<P>.cu)
