@@ -683,7 +683,8 @@ inline void dispatch_streams(int dim, bool hb, bool hc, const ApplyParams<T> &pr
             if (!hb && hc && prm.zc_kind == 2) run3d<T, P, false, true, 0, 2>(prm, st);        // CN stage
             else if (!hb && !hc && prm.za_kind == 1) run3d<T, P, false, false, 1, 0>(prm, st);   // mass
             else if (hb && hc) run3d<T, P, true, true>(prm, st);
-            else if (hb) run3d<T, P, true, false>(prm, st);
+            else if (hb && skip_rows<P, TileY<T, true, false>::v>(prm.n1)) run3d<T, P, true, false>(prm, st);
+            else if (hb) run3d<T, P, true, false, 0, 0, false>(prm, st);
             else if (hc) run3d<T, P, false, true>(prm, st);
             else run3d<T, P, false, false>(prm, st);
         } else if constexpr (std::is_same<T, float>::value) {

@@ -105,7 +105,8 @@ constexpr int kLoadsPerThread3 = 4;   // covers (TY+2p)(TX+2p) / (TX TY) for p <
 // outer combinations fixed at compile time (0 complex, 1 real, 2 imaginary);
 // the double-float CN stage (KC = 2) and mass (KA = 1) get their own
 // instantiations, which save a quarter of the outer-stage products.
-template <class T, int P, bool HB, bool HC, int TX, int TY, int KA, int KC>
+// SKIP: no products for tile rows past the grid (skip_rows below).
+template <class T, int P, bool HB, bool HC, int TX, int TY, int KA, int KC, bool SKIP>
 __device__ __noinline__ double2 apply3d_run(const ApplyParams<T> &prm, int x0, int y0, int z0, int z1) {
     using C = typename CT<T>::type;
     constexpr int BW = 2 * P + 1, RY = TY + 2 * P, RX = TX + 2 * P;
@@ -200,7 +201,7 @@ __device__ __noinline__ double2 apply3d_run(const ApplyParams<T> &prm, int x0, i
     auto xstage = [&](int it) {
         const int buf = it & 1;
         for (int r = ty; r < RY; r += TY) {
-            if (r >= rows_in) break;   // nobody reads the rows past the grid's last one
+            if (SKIP && r >= rows_in) break;   // nobody reads the rows past the grid's last one
             C uM = czero<C>(), uT = czero<C>(), uS = czero<C>();
 #pragma unroll
             for (int j = 0; j < BW; ++j) {
@@ -262,7 +263,7 @@ __device__ __noinline__ double2 apply3d_run(const ApplyParams<T> &prm, int x0, i
     // buffer a step writes was last read before the previous barrier.
     auto step = [&](int it, int ring) {
         xstage(it + 1);                // a plane past hi leaves results that nobody reads
-        if (gy < n1) yzstage(it, ring);
+        if (!SKIP || gy < n1) yzstage(it, ring);
         store_in(it + 2);
         fetch(it + 3);
         __syncthreads();
@@ -328,7 +329,7 @@ __device__ __noinline__ double2 apply3d_run(const ApplyParams<T> &prm, int x0, i
 // keeps the halo small and leaves no tail wave. A run is a separate
 // (not inlined) function, so the register allocation of its plane loop does
 // not carry the run loop's state.
-template <class T, int P, bool HB, bool HC, int TX, int TY, int KA = 0, int KC = 0>
+template <class T, int P, bool HB, bool HC, int TX, int TY, int KA, int KC, bool SKIP>
 __global__ void __launch_bounds__(TX *TY) k_apply3d(const __grid_constant__ ApplyParams<T> prm) {
     const int txw = blockDim.x;
     const int n0 = prm.n0, n1 = prm.n1, n2 = prm.n2;
@@ -344,7 +345,7 @@ __global__ void __launch_bounds__(TX *TY) k_apply3d(const __grid_constant__ Appl
         pos += z1 - z0;
         if (!first) __syncthreads();   // the last run's readers of the band rows are done
         const double2 r =
-            apply3d_run<T, P, HB, HC, TX, TY, KA, KC>(prm, (tile % tilesX) * txw, (tile / tilesX) * TY, z0, z1);
+            apply3d_run<T, P, HB, HC, TX, TY, KA, KC, SKIP>(prm, (tile % tilesX) * txw, (tile / tilesX) * TY, z0, z1);
         racc.x += r.x;
         racc.y += r.y;
     }
@@ -646,11 +647,20 @@ void set_forced_shape(int txw, int run);
 bool tune_lookup(const TuneKey &k, int *txw, int *zchunk);
 void tune_store(const TuneKey &k, int txw, int zchunk);
 
-template <class T, int P, bool HB, bool HC, int KA = 0, int KC = 0>
+// With the inner-axis stream the test for rows past the grid keeps the compiler
+// from mixing the x stage's products with the other stages' (64^3 elements of
+// degree 4: 383 us without it, 391 us with it), so there it is made only where
+// two fifths of the tile rows are past the grid (10 x 12 x 16 elements of degree 5:
+// 584 and 457 us) and at degree 2 (109 and 103 us).
+template <int P, int TY> inline bool skip_rows(int n1) {
+    const int rows = (n1 + TY - 1) / TY * TY;
+    return P == 2 || 5 * (rows - n1) >= 2 * rows;
+}
+template <class T, int P, bool HB, bool HC, int KA = 0, int KC = 0, bool SKIP = true>
 inline void run3d(const ApplyParams<T> &prm0, cudaStream_t st) {
     using C = typename CT<T>::type;
     constexpr int TY = TileY<T, HB, HC>::v, NU = 1 + (HB ? 1 : 0) + (HC ? 1 : 0);
-    auto kern = k_apply3d<T, P, HB, HC, kTX3, TY, KA, KC>;
+    auto kern = k_apply3d<T, P, HB, HC, kTX3, TY, KA, KC, SKIP>;
     const bool fp32 = std::is_same<T, float>::value;
     const size_t tile_smem = sizeof(C) * ((size_t)2 * (TY + 2 * P) * (kTX3 + 2 * P) + 2 * NU * (TY + 2 * P) * kTX3);
     auto smem_for = [&](int zchunk) {
