@@ -577,10 +577,9 @@ inline void run3d_rb(const ApplyParams<T> &prm0, cudaStream_t st) {
     using Sh = RbShape<T, MC, P, HB, HC, NTY, R>;
     auto kern = k_apply3d_rb<T, MC, P, HB, HC, NTY, R, KA, KC>;
     constexpr size_t kMaxDyn = 220 * 1024;
-    static const int nsm = [&] {   // once per instantiation (thread-safe static initialisation)
-        TDZ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn));
-        return sm_count();
-    }();
+    static std::atomic<unsigned long long> done{0};
+    once_per_device(done, [&] { allow_smem(kern, kMaxDyn); });
+    const int nsm = sm_count();
     const int n2 = prm0.n2;
     TDZ_CHECK(Sh::smem(n2 + 2 * P) <= kMaxDyn, TDZ_ERR_UNSUPPORTED, "outer axis too long for the 3D apply");
     thread_local int occ_n2 = -1, occ_slots = 0;

@@ -670,13 +670,9 @@ inline void run3d(const ApplyParams<T> &prm0, cudaStream_t st) {
     // shared memory grows with the run length (its band rows, at most n2 + 2p
     // planes): one opt-in to the largest size, occupancy at the largest size
     constexpr size_t kMaxDyn = 200 * 1024;
-    static const int nsm = [&] {   // once per instantiation (thread-safe static initialisation)
-        TDZ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMaxDyn));
-        int dev = 0, n = 0;
-        TDZ_CUDA(cudaGetDevice(&dev));
-        TDZ_CUDA(cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev));
-        return n;
-    }();
+    static std::atomic<unsigned long long> done{0};
+    once_per_device(done, [&] { allow_smem(kern, kMaxDyn); });
+    const int nsm = sm_count();
     const int n2 = prm0.n2;
     TDZ_CHECK(smem_for(n2) <= kMaxDyn, TDZ_ERR_UNSUPPORTED, "outer axis too long for the 3D apply");
     thread_local int occ_n2 = -1, occ_slots = 0;   // resident CTAs at the last n2 seen
@@ -803,11 +799,8 @@ inline void run2d(const ApplyParams<T> &prm0, cudaStream_t st) {
     }
     auto kern = k_apply2d<T, P, HB, HC>;
     constexpr size_t smem = Shape2D<T, P, HB, HC>::smem;
-    static const bool attr = [&] {
-        TDZ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-        return true;
-    }();
-    (void)attr;
+    static std::atomic<unsigned long long> done{0};
+    once_per_device(done, [&] { allow_smem(kern, smem); });
     const long long tiles = (long long)((prm0.n0 + kTX2 - 1) / kTX2) * ((prm0.n1 + kTY2 - 1) / kTY2);
     TDZ_CHECK(tiles < (1LL << 31), TDZ_ERR_UNSUPPORTED, "too many tiles for the 2D apply");
     kern<<<(unsigned)tiles, dim3(kTX2, kTY2), smem, st>>>(prm0);

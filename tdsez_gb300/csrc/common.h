@@ -4,6 +4,7 @@
 
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <complex>
 #include <cstdint>
 #include <cstdio>
@@ -96,6 +97,23 @@ struct HostBuf {
     // read by the host after a synchronisation (volatile: kernels write it)
     template <class T> T *as() const { return static_cast<T *>(ptr); }
 };
+
+// f() the first time a call site runs on each device (done: a static of the
+// site). A kernel's opt-in to dynamic shared memory beyond 48 KB holds for one
+// device, and is made once, to the largest size any launch takes, so that
+// launches from several host threads cannot lower it under each other. f may run
+// twice where two threads come first together.
+template <class F> inline void once_per_device(std::atomic<unsigned long long> &done, F f) {
+    int dev = 0;
+    TDZ_CUDA(cudaGetDevice(&dev));
+    const unsigned long long bit = dev < 64 ? 1ull << dev : 0;   // beyond: every time
+    if (done.load(std::memory_order_acquire) & bit) return;
+    f();
+    done.fetch_or(bit, std::memory_order_release);
+}
+template <class K> inline void allow_smem(K *kern, size_t bytes) {
+    TDZ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes));
+}
 
 template <class T> inline void upload(DevBuf &b, const std::vector<T> &v) {
     b.alloc(v.size() * sizeof(T));

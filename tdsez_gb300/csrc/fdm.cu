@@ -913,17 +913,12 @@ template <int P, bool IL> __global__ void __launch_bounds__(2 * kZSubLines) k_zs
 // fresh: the stored factor is not the current stage's
 template <int P, bool CI> void launch_zsolve_t(const ZSolveParams &zp, bool fresh, cudaStream_t st) {
     constexpr size_t kMax = 220 * 1024;
-    // the dynamic shared-memory limit is a property of the kernel, not of a
-    // launch: set it once to the largest size any line length may use, so
-    // that solves of different lengths from several host threads cannot
-    // lower it under each other's launches
-    static const bool attr = [] {
-        TDZ_CUDA(cudaFuncSetAttribute(k_zsolve<P, CI>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
-        TDZ_CUDA(cudaFuncSetAttribute(k_zsub<P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
-        TDZ_CUDA(cudaFuncSetAttribute(k_zsub<P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kMax));
-        return true;
-    }();
-    (void)attr;
+    static std::atomic<unsigned long long> done{0};
+    once_per_device(done, [] {
+        allow_smem(k_zsolve<P, CI>, kMax);
+        allow_smem(k_zsub<P, true>, kMax);
+        allow_smem(k_zsub<P, false>, kMax);
+    });
     const int nl = zp.n0 * zp.n1;
     if (zp.fac) {
         const int blocks = (nl + kZSubLines - 1) / kZSubLines;

@@ -361,13 +361,8 @@ void run_axis_long(const T *L, int axis, typename CT<T>::type *x, int n0, int n1
         while (rows > 1 && (size_t)rows * n0 * sizeof(C) > 96 * 1024) rows /= 2;
         const size_t smem = (size_t)rows * n0 * sizeof(C);
         TDZ_CHECK(smem <= kLineSmem, TDZ_ERR_UNSUPPORTED, "axis too long for the row line solve");
-        // set once to the largest size (a per-kernel limit: concurrent solves of
-        // other lengths must not lower it under this launch)
-        static const bool attr = [] {
-            TDZ_CUDA(cudaFuncSetAttribute(k_line_rows<T, P>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kLineSmem));
-            return true;
-        }();
-        (void)attr;
+        static std::atomic<unsigned long long> done{0};
+        once_per_device(done, [] { allow_smem(k_line_rows<T, P>, kLineSmem); });
         const int nrows = n1 * n2;
         k_line_rows<T, P><<<(nrows + rows - 1) / rows, rows, smem, st>>>(L, n0, x, nrows);
     } else if (axis == 1) {
@@ -430,12 +425,11 @@ bool run_axis(const BandChol &F, int axis, const typename CT<T>::type *src, type
             if (waves < 0 || k < waves) { waves = k; warps = w; }
         }
         auto kern = axis == 0 ? k_line_tile<T, P, true> : k_line_tile<T, P, false>;
-        static const bool attr = [] {   // once, to the largest size (see run_axis_long)
-            TDZ_CUDA(cudaFuncSetAttribute(k_line_tile<T, P, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem));
-            TDZ_CUDA(cudaFuncSetAttribute(k_line_tile<T, P, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kTileSmem));
-            return true;
-        }();
-        (void)attr;
+        static std::atomic<unsigned long long> done{0};
+        once_per_device(done, [] {
+            allow_smem(k_line_tile<T, P, true>, kTileSmem);
+            allow_smem(k_line_tile<T, P, false>, kTileSmem);
+        });
         const long long grid = (g.tiles + warps - 1) / warps;
         TDZ_CHECK(grid < (1LL << 31), TDZ_ERR_UNSUPPORTED, "too many lines");
         kern<<<(unsigned)grid, 32 * warps, tab + warps * per_warp, st>>>(g);

@@ -327,13 +327,12 @@ bool DenseLevel::prepare(const Operator &op, cudaStream_t st) {
 }
 
 void DenseLevel::step(const Operator &op, void *z, void *d, void *x, void *u, cd a, cd b, cudaStream_t st) const {
-    static const bool attr = [] {   // once, to the largest size any level may use
-        TDZ_CUDA(cudaFuncSetAttribute(k_dense_xy, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
-        TDZ_CUDA(cudaFuncSetAttribute(k_dense_z<8>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
-        TDZ_CUDA(cudaFuncSetAttribute(k_dense_z<4>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDenseSmem));
-        return true;
-    }();
-    (void)attr;
+    static std::atomic<unsigned long long> done{0};
+    once_per_device(done, [] {
+        allow_smem(k_dense_xy, kDenseSmem);
+        allow_smem(k_dense_z<8>, kDenseSmem);
+        allow_smem(k_dense_z<4>, kDenseSmem);
+    });
     const int tasks = (n[0] + 31) / 32 * (py / kRows), rounds = (tasks + 15) / 16;   // one per warp and round
     k_dense_xy<<<n[2], 32 * std::max(8, (tasks + rounds - 1) / rounds), xy_smem(n[0], n[1]), st>>>(
         rx.as<float>(), ry.as<float>(), n[0], n[1], n[0], pd, py, static_cast<const float2 *>(d),

@@ -699,11 +699,8 @@ void launch_q3s(const QuadTerm &q, const QuadParams<typename QArith<A>::TT> &prm
     using S = QStream<A, P, TE>;
     auto kern = k_quad3_stream<A, P, TE>;
     static_assert(S::smem <= 200 * 1024, "quadrature rings larger than the shared memory");
-    static const bool attr = [&] {
-        TDZ_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)S::smem));
-        return true;
-    }();
-    (void)attr;
+    static std::atomic<unsigned long long> done{0};
+    once_per_device(done, [&] { allow_smem(kern, S::smem); });
     const int tiles = ((q.nel[0] + TE - 1) / TE) * ((q.nel[1] + TE - 1) / TE);
     // about two CTAs per SM in total, z chunks no shorter than 4 (p + 1) elements
     int chunks = std::max(1, (2 * sm_count() + tiles - 1) / tiles);

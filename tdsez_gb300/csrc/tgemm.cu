@@ -889,19 +889,11 @@ int variant() {
 // the B-resident kernel: in / out FP32 planar, or in64 / out64 FP64 natural order
 void launch_b3(const TransformMat &T, const float *in, const double2 *in64, int planes, int R, int ldi, float *out,
                int ldo, double2 *out64, double *norm, cudaStream_t st) {
-    // opt-in to the largest size once per device (the batch API steps runs from several host threads)
-    {
-        static std::mutex mu;
-        static std::set<int> done;
-        int dev = 0;
-        TDZ_CUDA(cudaGetDevice(&dev));
-        std::lock_guard<std::mutex> lk(mu);
-        if (!done.count(dev)) {
-            for (auto k : {k_transform_b3<false, false>, k_transform_b3<true, false>, k_transform_b3<false, true>})
-                TDZ_CUDA(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kB3Max));
-            done.insert(dev);
-        }
-    }
+    static std::atomic<unsigned long long> done{0};
+    once_per_device(done, [] {
+        for (auto k : {k_transform_b3<false, false>, k_transform_b3<true, false>, k_transform_b3<false, true>})
+            allow_smem(k, kB3Max);
+    });
     TDZ_CHECK((reinterpret_cast<uintptr_t>(in) & 15) == 0, TDZ_ERR_ARG, "transform operand not 16-byte aligned");
     TDZ_CHECK(ldi % 4 == 0, TDZ_ERR_ARG, "transform row pitch not a multiple of 16 bytes");
     const long long rows = 2LL * planes * R;
@@ -937,22 +929,11 @@ void launch(const TransformMat &T, const float *in, int ldi, TGParams prm, cudaS
     const bool ws = variant() != 2;
     constexpr int MS = sub_tiles<NP>();
     const size_t smem = ws ? WSShape<NP>::SMEM : TGShape<NP, MS>::SMEM;
-    // opt-in to the tile's shared memory once per device (guarded: the batch
-    // API steps runs from several host threads)
-    {
-        static std::mutex mu;
-        static std::set<int> done;
-        int dev = 0;
-        TDZ_CUDA(cudaGetDevice(&dev));
-        std::lock_guard<std::mutex> lk(mu);
-        if (!done.count(dev)) {
-            TDZ_CUDA(cudaFuncSetAttribute(k_transform<NP, MS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)TGShape<NP, MS>::SMEM));
-            TDZ_CUDA(cudaFuncSetAttribute(k_transform_ws<NP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                          (int)WSShape<NP>::SMEM));
-            done.insert(dev);
-        }
-    }
+    static std::atomic<unsigned long long> done{0};
+    once_per_device(done, [] {
+        allow_smem(k_transform<NP, MS>, TGShape<NP, MS>::SMEM);
+        allow_smem(k_transform_ws<NP>, WSShape<NP>::SMEM);
+    });
     CUtensorMap amap;
     const int rows_per_tile = ws ? TM : TM * MS;
     make_map(&amap, in, (uint64_t)T.K, (uint64_t)prm.rows, (uint64_t)ldi, (uint32_t)rows_per_tile);
