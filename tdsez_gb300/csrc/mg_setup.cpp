@@ -232,7 +232,8 @@ void Multigrid::setup(Operator *fine_, const MGOptions &o, cudaStream_t st) {
             op->upload_bases();
             // the non-separable term is rediscretised on the level (its Galerkin
             // product is not a Kronecker sum)
-            if (fo.quad.on) op->quad.build(op->space, fo.quad.nsoft, &fo.quad.soft[0][0]);
+            if (fo.quad.on)
+                op->quad.build(op->space, fo.quad.nsoft, &fo.quad.soft[0][0], prec == TDZ_FP64 ? kQuad64 : kQuad32);
             m.opp = op.get();
             m.op = std::move(op);
         }

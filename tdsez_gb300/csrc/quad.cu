@@ -4,7 +4,8 @@
 // memory ping-pong), multiply by w V with V from the closed form, project back
 // axis by axis and add coef * result to y with atomics (neighbouring elements
 // share coefficients); or, for ordinary knots, the streaming kernel below.
-// 2D: the assembled stencil (k_stencil2).
+// 2D: the assembled stencil (k_stencil2), or for tables beyond kQuad2Table one
+// CTA per element (k_quad2).
 #include "quad.h"
 
 #include <algorithm>
@@ -134,6 +135,71 @@ __global__ void __launch_bounds__(kQThreads) k_quad(const QuadParams<T> prm) {
     }
 }
 
+// the same in 2D, for stencils that would take too much memory
+template <class T, int P>
+__global__ void __launch_bounds__(kQThreads) k_quad2(const QuadParams<T> prm) {
+    using C = typename CT<T>::type;
+    constexpr int NP = P + 1, M = NP > kMaxQ ? NP : kMaxQ;
+    __shared__ C bufA[M * M], bufB[M * M];
+    __shared__ T sN[2][kMaxQ * NP], sW[2][kMaxQ], sX[2][kMaxQ];
+    const int Q = prm.nq, tid = threadIdx.x;
+    const int el[2] = {(int)(blockIdx.x % prm.nel[0]), (int)(blockIdx.x / prm.nel[0])};
+    const int ox = prm.off[0][el[0]], oy = prm.off[1][el[1]];
+    for (int d = 0; d < 2; ++d) {
+        for (int i = tid; i < Q * NP; i += kQThreads) sN[d][i] = prm.N[d][(size_t)el[d] * Q * NP + i];
+        for (int i = tid; i < Q; i += kQThreads) {
+            sW[d][i] = prm.w[d][(size_t)el[d] * Q + i];
+            sX[d][i] = prm.xq[d][(size_t)el[d] * Q + i];
+        }
+    }
+    const C *X = static_cast<const C *>(prm.x);
+    C *Y = static_cast<C *>(prm.y);
+    for (int i = tid; i < NP * NP; i += kQThreads) bufA[i] = X[(size_t)(oy + i / NP) * prm.n[0] + ox + i % NP];
+    __syncthreads();
+    // x: A[ky][kx] -> B[ky][qx]
+    for (int i = tid; i < NP * Q; i += kQThreads) {
+        const int qx = i % Q, ky = i / Q;
+        C acc = czero<C>();
+        for (int k = 0; k < NP; ++k) rfma(acc, sN[0][qx * NP + k], bufA[ky * NP + k]);
+        bufB[i] = acc;
+    }
+    __syncthreads();
+    // y: B[ky][qx] -> A[qy][qx], times w V
+    for (int i = tid; i < Q * Q; i += kQThreads) {
+        const int qx = i % Q, qy = i / Q;
+        C acc = czero<C>();
+        for (int k = 0; k < NP; ++k) rfma(acc, sN[1][qy * NP + k], bufB[k * Q + qx]);
+        T v = T(0);
+        for (int c = 0; c < prm.nsoft; ++c) {
+            const T dx = sX[0][qx] - prm.soft[c][1], dy = sX[1][qy] - prm.soft[c][2];
+            v -= prm.soft[c][0] * rsqrt_t<T>(dx * dx + dy * dy + prm.soft[c][4]);
+        }
+        const T f = sW[0][qx] * sW[1][qy] * v;
+        acc.x *= f;
+        acc.y *= f;
+        bufA[i] = acc;
+    }
+    __syncthreads();
+    // back y: A[qy][qx] -> B[ky][qx]
+    for (int i = tid; i < NP * Q; i += kQThreads) {
+        const int qx = i % Q, ky = i / Q;
+        C acc = czero<C>();
+        for (int q = 0; q < Q; ++q) rfma(acc, sN[1][q * NP + ky], bufA[q * Q + qx]);
+        bufB[i] = acc;
+    }
+    __syncthreads();
+    // back x and scatter
+    for (int i = tid; i < NP * NP; i += kQThreads) {
+        const int kx = i % NP, ky = i / NP;
+        C acc = czero<C>();
+        for (int q = 0; q < Q; ++q) rfma(acc, sN[0][q * NP + kx], bufB[ky * Q + q]);
+        C out;
+        out.x = prm.cre * acc.x - prm.cim * acc.y;
+        out.y = prm.cre * acc.y + prm.cim * acc.x;
+        atomic_add_c(&Y[(size_t)(oy + ky) * prm.n[0] + ox + kx], out);
+    }
+}
+
 // ---------------------------------------------------------------- 2D stencil
 // The term couples a coefficient to the (2p+1)^2 around it. Its entries are
 // stored one triangle only, entry-major (entry e of every coefficient is
@@ -157,7 +223,7 @@ struct Asm2Params {
     int nel0, nel1, nsoft;
     double soft[kMaxSoft][5];
     double *wv;                            // w V at the Gauss points, [nel1 Q][nel0 Q]
-    double *st64;
+    double *st64;                          // tables to fill (null: not held)
     float *st32;
 };
 
@@ -203,8 +269,8 @@ __global__ void __launch_bounds__(128) k_assemble2(const Asm2Params prm) {
             }
         }
     }
-    prm.st64[(size_t)e * N + idx] = sum;
-    prm.st32[(size_t)e * N + idx] = (float)sum;
+    if (prm.st64) prm.st64[(size_t)e * N + idx] = sum;
+    if (prm.st32) prm.st32[(size_t)e * N + idx] = (float)sum;
 }
 
 // y += coef * V_q x from the stencil; a 32 x 8 tile of coefficients per CTA
@@ -738,14 +804,15 @@ QuadParams<T> make_qparams(const QuadTerm &q, cd coef, const void *x, void *y) {
 
 template <class T, int P>
 void launch_q(const QuadTerm &q, const QuadParams<T> &prm, cudaStream_t st) {
-    const long long nel = (long long)q.nel[0] * q.nel[1] * q.nel[2];
+    const long long nel = (long long)q.nel[0] * q.nel[1] * (q.dim == 3 ? q.nel[2] : 1);
     TDZ_CHECK(nel < (1LL << 31), TDZ_ERR_UNSUPPORTED, "too many elements for the quadrature term");
-    k_quad<T, P><<<(unsigned)nel, kQThreads, 0, st>>>(prm);
+    if (q.dim == 3) k_quad<T, P><<<(unsigned)nel, kQThreads, 0, st>>>(prm);
+    else k_quad2<T, P><<<(unsigned)nel, kQThreads, 0, st>>>(prm);
 }
 
 template <class T>
 void dispatch_q(const QuadTerm &q, cd coef, const void *x, void *y, cudaStream_t st) {
-    if (q.dim == 2) {
+    if (q.dim == 2 && (sizeof(T) == 8 ? q.st64 : q.st32).ptr) {
         switch (q.p) {
         case 2: launch_stencil2<T, 2>(q, coef, x, y, st); return;
         case 3: launch_stencil2<T, 3>(q, coef, x, y, st); return;
@@ -778,7 +845,7 @@ void dispatch_q(const QuadTerm &q, cd coef, const void *x, void *y, cudaStream_t
     }
 }
 
-void assemble2(QuadTerm &q, const Space &s) {
+void assemble2(QuadTerm &q, const Space &s, int precs) {
     Asm2Params prm{};
     prm.n0 = q.n[0];
     prm.n1 = q.n[1];
@@ -810,8 +877,8 @@ void assemble2(QuadTerm &q, const Space &s) {
     const size_t N = (size_t)q.n[0] * q.n[1], pts = (size_t)q.nel[0] * q.nel[1] * q.nq * q.nq;
     const int ne = quad2_entries(q.p);
     wv.alloc(pts * sizeof(double));
-    q.st64.alloc(N * ne * sizeof(double));
-    q.st32.alloc(N * ne * sizeof(float));
+    if (precs & kQuad64) q.st64.alloc(N * ne * sizeof(double));
+    if (precs & kQuad32) q.st32.alloc(N * ne * sizeof(float));
     prm.wv = wv.as<double>();
     prm.st64 = q.st64.as<double>();
     prm.st32 = q.st32.as<float>();
@@ -826,7 +893,7 @@ void assemble2(QuadTerm &q, const Space &s) {
 
 }  // namespace
 
-void QuadTerm::build(const Space &s, int nsoft_, const double *soft_) {
+void QuadTerm::build(const Space &s, int nsoft_, const double *soft_, int precs, size_t table) {
     on = nsoft_ > 0;
     if (!on) return;
     TDZ_CHECK(s.dim >= 2, TDZ_ERR_UNSUPPORTED, "soft-core centres need a 2D or 3D space");
@@ -858,7 +925,7 @@ void QuadTerm::build(const Space &s, int nsoft_, const double *soft_) {
         upload(w32[d], std::vector<float>(a.wq.begin(), a.wq.end()));
         upload(x32[d], std::vector<float>(a.xq.begin(), a.xq.end()));
     }
-    if (dim == 2) assemble2(*this, s);
+    if (dim == 2 && (size_t)n[0] * n[1] * quad2_entries(p) * sizeof(double) <= table) assemble2(*this, s, precs);
 }
 
 void QuadTerm::apply(cd coef, int prec, const void *x, void *y, cudaStream_t st) const {
