@@ -41,7 +41,7 @@ struct DenseLevel {
     int n[3] = {1, 1, 1}, pd = 0, py = 0, pz = 0;
     DevBuf base[3];                       // per axis M_d^-1 B of every base band, [band][n][n] FP32
     DevBuf rx, ry, rz, cz;                // the stage's combinations (transposed, padded)
-    static bool pays(const int *n, size_t ndof);
+    static bool pays(const int *n, int p, size_t ndof);
     void build(const Operator &op, const int *n);
     // matrices of the operator's current stage; false when the stage is outside
     // the form (complex ratios to g)

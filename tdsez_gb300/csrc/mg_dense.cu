@@ -16,13 +16,13 @@
 //                and the matrices streamed through it
 // Products are packed FP32 on both components; the z matrices are stored as
 // equal pairs, so a coefficient needs no move to become an operand. Used for
-// 3D FP32 levels whose estimated step is shorter (dense_pays) and whose stage
+// 3D FP32 levels whose estimated step is shorter (pays) and whose stage
 // has real ratios to g (no absorbing layer); checked per cycle, else the
 // general step runs.
 //
-// 51 x 51 x 109 level, degree 3: a step of 4 launches and 56 us becomes 2
-// launches and 33 us; on the small levels the launches count, 40 us and more
-// against 14 (27 x 27 x 64) and 11 (15 x 15 x 39).
+// 51 x 51 x 109 level, degree 3: a step of 4 launches and 57 us becomes 2
+// launches and 35 us; on the small levels the launches count, 39 against 19 us
+// (27 x 27 x 74) and 33 against 15 us (15 x 15 x 49).
 #include <algorithm>
 #include <cmath>
 
@@ -125,7 +125,8 @@ struct DenseStep {
 // s.zc columns per CTA, KR rows per thread, the matrices in stages of s.chunk
 // rows. Where they make a CTA for each SM: 8 rows, stages of 16 rows, and as many
 // columns as give every SM the same number of CTAs (51 x 51 x 109: 16 columns, 163
-// CTAs, 26.5 us; 18 columns, 145 CTAs, 19.8 us). Else 8 columns, 4 rows and both
+// CTAs, 26.5 us; 18 columns, 145 CTAs, 19.8 us), an even number of them (61 x 61 x
+// 131, both kernels: 13 columns 63 us, 14 columns 51 us). Else 8 columns, 4 rows and both
 // matrices requested whole at the start, since there a thread's chain of stages
 // and products is all the time (with 16 columns, 8 rows and stages: 27 x 27 x 64
 // 15.6 us, now 7.2 us; 15 x 15 x 39 12.4 and 6.0 us; 9 x 9 x 28 9.9 and 5.0 us).
@@ -223,15 +224,23 @@ size_t z_smem(int n2, int zc, int chunk) {
 
 }  // namespace
 
-// Estimated step times (us): dense, two launches and n_x + n_y + 2 n_z products
-// per coefficient at a third of the FP32 rate; general, four launches of
-// latency-bound kernels plus 43 ps per coefficient (the banded apply's 17 and
-// the line solves' 26 on large grids). Both sides measured at 51 x 51 x 109
-// (33 against 56) and on the benchmark's 163 x 163 x 333 level (general).
-bool DenseLevel::pays(const int *n, size_t ndof) {
-    const double dense = 6.0 + 0.08e-6 * 2.0 * ndof * (n[0] + n[1] + 2 * n[2]);
-    const double general = 35.0 + 43e-6 * ndof;
-    return dense < general && xy_smem(n[0], n[1]) <= kDenseSmem && z_smem(n[2], 16, 16) <= kDenseSmem && n[2] <= 512;
+// Estimated step times (us). Dense: latency; the products of a plane, n_x n_y (n_x +
+// n_y), on one SM, which a second one shares where there are more planes than SMs;
+// the 2 n_z^2 products of an SM's share of the columns, two CTAs of which overlap.
+// General: four launches of kernels bound by the latency of their lines. Measured
+// (coefficients, degree 3 but for the last; dense and general):
+//   27 x 27 x 74   21 and 45      66 x 66 x 133   61 and 65
+//   53 x 53 x 113  37 and 57      75 x 75 x 153  117 and 75
+//   33 x 33 x 193  43 and 61      88 x 88 x 113   92 and 71
+//   83 x 83 x 43   49 and 53      98 x 98 x 53    77 and 61
+//   73 x 73 x 155 of degree 5: 110 and 116
+bool DenseLevel::pays(const int *n, int p, size_t ndof) {
+    if (xy_smem(n[0], n[1]) > kDenseSmem || z_smem(n[2], 16, 16) > kDenseSmem) return false;
+    const double cols = std::max(8.0, std::ceil((double)n[0] * n[1] / sm_count()));
+    const double xy = (double)n[0] * n[1] * (n[0] + n[1]) / 32e3 * (n[2] <= sm_count() ? 1.0 : 1.6);
+    const double z = cols * 2.0 * n[2] * n[2] / 26e3 * (cols > 20 ? 0.8 : 1.0);
+    const double general = (22.0 + 0.13 * (n[0] + n[1] + n[2]) + 15e-6 * ndof) * (p == 5 ? 1.5 : 0.55 + 0.15 * p);
+    return 8.0 + xy + z < general;
 }
 
 void DenseLevel::build(const Operator &op, const int *n_) {
@@ -355,7 +364,7 @@ void DenseLevel::step(const Operator &op, void *z, void *d, void *x, void *u, cd
     if (s.cols > (size_t)8 * sm_count() || z_smem(n[2], 8, n[2]) > kDenseSmem) {
         const size_t most = z_smem(n[2], 20, 16) <= kDenseSmem ? 20 : 16, sms = sm_count();
         const size_t ctas = (s.cols + sms * most - 1) / (sms * most) * sms;
-        s.zc = (int)std::max<size_t>(8, (s.cols + ctas - 1) / ctas);
+        s.zc = (int)std::max<size_t>(8, ((s.cols + ctas - 1) / ctas + 1) / 2 * 2);
         s.chunk = 16;
         k_dense_z<8><<<(unsigned)((s.cols + s.zc - 1) / s.zc), s.zc * (pz / 8), z_smem(n[2], s.zc, 16), st>>>(s);
     } else {

@@ -245,9 +245,9 @@ void Multigrid::setup(Operator *fine_, const MGOptions &o, cudaStream_t st) {
         const size_t es = prec == TDZ_FP64 ? sizeof(double2) : sizeof(float2);
         for (DevBuf *b : {&m.x, &m.b, &m.r, &m.d, &m.z, &m.t1, &m.t2}) b->alloc(m.ndof * es);
     }
-    if (prec == TDZ_FP32)
+    if (prec == TDZ_FP32 && dim == 3)
         for (auto &m : lv)
-            if (DenseLevel::pays(m.n, m.ndof)) m.dense.build(*m.opp, m.n);
+            if (DenseLevel::pays(m.n, p, m.ndof)) m.dense.build(*m.opp, m.n);
     red.init();
     estimate_bounds(st);
     if (opt.learned) learned_setup();
