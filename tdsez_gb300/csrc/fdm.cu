@@ -959,13 +959,19 @@ size_t zsolve_state_size(int P, int n2, size_t lines) {
     default: return state_entries<5>(n2, lines);
     }
 }
-// stored factor (float4 entries), 0 where it is not used: beyond 64 MB it would
-// not stay in L2, and streaming it (88 bytes per coefficient and application
-// at P = 3) costs more than redoing the elimination (97 us against about 120
-// on 163 x 163 lines of 343 rows)
+// Stored factor (float4 entries), 0 where it is not used: beyond 64 MB it would not
+// stay in L2, and with more lines than one CTA of k_zsub per SM (two at degree 5,
+// whose elimination is the longest) the substitution is no longer the shorter chain.
+// Applications of the whole inverse, us, elimination and stored factor; then two
+// applications with a factorisation before them, as a step with new field values
+// takes them (degree 3, lines x rows):
+//   4489 x 69: 66 and 56, 128 and 128       5041 x 69: 66 and 62, 129 and 142
+//   10609 x 59: 72 and 70, 140 and 148      17689 x 69: 88 and 97, 169 and 201
+//   degree 5: 9409 x 65: 93 and 77, 171 and 165
 template <int P> size_t factor_entries(int n2, size_t lines) {
     const size_t e = (size_t)2 * z_blocks(n2, ZBlk<P>::B) * ZBlk<P>::B * ZFac<P>::FP * lines;
-    return e * sizeof(float4) <= ((size_t)64 << 20) && zsub_smem<P>(n2) <= 220 * 1024 ? e : 0;
+    const size_t most = (size_t)(P == 5 ? 2 : 1) * kZSubLines * sm_count();
+    return lines <= most && e * sizeof(float4) <= ((size_t)64 << 20) && zsub_smem<P>(n2) <= 220 * 1024 ? e : 0;
 }
 size_t zsolve_factor_size(int P, int n2, size_t lines) {
     switch (P) {
