@@ -292,8 +292,9 @@ tdz_status tdz_vec_mdot(const void *const *V, int k, const void *w, long long n,
 tdz_status tdz_vec_mdot_noalloc(const void *const *V, int k, const void *w, long long n, int precision, void *out,
                                 void *stream);
 
-/* Batched complex-by-real transform on the tensor cores (tcgen05, TF32 with
- * a hi/lo split of both operands: FP32 accuracy), the eigenvector transform of the
+/* Batched complex-by-real transform on the tensor cores (tcgen05, both operands
+ * as three BF16 slices, or beyond 176 x 176 as TF32 hi/lo pairs: FP32 accuracy),
+ * the eigenvector transform of the
  * fast-diagonalisation preconditioner; the counterpart of the per-axis
  * contraction of TDSEZTensorOps::Term (src/tensorops.cpp:97-153) for a dense
  * matrix:

@@ -41,13 +41,14 @@ struct PcFDM : Precond {
     // dropped, or the dropped terms' stage scalars are zero now
     bool exact_now() const;
     DevBuf zb;                 // FP32 upper band rows (Bc, Cc) of the line matrices in elimination order
-    DevBuf zfac;               // stored line factor of small problems (empty: eliminated in every application)
+    DevBuf zfac;               // stored line factor of few lines, up to 64 MB (empty: eliminated in every
+                               // application; captured applications eliminate, so ufac is held as well)
     std::vector<float> zfac_key;   // the coefficients it was computed for
     bool zfac_valid = false;
     DevBuf b1, b2, ufac;       // FP32 work vectors and the saved elimination states of the line solves
     bool exact = true;         // false: inner one-axis terms were dropped (stiffness-only pencil, or a
                                // field along an inner axis)
-    // 3D with n_x, n_y <= 256: transforms on the tensor cores (tcgen05, TF32 hi/lo split) over
+    // 3D with n_x, n_y <= 256: transforms on the tensor cores (tcgen05, tgemm.h) over
     // row-planar FP32 buffers pa ([z][y][c][x], pitch ldx) and pb ([z][x][c][y], pitch ldy)
     bool tensor = false;
     TransformMat Tf[2], Ti[2];

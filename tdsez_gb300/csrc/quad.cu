@@ -541,7 +541,8 @@ __global__ void __launch_bounds__(kQsThreads) k_quad3_stream(const QuadParams<ty
 // 8 x 8 elements in (x, y) and streams a chunk of their z column; thread (ex,
 // qy) owns the Q quadrature columns of element ex at quadrature row qy, so a
 // column's interpolated planes (v, the last p + 1) and its z-projected
-// accumulators (g, the next p + 1) never leave its registers, and the
+// accumulators (g, the next p + 1) stay in its registers (degrees 2 and 3; 24
+// bytes of a thread are spilled at degree 4, 424 at degree 5), and the
 // contractions along x at either end are register loops too. Per coefficient
 // plane: y interpolation through shared memory (sX -> sY), then per thread the
 // x interpolation, the z element (interpolate, times w V from the closed form,
